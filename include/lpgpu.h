@@ -77,11 +77,13 @@ typedef struct {
 /* lpgpu_config.flags: run the refine as one persistent launch per round (every
  * CTA refines whole instances taken from a device work queue), or force the
  * multi-launch sub-round pipeline. Without either flag the session's tuning
- * decides (lpgpu_session_set_tuning, else the process-wide tuning table).
+ * decides (lpgpu_session_set_tuning, else the process-wide tuning table), and
+ * a single instance with k <= 128 that no tuning covers runs all its rounds in
+ * one launch (a CTA, a thread-block cluster or the whole grid, by its size).
  * The persistent form needs every instance's k <= LPGPU_PERSISTENT_MAX_K and
  * no explicit refinement node list; otherwise the refine returns
  * LPGPU_ERR_INVALID_ARG when it is forced and takes the multi-launch form
- * when it is only tuned. Both forms give identical results. */
+ * when it is only tuned. All forms give identical results. */
 #define LPGPU_FLAG_PERSISTENT 2
 #define LPGPU_FLAG_MULTI_LAUNCH 4
 #define LPGPU_PERSISTENT_MAX_K 64
@@ -275,8 +277,9 @@ LPGPU_API lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config
 
 /* Process-wide tuning table (the autotuner's output, rows in priority order;
  * the first row that applies wins; count 0 clears it). Without a matching
- * row, and without a session tuning, refines use the multi-launch form. This
- * has no counterpart in the reference, which has no device code to tune. */
+ * row, and without a session tuning, refines use the grid-wide form (one
+ * launch for a single instance with k <= 128, else the multi-launch pipeline;
+ * reported as LPGPU_MODE_MULTI_LAUNCH). This has no counterpart in the reference, which has no device code to tune. */
 LPGPU_API lpgpu_status lpgpu_set_tuning_table(const lpgpu_tuning_entry* entries, int32_t count);
 
 /* Tuning of one session (NULL: back to the table). lpgpu_session_tuning gives

@@ -221,6 +221,13 @@ struct Launch {
   int num_sms;
 };
 
+// Counts the launch and reports a kernel that failed to launch through the
+// library's error text.
+cudaError_t launched(const char* name);
+// Raises a kernel's dynamic shared memory limit on the current device to at
+// least `bytes` (it only ever grows).
+void allow_dyn_smem_of(const void* kern, size_t bytes);
+
 cudaError_t scan_exclusive_i64(const int64_t* in, int64_t* out, int64_t count, int64_t* tmp,
                                int64_t tmp_elems, cudaStream_t st);
 int64_t scan_tmp_elems(int64_t count);
@@ -301,16 +308,17 @@ cudaError_t launch_rebalance_round(const Launch& L, const RoundCtx& c, int round
 cudaError_t launch_repair_candidates(const Launch& L, const RoundCtx& c, int blk, uint64_t* keys, int32_t* ws,
                                      int4* out, int64_t* scratch);
 
-// ---- persistent rounds (one launch per LP round of a batch of small instances)
+// ---- team rounds (LP rounds of whole instances inside one launch)
 
-// Largest k of an instance the persistent round kernel takes (Λ records of
-// at most 2 words).
+// Largest k of an instance the team kernel takes (Λ records of at most 4
+// words), and the largest one the persistent form of the API accepts.
+constexpr int kTeamMaxK = 128;
 constexpr int kPxMaxK = 64;
 
-// One instance of a persistent round. Arrays are indexed by the ids the
-// instance's CSR stores (union ids in a batched session), so several
-// instances may share one set of arrays; keys / kw / cand hold v1 - v0
-// entries of per-instance scratch starting at their pointer.
+// One instance of a team launch. Arrays are indexed by the ids the instance's
+// CSR stores (union ids in a batched session), so several instances may share
+// one set of arrays; keys / kw / cand / list hold v1 - v0 entries of
+// per-instance scratch starting at their pointer.
 struct PxInst {
   const int64_t* net_off;
   const int32_t* pins;
@@ -324,35 +332,54 @@ struct PxInst {
   int64_t* bw;          // block weights at [boff, boff + k)
   const int64_t* lmax;
   const int64_t* perfect;
-  uint8_t* flag;        // bit 0: active this round, bit 1: active next round
-  int4* rec;            // per vertex: (to, gain, -, from) of its candidate move
-  uint8_t* status;      // per vertex: 1 committed, 2 reverted, 3 rolled back
+  uint8_t* flag;        // 1: active in the next round
+  int4* rec;            // candidate records (vertex, gain, to | from << 16, weight)
+  uint8_t* status;      // per candidate: 1 committed, 2 reverted, 3 rolled back
   uint64_t* keys;       // selection keys (scratch)
-  int32_t* kw;          // selection weights (scratch)
-  int32_t* cand;        // the sub-round's candidates as local ids (scratch)
+  int32_t* kw;          // selection weights, heavy vertices of a sweep (scratch)
+  int32_t* cand;        // the round's kept moves as local ids (scratch)
+  int32_t* list;        // the round's active vertices by sub-round, local ids (scratch)
   int32_t* net_epoch;   // round stamp of nets whose pins were activated
   int64_t* stats;       // kStats counters per round, round r at r * kStats (added to)
   int64_t v0, v1;
+  int64_t e0, e1;       // the instance's nets
   int32_t boff, k;
   int32_t kstride;      // Φ row length
-  int32_t W;            // Λ words per record half (1 or 2)
+  int32_t W;            // Λ words per record half (1, 2 or 4)
   int32_t unit_nets, phi16, max_we;
-  int32_t round;        // round of this instance (when the launch does not set one)
+  int32_t round;        // first round of this instance (when the launch does not set one)
 };
 
 struct PxParams {
   int32_t S, zero_gain, revert, rollback;
   int64_t act_threshold;
-  int32_t round;        // >= 0: every instance runs this round; < 0: its own `round`
-  int32_t unroll;       // incidences per lane step of the sweep (4 or 8)
+  int32_t round;        // >= 0: every instance starts at this round; < 0: at its own `round`
+  int32_t rounds;       // rounds to run (an instance without active vertices stops earlier)
+  int32_t activate_last;  // 1: the last of them also activates its successor's vertices
+  int32_t unroll;       // incidences per lane step of the sweep (4 or 8; W = 4: always 4)
+  int32_t T;            // CTAs per team
+  int32_t kcap;         // largest k of the launch
 };
 
-// Runs one LP round of `count` instances, taken in `order` (null:
-// 0..count-1) from the work queue counter `queue` (zeroed here). W: Λ words
-// class of all instances (1 or 2); unit: every net weight is 1; ctas_per_sm:
-// the 1- or 2-CTA-per-SM build of the kernel.
+// int64 words of global scratch one team of more than one CTA needs.
+inline int64_t team_scratch_words(int kcap) { return 32 + 17 * (int64_t)kcap; }
+
+// CTAs per team of a launch over one instance of n vertices (1: a CTA; up to
+// kTeamMaxCluster: a thread-block cluster; more: the whole cooperative grid).
+constexpr int kTeamMaxCluster = 16;
+
+// Runs LP rounds of `count` instances, taken in `order` (null: 0..count-1)
+// from the work queue counter `queue` (zeroed here) by `teams` teams of P.T
+// CTAs each. W: Λ words class of all instances (1, 2 or 4); unit: every net
+// weight is 1; ctas_per_sm: the 1- or 2-CTA-per-SM build of the kernel.
+// `scratch`: teams * team_scratch_words(P.kcap) words (P.T > 1, zeroed here).
+// A grid barrier that gives up sets *err. More than kTeamMaxCluster CTAs per
+// team need count == 1.
 cudaError_t launch_px_round(const Launch& L, const PxInst* insts, const int32_t* order, int32_t count,
-                            const PxParams& P, int W, bool unit, int ctas_per_sm, int64_t* queue);
+                            PxParams P, int W, bool unit, int ctas_per_sm, int teams, int64_t* scratch,
+                            int64_t* queue, int64_t* err);
+// Largest number of CTAs of the kernel build that can be resident at once.
+int team_resident(const Launch& L, int W, bool unit, int unroll, int ctas_per_sm);
 // out[i]: active vertices of instance i's round `insts[i].round` (from its statistics).
 cudaError_t launch_px_active(const Launch& L, const PxInst* insts, int32_t count, int64_t* out);
 

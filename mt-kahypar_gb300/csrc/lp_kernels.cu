@@ -9,63 +9,9 @@
 #include <mutex>
 #include <utility>
 
-#include "common.cuh"
+#include "lp_device.cuh"
 
 namespace lpgpu {
-
-#define FULLMASK 0xffffffffu
-
-
-__device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
-__device__ __forceinline__ unsigned lanemask_lt() { return (1u << lane_id()) - 1u; }
-
-template <typename T>
-__device__ __forceinline__ T warp_sum(T v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULLMASK, v, o);
-  return v;
-}
-
-// Block-wide sum of an int64 (any blockDim multiple of 32, <= 1024). All threads get the total.
-__device__ int64_t block_sum_i64(int64_t v) {
-  __shared__ int64_t ws[32];
-  v = warp_sum(v);
-  const int w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  __syncthreads();
-  if (lane_id() == 0) ws[w] = v;
-  __syncthreads();
-  int64_t t = lane_id() < nw ? ws[lane_id()] : 0;
-  t = warp_sum(t);
-  return t;
-}
-
-// Block-wide exclusive scan of an int64 (blockDim multiple of 32, <= 1024).
-__device__ int64_t block_scan_excl_i64(int64_t v, int64_t* total) {
-  __shared__ int64_t ws[32];
-  const int lane = lane_id(), w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  int64_t x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int64_t y = __shfl_up_sync(FULLMASK, x, o);
-    if (lane >= o) x += y;
-  }
-  __syncthreads();
-  if (lane == 31) ws[w] = x;
-  __syncthreads();
-  if (w == 0) {
-    int64_t s = lane < nw ? ws[lane] : 0;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int64_t y = __shfl_up_sync(FULLMASK, s, o);
-      if (lane >= o) s += y;
-    }
-    if (lane < nw) ws[lane] = s;
-  }
-  __syncthreads();
-  const int64_t prefix = w > 0 ? ws[w - 1] : 0;
-  *total = ws[nw - 1];
-  return prefix + x - v;
-}
 
 static int blocks_per_sm_hint = 4;
 
@@ -80,9 +26,7 @@ static int grid_for(const Launch& L, int64_t work_items, int threads, int per_sm
 // sessions driven from several host threads launch the same kernel with
 // different sizes: it only ever grows, under a lock, so that no thread lowers
 // it below the size another thread is about to launch with.
-template <typename Kernel>
-static void allow_dyn_smem(Kernel kern_fn, size_t bytes) {
-  const void* kern = (const void*)kern_fn;
+void allow_dyn_smem_of(const void* kern, size_t bytes) {
   static std::mutex mu;
   static std::map<std::pair<int, const void*>, size_t> limits;
   int dev = 0;
@@ -91,6 +35,10 @@ static void allow_dyn_smem(Kernel kern_fn, size_t bytes) {
   size_t& cur = limits[{dev, kern}];
   if (bytes > cur && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess)
     cur = bytes;
+}
+template <typename Kernel>
+static void allow_dyn_smem(Kernel kern, size_t bytes) {
+  allow_dyn_smem_of((const void*)kern, bytes);
 }
 
 // Resident CTAs per SM of `kern` (at least 1).
@@ -108,7 +56,7 @@ static thread_local int64_t t_launches = 0;
 int64_t kernel_launches() { return t_launches; }
 void add_kernel_launches(int64_t n) { t_launches += n; }
 
-static cudaError_t launched(const char* name) {
+cudaError_t launched(const char* name) {
   ++t_launches;
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) set_error(std::string(name) + ": " + cudaGetErrorString(e));
@@ -180,74 +128,6 @@ cudaError_t scan_exclusive_i64(const int64_t* in, int64_t* out, int64_t count, i
   k_scan_tiles<<<(unsigned)tiles, kScanThreads, 0, st>>>(in, out, count, sums);
   LAUNCHED("k_scan_tiles");
   return cudaGetLastError();
-}
-
-// Incidence packing shared by the kernels that walk the incidences of a set
-// of vertices (one per lane). Vertices of degree 1..32 are packed greedily
-// into groups of <= 32 incidences (lane = incidence, contiguous per vertex);
-// longer vertices are walked alone in 32-incidence chunks. For every group
-// `body(has, ow, j, seg_end)` runs on all lanes: lane `has` holds incidence j
-// (index into inets) of the vertex held by lane `ow`. The return value is, on
-// each selected lane, the sum over its vertex's incidences of the ints
-// returned by body (segmented sums inside a group).
-template <typename Body>
-__device__ __forceinline__ int packed_incidences(bool sel, int64_t o0, int deg,
-                                                 unsigned char* __restrict__ s_owner, Body&& body) {
-  const int lane = lane_id();
-  int my_total = 0;
-  const bool small = sel && deg >= 1 && deg <= 32;
-  const int dsm = small ? deg : 0;
-  int incl = dsm;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(FULLMASK, incl, o);
-    if (lane >= o) incl += y;
-  }
-  const int excl = incl - dsm;
-  unsigned rem = __ballot_sync(FULLMASK, small);
-  while (rem) {
-    const int q = __ffs(rem) - 1;
-    const int start = __shfl_sync(FULLMASK, excl, q);
-    const bool inpack = ((rem >> lane) & 1u) && incl - start <= 32;
-    const unsigned pmask = __ballot_sync(FULLMASK, inpack);
-    const int D = __shfl_sync(FULLMASK, incl, 31 - __clz(pmask)) - start;
-    const int st = excl - start;
-    __syncwarp();
-    if (inpack) s_owner[__popc(pmask & lanemask_lt())] = (unsigned char)lane;
-    const unsigned starts = __reduce_or_sync(FULLMASK, inpack ? (1u << st) : 0u);
-    __syncwarp();
-    const bool has = lane < D;
-    const int ow = has ? s_owner[__popc(starts & ((2u << lane) - 1u)) - 1] : lane;
-    const int64_t o_ow = __shfl_sync(FULLMASK, o0, ow);
-    const int st_ow = __shfl_sync(FULLMASK, st, ow);
-    const int d_ow = __shfl_sync(FULLMASK, deg, ow);
-    const int seg_end = has ? st_ow + d_ow : lane + 1;
-    int x = body(has, ow, has ? o_ow + lane - st_ow : (int64_t)0);
-    // segmented suffix sums: the first lane of every vertex gets its total
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_down_sync(FULLMASK, x, o);
-      if (lane + o < seg_end) x += y;
-    }
-    const int tot = __shfl_sync(FULLMASK, x, inpack ? st : 0);
-    if (inpack) my_total = tot;
-    rem &= ~pmask;
-  }
-  unsigned bigm = __ballot_sync(FULLMASK, sel && deg > 32);
-  while (bigm) {
-    const int j = __ffs(bigm) - 1;
-    bigm &= bigm - 1;
-    const int64_t oj = __shfl_sync(FULLMASK, o0, j);
-    const int dj = __shfl_sync(FULLMASK, deg, j);
-    int acc = 0;
-    for (int base = 0; base < dj; base += 32) {
-      const bool has = base + lane < dj;
-      acc += body(has, j, has ? oj + base + lane : (int64_t)0);
-    }
-    acc = warp_sum(acc);
-    if (lane == j) my_total = acc;
-  }
-  return my_total;
 }
 
 // ============================================================ incidence
@@ -566,343 +446,9 @@ cudaError_t launch_metrics(const Launch& L, const RoundCtx& c) {
 
 // ====================================================== sweep / best move
 
-// 32 x 32 bit transpose across a warp (recursive block swap with shuffles):
-// on return lane j holds the word whose bit i is bit j of lane i's input.
-__device__ __forceinline__ uint32_t transpose32(uint32_t x) {
-  const int lane = lane_id();
-#pragma unroll
-  for (int s = 16; s >= 1; s >>= 1) {
-    const uint32_t m = s == 16 ? 0x0000FFFFu : s == 8 ? 0x00FF00FFu : s == 4 ? 0x0F0F0F0Fu
-                     : s == 2 ? 0x33333333u : 0x55555555u;
-    const uint32_t y = __shfl_xor_sync(FULLMASK, x, s);
-    x = (lane & s) ? ((x & ~m) | ((y >> s) & m)) : ((x & m) | ((y << s) & ~m));
-  }
-  return x;
-}
-
-// W words of a Λ record. NC: through the read-only data path (records that
-// no thread of the running kernel changes); otherwise plain coherent loads.
-template <int W, bool NC = true>
-__device__ __forceinline__ void load_words(const uint32_t* __restrict__ p, uint32_t (&w)[W]) {
-  if constexpr (W % 4 == 0) {
-#pragma unroll
-    for (int i = 0; i < W / 4; ++i) {
-      const uint4 q = NC ? __ldg(reinterpret_cast<const uint4*>(p) + i) : reinterpret_cast<const uint4*>(p)[i];
-      w[4 * i] = q.x; w[4 * i + 1] = q.y; w[4 * i + 2] = q.z; w[4 * i + 3] = q.w;
-    }
-  } else if constexpr (W == 2) {
-    const uint2 q = NC ? __ldg(reinterpret_cast<const uint2*>(p)) : *reinterpret_cast<const uint2*>(p);
-    w[0] = q.x; w[1] = q.y;
-  } else {
-#pragma unroll
-    for (int i = 0; i < W; ++i) w[i] = NC ? __ldg(p + i) : p[i];
-  }
-}
-
-// Weighted sum over the lanes in `mask` from weight bit-planes:
-// sum_p popc(bits[p] & mask) << p (planes beyond kPlanes recomputed by the caller).
-constexpr int kPlanes = 4;
-
-struct Planes {
-  uint32_t b[kPlanes];
-  int n;  // number of planes in use (<= 31)
-};
-
-// Bit-planes of a per-lane non-negative weight `w` (all lanes participate).
-__device__ __forceinline__ Planes make_planes(int w, int nplanes) {
-  Planes p;
-  p.n = nplanes;
-#pragma unroll
-  for (int i = 0; i < kPlanes; ++i) p.b[i] = i < nplanes ? __ballot_sync(FULLMASK, (w >> i) & 1) : 0u;
-  return p;
-}
-
-// sum over lanes in mask of w; warp-uniform call (extra planes via ballot).
-__device__ __forceinline__ int plane_sum(const Planes& p, uint32_t mask, int w) {
-  int s = 0;
-#pragma unroll
-  for (int i = 0; i < kPlanes; ++i) s += __popc(p.b[i] & mask) << i;
-  for (int i = kPlanes; i < p.n; ++i) s += __popc(__ballot_sync(FULLMASK, (w >> i) & 1) & mask) << i;
-  return s;
-}
-
-// Decision of Km1Policy::computeMaxGainMoveImpl (gain_policy.h:147-166,
-// disable_randomization) from penalties held by block-owning lanes: lane l
-// owns blocks l + 32 t and pen[t] = sum of w(e) over incident nets with that
-// block in Λ(e). score(b) = internal - pen(b); the move goes to the feasible
-// block (slack(b) >= w(v), b != from) of minimum score < 0, lowest id on ties.
-// Without one, and with zero_gain, the lowest feasible block of score 0 is
-// taken if the rebalancing rule of label_propagation_refiner.h:88-95 holds.
-template <int W, bool PACKED>
-__device__ __forceinline__ void decide(int k, int from, int wv, int internal, int zero_gain,
-                                       const int (&pen)[W], const int (&slack)[W],
-                                       const int64_t* __restrict__ s_bw,
-                                       const int64_t* __restrict__ s_perf, int& to, int& gain) {
-  const int lane = lane_id();
-  // quick reject: neither an improving move (pen > internal) nor a zero-gain
-  // candidate (pen == internal) exists when every other block's penalty is
-  // below the internal weight
-  int any = -1;
-#pragma unroll
-  for (int t = 0; t < W; ++t) {
-    const int blk = 32 * t + lane;
-    if (blk != from && pen[t] > any) any = pen[t];
-  }
-  if (__reduce_max_sync(FULLMASK, any) < internal) return;
-  int zb = INT_MAX;
-  if constexpr (PACKED) {
-    // penalties below 2^20: one max over (pen << 11 | 2047 - blk) gives the
-    // largest penalty and, on ties, the lowest block; 0 = no feasible block
-    unsigned key = 0;
-#pragma unroll
-    for (int t = 0; t < W; ++t) {
-      const int blk = 32 * t + lane;
-      if (blk < k && blk != from && slack[t] >= wv) {
-        const unsigned kk = ((unsigned)pen[t] << 11) | (unsigned)(2047 - blk);
-        key = kk > key ? kk : key;
-        if (zb == INT_MAX && pen[t] == internal) zb = blk;
-      }
-    }
-    const unsigned mk = __reduce_max_sync(FULLMASK, key);
-    if (mk != 0 && (int)(mk >> 11) > internal) {
-      to = 2047 - (int)(mk & 2047u);
-      gain = internal - (int)(mk >> 11);
-      return;
-    }
-  } else {
-    int bp = -1, bb = INT_MAX;
-#pragma unroll
-    for (int t = 0; t < W; ++t) {
-      const int blk = 32 * t + lane;
-      if (blk < k && blk != from && slack[t] >= wv) {
-        if (pen[t] > bp) { bp = pen[t]; bb = blk; }
-        if (zb == INT_MAX && pen[t] == internal) zb = blk;
-      }
-    }
-    const int mp = __reduce_max_sync(FULLMASK, bp);
-    if (mp > internal) {
-      to = __reduce_min_sync(FULLMASK, bp == mp ? bb : INT_MAX);
-      gain = internal - mp;
-      return;
-    }
-  }
-  if (zero_gain) {
-    const int z = __reduce_min_sync(FULLMASK, zb);
-    if (z != INT_MAX && s_bw[from] - 1 > s_bw[z] + 1 && s_bw[z] < s_perf[z]) {
-      to = z;
-      gain = 0;
-    }
-  }
-}
-
 constexpr int kSweepThreads = 256;
-
 __device__ bool last_cta(int64_t* counter);
 __device__ void plan_to(const RoundCtx& c);
-
-// ---- lane-per-vertex sweep (k <= 128)
-//
-// A lane evaluates its own vertex: it walks the vertex's incident nets and adds
-// each net's Λ(e) bit vector (times w(e)) into bit-sliced counters, one
-// 32-block word t and plane p per register cnt[t][p], so that bit l of plane p
-// is bit p of the penalty of block 32 t + l. The best target then comes from a
-// bit-sliced maximum over the feasible blocks. Vertices whose summed incident
-// net weight stays below 2^PL take this path; the others take the
-// warp-cooperative windows below.
-constexpr int kLvWeights = 16;  // vertex weights 1..16 have precomputed feasibility masks
-// Incidences per lane whose gathers are issued together (a multiple of 4), and
-// resident CTAs per SM the k <= 128 sweep is compiled for.
-#ifndef LPGPU_LV_UNROLL
-#define LPGPU_LV_UNROLL 4
-#endif
-#ifndef LPGPU_SWEEP_MIN_BLOCKS
-#define LPGPU_SWEEP_MIN_BLOCKS 3
-#endif
-static_assert(LPGPU_LV_UNROLL % 4 == 0, "the carry-save adder takes four vectors at a time");
-
-// cnt += s0 + 2 s1 + 4 s2 (bit-sliced, ripple carry).
-template <int PL>
-__device__ __forceinline__ void lv_add3(uint32_t (&cnt)[PL], uint32_t s0, uint32_t s1, uint32_t s2) {
-  uint32_t cy = cnt[0] & s0;
-  cnt[0] ^= s0;
-  uint32_t t = cnt[1];
-  cnt[1] = t ^ s1 ^ cy;
-  cy = (t & s1) | (cy & (t ^ s1));
-  t = cnt[2];
-  cnt[2] = t ^ s2 ^ cy;
-  cy = (t & s2) | (cy & (t ^ s2));
-#pragma unroll
-  for (int p = 3; p < PL; ++p) {
-    const uint32_t c2 = cnt[p] & cy;
-    cnt[p] ^= cy;
-    cy = c2;
-  }
-}
-
-// cnt += w * x (bit-sliced; w < 2^PL).
-template <int PL>
-__device__ __forceinline__ void lv_add_weighted(uint32_t (&cnt)[PL], uint32_t x, int w) {
-  uint32_t cy = 0;
-#pragma unroll
-  for (int p = 0; p < PL; ++p) {
-    const uint32_t a = ((w >> p) & 1) ? x : 0u;
-    const uint32_t t = cnt[p];
-    cnt[p] = t ^ a ^ cy;
-    cy = (t & a) | (cy & (t ^ a));
-  }
-}
-
-// One step of a lane's vertex: the next U incidences (from index j) of the
-// vertex with incidences [o0, o0 + d) and source block `from` (local) are
-// added into the bit-sliced counters and the internal weight.
-template <int W, bool UNIT, int PL, int U, bool NC = true>
-__device__ __forceinline__ void lv_accumulate(const RoundCtx& c, int64_t o0, int d, int j, int from,
-                                              uint32_t (&cnt)[W][PL], int& internal) {
-  constexpr int W2 = 2 * W;
-  const int fw = from >> 5;
-  const uint32_t fbit = 1u << (from & 31);
-  int32_t ee[U];
-#pragma unroll
-  for (int u = 0; u < U; ++u) ee[u] = j + u < d ? __ldg(&c.inets[o0 + j + u]) : -1;
-  uint32_t wd[U][W], l1[U];
-  int we[U];
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-#pragma unroll
-    for (int t = 0; t < W; ++t) wd[u][t] = 0;
-    l1[u] = fbit;
-    we[u] = 0;
-    if (ee[u] >= 0) {
-      const uint32_t* rec = c.conn + (int64_t)ee[u] * W2;
-      load_words<W, NC>(rec, wd[u]);
-      l1[u] = NC ? __ldg(rec + W + fw) : rec[W + fw];
-      we[u] = UNIT ? 1 : __ldg(&c.w_e[ee[u]]);
-    }
-  }
-#pragma unroll
-  for (int u = 0; u < U; ++u) internal += (l1[u] & fbit) ? 0 : we[u];
-  if constexpr (UNIT) {
-    // carry-save sum of each four vectors, then one 3-bit ripple add
-#pragma unroll
-    for (int g = 0; g < U; g += 4)
-#pragma unroll
-      for (int t = 0; t < W; ++t) {
-        const uint32_t a = wd[g][t], b = wd[g + 1][t], e = wd[g + 2][t], f = wd[g + 3][t];
-        const uint32_t s = a ^ b ^ e;
-        const uint32_t c1 = (a & b) | (e & (a ^ b));
-        const uint32_t c2 = s & f;
-        lv_add3<PL>(cnt[t], s ^ f, c1 ^ c2, c1 & c2);
-      }
-  } else {
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-#pragma unroll
-      for (int t = 0; t < W; ++t) lv_add_weighted<PL>(cnt[t], wd[u][t], we[u]);
-  }
-}
-
-// Best move of one vertex from its counters: the same decision as `decide`
-// (Km1Policy::computeMaxGainMoveImpl with disable_randomization, plus the
-// zero-gain rebalancing rule of label_propagation_refiner.h:88-95). `from`,
-// `to` are local block ids; `bo` is the instance's first global block.
-template <int W, int PL>
-__device__ __forceinline__ void lv_decide(const RoundCtx& c, const uint32_t (&cnt)[W][PL], int internal, int from,
-                                          int wv, int bo, int inst, bool batched, int zero_gain,
-                                          const uint32_t* __restrict__ s_fmask, const int* __restrict__ s_slack,
-                                          const int64_t* __restrict__ s_bw, const int64_t* __restrict__ s_perf,
-                                          int& to, int& gain, bool& border) {
-  const int fw = from >> 5;
-  const uint32_t fbit = 1u << (from & 31);
-  // feasible targets: c(V_b) + w(v) <= L_max(b)
-  uint32_t cand[W];
-  if (!batched && wv >= 1 && wv <= kLvWeights) {
-#pragma unroll
-    for (int t = 0; t < W; ++t) cand[t] = s_fmask[(wv - 1) * W + t];
-  } else {
-    const int kk = batched ? c.inst_k[inst] : c.k;
-#pragma unroll
-    for (int t = 0; t < W; ++t) {
-      uint32_t msk = 0;
-      for (int l = 0; l < 32; ++l) {
-        const int b = 32 * t + l;
-        if (b < kk) {
-          const int64_t sl = batched ? c.lmax[bo + b] - c.bw[bo + b] : (int64_t)s_slack[b];
-          if (sl >= wv) msk |= 1u << l;
-        }
-      }
-      cand[t] = msk;
-    }
-  }
-  // isBorderNode: some incident net holds a block other than `from`
-  uint32_t other = 0, anyc = 0;
-#pragma unroll
-  for (int t = 0; t < W; ++t) {
-    const uint32_t fm = t == fw ? ~fbit : ~0u;
-    uint32_t o = 0;
-#pragma unroll
-    for (int p = 0; p < PL; ++p) o |= cnt[t][p];
-    other |= o & fm;
-    cand[t] &= fm;
-    anyc |= cand[t];
-  }
-  if (!other) return;
-  border = true;
-  if (!anyc) return;
-  // maximum penalty over the candidates, plane by plane from the top
-  int val = 0;
-#pragma unroll
-  for (int p = PL - 1; p >= 0; --p) {
-    uint32_t tt[W], o = 0;
-#pragma unroll
-    for (int t = 0; t < W; ++t) {
-      tt[t] = cand[t] & cnt[t][p];
-      o |= tt[t];
-    }
-    if (o) {
-#pragma unroll
-      for (int t = 0; t < W; ++t) cand[t] = tt[t];
-      val |= 1 << p;
-    }
-  }
-  if (val < internal || (val == internal && !zero_gain)) return;
-  int b = 0;  // lowest block of maximum penalty
-#pragma unroll
-  for (int t = W - 1; t >= 0; --t)
-    if (cand[t]) b = 32 * t + __ffs(cand[t]) - 1;
-  if (val > internal) {
-    to = b;
-    gain = internal - val;
-    return;
-  }
-  const int64_t* bwp = batched ? c.bw + bo : s_bw;
-  const int64_t* pfp = batched ? c.perfect + bo : s_perf;
-  if (bwp[from] - 1 > bwp[b] + 1 && bwp[b] < pfp[b]) {
-    to = b;
-    gain = 0;
-  }
-}
-
-// Best move of one vertex by its own lane (accumulate all incidences, decide);
-// U incidences per step have their gathers in flight together; NC as in
-// load_words.
-template <int W, bool UNIT, int PL, int U = LPGPU_LV_UNROLL, bool NC = true>
-__device__ __forceinline__ void lv_vertex(const RoundCtx& c, int64_t o0, int d, int from, int wv, int bo,
-                                          int inst, bool batched, int zero_gain,
-                                          const uint32_t* __restrict__ s_fmask, const int* __restrict__ s_slack,
-                                          const int64_t* __restrict__ s_bw, const int64_t* __restrict__ s_perf,
-                                          int& to, int& gain, bool& border) {
-  static_assert(U % 4 == 0, "the carry-save adder takes four vectors at a time");
-  uint32_t cnt[W][PL];
-#pragma unroll
-  for (int t = 0; t < W; ++t)
-#pragma unroll
-    for (int p = 0; p < PL; ++p) cnt[t][p] = 0;
-  int internal = 0;  // Σ w(e) over incident nets with Φ(e, from) > 1
-  for (int j = 0; j < d; j += U) lv_accumulate<W, UNIT, PL, U, NC>(c, o0, d, j, from, cnt, internal);
-  lv_decide<W, PL>(c, cnt, internal, from, wv, bo, inst, batched, zero_gain, s_fmask, s_slack, s_bw, s_perf, to,
-                   gain, border);
-}
-
 
 // One heavy vertex (sweep_heavy: summed net weight too large for the lane
 // counters, or more than kHeavyDegree incidences) evaluated by the whole CTA:
@@ -2461,167 +2007,6 @@ __device__ __forceinline__ void activate_incidence(const RoundCtx& c, int64_t e,
 }
 
 
-// ---- CTA-flat incidence walks
-//
-// A CTA collects the selected vertices of a range of list positions in shared
-// memory (first incidence and degree), scans the degrees, and then spreads
-// every incidence of every collected vertex over all its threads: thread t
-// takes incidences t, t + blockDim, ... and finds its vertex by binary search
-// in the scanned degrees. Hub vertices are split across the whole CTA, and the
-// gathers and atomics of different vertices are in flight together.
-#ifndef LPGPU_FLAT_THREADS
-#define LPGPU_FLAT_THREADS 512
-#endif
-constexpr int kFlatThreads = LPGPU_FLAT_THREADS;
-constexpr int kFlatItems = 1024;  // list positions (and so at most this many vertices) per CTA pass
-static_assert(kFlatItems % kFlatThreads == 0, "whole items per thread");
-
-struct FlatSmem {
-  int64_t o0[kFlatItems];    // first incidence
-  int pre[kFlatItems + 1];   // degrees, then their exclusive prefix sums
-  int ft[kFlatItems];        // local from | local to << 16
-  int att[kFlatItems];       // per-vertex sums (attributed delta, or the reverse move's gain)
-  int inst[kFlatItems];      // instance (batched)
-  int pos[kFlatItems];       // list position
-  int wsum[kFlatThreads / 32];
-  int n;
-};
-
-// Warp-aggregated append to a shared counter; returns each selected lane's slot.
-__device__ __forceinline__ int flat_append_to(int* counter, bool sel) {
-  const unsigned m = __ballot_sync(FULLMASK, sel);
-  if (!m) return -1;
-  const int leader = __ffs(m) - 1;
-  int base = 0;
-  if (lane_id() == leader) base = atomicAdd(counter, __popc(m));
-  base = __shfl_sync(FULLMASK, base, leader);
-  return sel ? base + __popc(m & lanemask_lt()) : -1;
-}
-
-// Appends the lanes with `sel` to the CTA's item list; returns each lane's slot.
-__device__ __forceinline__ int flat_append(FlatSmem& f, bool sel) { return flat_append_to(&f.n, sel); }
-
-// In-place exclusive scan of f.pre[0 .. n) (n <= kFlatItems); f.pre[n] = total.
-__device__ __forceinline__ int flat_scan(FlatSmem& f, int n) {
-  constexpr int PER = kFlatItems / kFlatThreads;
-  const int t = threadIdx.x, lane = lane_id(), wid = t >> 5;
-  int v[PER], sum = 0;
-#pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int i = t * PER + q;
-    v[q] = i < n ? f.pre[i] : 0;
-    sum += v[q];
-  }
-  int incl = sum;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(FULLMASK, incl, o);
-    if (lane >= o) incl += y;
-  }
-  if (lane == 31) f.wsum[wid] = incl;
-  __syncthreads();
-  int wbase = 0, total = 0;
-#pragma unroll
-  for (int w = 0; w < kFlatThreads / 32; ++w) {
-    const int x = f.wsum[w];
-    if (w < wid) wbase += x;
-    total += x;
-  }
-  int run = wbase + incl - sum;
-#pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int i = t * PER + q;
-    if (i < n) f.pre[i] = run;
-    run += v[q];
-  }
-  if (t == 0) f.pre[n] = total;
-  __syncthreads();
-  return total;
-}
-
-// Vertex of flat incidence index x: the largest i with pre[i] <= x.
-__device__ __forceinline__ int flat_find(const FlatSmem& f, int n, int x) {
-  int lo = 0, hi = n - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (f.pre[mid] <= x) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
-
-// Commit of Q incidences (e[q], from f[q], to t[q]; h[q]: present): all 2Q Φ
-// atomics are issued before any result is used, then per incidence the
-// decrement of Φ(e, f) and increment of Φ(e, t) toggle Λ when Φ(e, f) reaches
-// 0 or Φ(e, t) leaves 0, and Λ1 when either passes through 1. The attributed
-// delta (km1Delta, hypergraph_common.h:133-140) is -w(e) when Φ(e, f) reaches
-// 0 and +w(e) when Φ(e, t) reaches 1; a[q] is each incidence's part.
-template <int Q>
-__device__ __forceinline__ void commit_group(const RoundCtx& c, const bool (&h)[Q], const int64_t (&e)[Q],
-                                             const int (&f)[Q], const int (&t)[Q], int (&a)[Q], int& toggles) {
-  const int W = c.W;
-  const int64_t k = c.kmax;
-  int of[Q], ot[Q];
-#pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    of[q] = ot[q] = 0;
-    if (h[q]) {
-      of[q] = phi_add(c, e[q] * k + f[q], -1);
-      ot[q] = phi_add(c, e[q] * k + t[q], 1);
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    a[q] = 0;
-    if (!h[q]) continue;
-    const int we = c.unit_nets ? 1 : c.w_e[e[q]];
-    uint32_t* rec = c.conn + e[q] * 2 * W;
-    const uint32_t fb = 1u << (f[q] & 31), tb = 1u << (t[q] & 31);
-    if (of[q] == 1) { atomicXor(&rec[f[q] >> 5], fb); a[q] -= we; ++toggles; }
-    if (of[q] == 1 || of[q] == 2) atomicXor(&rec[W + (f[q] >> 5)], fb);
-    if (ot[q] == 0) { atomicXor(&rec[t[q] >> 5], tb); a[q] += we; ++toggles; }
-    if (ot[q] == 0 || ot[q] == 1) atomicXor(&rec[W + (t[q] >> 5)], tb);
-  }
-}
-
-// Incidences a thread of the CTA-flat commit handles per step.
-#ifndef LPGPU_COMMIT_GROUP
-#define LPGPU_COMMIT_GROUP 2  // 4 and 8 measured slower on rownet
-#endif
-
-// Moves every incidence of the CTA's collected vertices from their `from` to
-// their `to` block (flat over the CTA). Returns this thread's summed delta;
-// per-vertex sums go to f.att when `per_item`; *toggles counts this thread's
-// Λ bit changes.
-__device__ __forceinline__ int64_t flat_commit(const RoundCtx& c, FlatSmem& f, int n, int total, bool per_item,
-                                               int64_t* toggles = nullptr) {
-  constexpr int Q = LPGPU_COMMIT_GROUP;
-  int64_t att = 0;
-  int tg = 0;
-  for (int x0 = threadIdx.x; x0 < total; x0 += Q * kFlatThreads) {
-    bool h[Q];
-    int64_t e[Q];
-    int fr[Q], to[Q], it[Q], a[Q];
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      const int x = x0 + q * kFlatThreads;
-      h[q] = x < total;
-      it[q] = h[q] ? flat_find(f, n, x) : 0;
-      e[q] = h[q] ? c.inets[f.o0[it[q]] + (x - f.pre[it[q]])] : 0;
-      const int ft = h[q] ? f.ft[it[q]] : 0;
-      fr[q] = ft & 0xffff;
-      to[q] = ft >> 16;
-    }
-    commit_group<Q>(c, h, e, fr, to, a, tg);
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      att += a[q];
-      if (per_item && a[q]) atomicAdd(&f.att[it[q]], a[q]);
-    }
-  }
-  if (toggles) *toggles += tg;
-  return att;
-}
-
 // Commit of the accepted moves (changeNodePart, h:539-563, without the
 // per-move weight check: the selection already guarantees both bounds).
 // Marks status[pos] = 1 for committed moves. CTA-flat over ranges of
@@ -3370,503 +2755,6 @@ cudaError_t launch_subround(const Launch& L, const RoundCtx& c, int round, int s
     LAUNCHED("k_rollback");
   }
   return cudaSuccess;
-}
-
-// ======================================================= persistent rounds
-//
-// A batch of many small instances runs one launch per LP round. Every CTA
-// takes whole instances from a device work queue (largest first unless the
-// tuning says otherwise) and runs all S sub-rounds of that instance's round
-// itself: sweep, target- and source-side selection, commit, hindsight
-// reverts, rollback and activation, separated by CTA barriers instead of
-// grid-wide launch boundaries. Instances are independent, so no CTA ever
-// waits for another, and a CTA that finishes a small instance takes the next
-// one while others are still on large ones. Each phase follows the same rule
-// as the multi-launch pipeline (the same lane-per-vertex sweep, selection
-// thresholds and CTA-flat commit), so every instance ends exactly as when it
-// is refined alone. The sweep reads the Λ records that the same kernel's
-// commits change, so it loads them through the coherent path, not __ldg.
-
-constexpr int kPxThreads = kFlatThreads;  // the CTA-flat helpers are written for this width
-constexpr int kPxWarps = kPxThreads / 32;
-static_assert(kPxThreads <= kSelThreads, "the radix selection's histograms cover the CTA");
-
-struct PxShared {
-  int64_t bw[kPxMaxK], lmax[kPxMaxK], perf[kPxMaxK];
-  int slack[kPxMaxK];
-  uint32_t fmask[kLvWeights * 2];
-  ull in_w[kPxMaxK], acc_w[kPxMaxK];
-  unsigned in_cnt[kPxMaxK], acc_cnt[kPxMaxK];
-  int64_t seg[kPxMaxK + 1];
-  unsigned cursor[kPxMaxK];
-  uint64_t thr_to[kPxMaxK], thr_from[kPxMaxK];
-  int pen[kPxWarps][kPxMaxK];
-  int ncand, nrev, item;
-  long long st[kStats];
-};
-
-__device__ __forceinline__ RoundCtx px_ctx(const PxInst& I) {
-  RoundCtx c{};
-  c.vtx_off = I.vtx_off;
-  c.inets = I.inets;
-  c.w_v = I.w_v;
-  c.w_e = I.w_e;
-  c.part = I.part;
-  c.phi = I.phi;
-  c.conn = I.conn;
-  c.k = I.k;
-  c.W = I.W;
-  c.kmax = I.kstride;
-  c.unit_nets = I.unit_nets;
-  c.phi16 = I.phi16;
-  c.max_we = I.max_we;
-  return c;
-}
-
-// A candidate move of local vertex lv: its record, the per-block totals and
-// the sub-round's candidate list.
-__device__ __forceinline__ void px_candidate(const PxInst& I, PxShared& s, int64_t lv, int from, int to, int gain,
-                                             int wv) {
-  I.rec[I.v0 + lv] = make_int4(to, gain, 0, from);
-  atomicAdd(&s.in_w[to], (ull)(int64_t)wv);
-  atomicAdd(&s.in_cnt[to], 1u);
-  I.cand[atomicAdd(&s.ncand, 1)] = (int32_t)lv;
-}
-
-// A heavy vertex (summed net weight beyond the lane counters), evaluated by
-// the warp that found it: lanes split its incidences, penalties are summed per
-// block in the warp's shared row, then the block-owning lanes decide (decide:
-// the rule of Km1Policy::computeMaxGainMoveImpl).
-template <int W, bool UNIT>
-__device__ void px_heavy(const PxInst& I, const PxParams& P, PxShared& s, int64_t lv) {
-  const int lane = lane_id(), wid = threadIdx.x >> 5, k = I.k;
-  int* pen = s.pen[wid];
-  const int64_t v = I.v0 + lv;
-  const int64_t o0 = I.vtx_off[v];
-  const int d = (int)(I.vtx_off[v + 1] - o0);
-  const int from = I.part[v] - I.boff, wv = I.w_v[v];
-  for (int b = lane; b < k; b += 32) pen[b] = 0;
-  __syncwarp();
-  const int fw = from >> 5;
-  const uint32_t fbit = 1u << (from & 31);
-  int internal = 0;
-  bool border = false;
-  for (int j = lane; j < d; j += 32) {
-    const int64_t e = I.inets[o0 + j];
-    const int we = UNIT ? 1 : I.w_e[e];
-    const uint32_t* rec = I.conn + e * 2 * W;
-    if (!(rec[W + fw] & fbit)) internal += we;  // Φ(e, from) > 1
-#pragma unroll
-    for (int t = 0; t < W; ++t) {
-      uint32_t bits = rec[t] & (t == fw ? ~fbit : ~0u);
-      border = border || bits != 0;
-      while (bits) {
-        atomicAdd(&pen[32 * t + __ffs(bits) - 1], we);
-        bits &= bits - 1;
-      }
-    }
-  }
-  internal = warp_sum(internal);
-  border = __any_sync(FULLMASK, border);
-  __syncwarp();
-  if (border) {
-    int pn[W], sl[W];
-#pragma unroll
-    for (int t = 0; t < W; ++t) {
-      const int b = 32 * t + lane;
-      pn[t] = b < k ? pen[b] : 0;
-      sl[t] = b < k ? s.slack[b] : -1;
-    }
-    int to = from, gain = 0;
-    decide<W, false>(k, from, wv, internal, P.zero_gain, pn, sl, s.bw, s.perf, to, gain);
-    if (lane == 0 && to != from) px_candidate(I, s, lv, from, to, gain, wv);
-  }
-  __syncwarp();
-}
-
-constexpr int kPxStage = 2048;  // selection keys staged in the CTA-flat area (not in use then)
-static_assert(sizeof(FlatSmem) >= (size_t)kPxStage * 12, "staged keys and weights fit the CTA-flat area");
-
-#ifndef LPGPU_PX_WARP_SEL
-#define LPGPU_PX_WARP_SEL 512  // segments of at most this many keys get one warp each
-#endif
-constexpr int kPxWarpSelKeys = LPGPU_PX_WARP_SEL;
-static_assert(sizeof(FlatSmem) >= (size_t)(kPxThreads / 32) * 256 * sizeof(unsigned),
-              "every warp's selection histogram fits the CTA-flat area");
-
-// Thresholds of the blocks flagged in `over` (bit b): the first key of the
-// block's segment whose weighted prefix exceeds budget(b). The segments are
-// filled from the candidate list by member(rec, lv) (the block a candidate
-// belongs to, or -1); cnt[b] is the size of block b's segment.
-template <typename Member, typename Budget>
-__device__ void px_select(const PxInst& I, PxShared& s, FlatSmem& f, uint64_t over, const unsigned* cnt,
-                          uint64_t* thr, Member member, Budget budget) {
-  if (threadIdx.x == 0) {
-    int64_t run = 0;
-    for (int b = 0; b < I.k; ++b) {
-      s.seg[b] = run;
-      s.cursor[b] = (unsigned)run;
-      if ((over >> b) & 1) run += cnt[b];
-    }
-    s.seg[I.k] = run;
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < s.ncand; i += blockDim.x) {
-    const int lv = I.cand[i];
-    const int4 r = I.rec[I.v0 + lv];
-    const int b = member(r, lv);
-    if (b >= 0 && ((over >> b) & 1)) {
-      const unsigned slot = atomicAdd(&s.cursor[b], 1u);
-      I.keys[slot] = move_key(r.y, lv);
-      I.kw[slot] = I.w_v[I.v0 + lv];
-    }
-  }
-  __syncthreads();
-  // with several blocks to select, small segments get one warp each, all at
-  // once (histograms in the CTA-flat area, not in use here); the others take
-  // the whole CTA, one after another
-  const int64_t warp_keys = __popcll(over) > 1 ? kPxWarpSelKeys : -1;
-  const int wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  unsigned* whist = reinterpret_cast<unsigned*>(&f) + 256 * wid;
-  for (int b = wid; b < I.k; b += nw) {
-    const int64_t nb = s.seg[b + 1] - s.seg[b];
-    if (((over >> b) & 1) && nb <= warp_keys) {
-      const uint64_t t = warp_radix_select(I.keys + s.seg[b], I.kw + s.seg[b], (int)nb, budget(b), whist);
-      if (lane_id() == 0) thr[b] = t;
-    }
-  }
-  __syncthreads();
-  for (int b = 0; b < I.k; ++b) {
-    if (!((over >> b) & 1) || s.seg[b + 1] - s.seg[b] <= warp_keys) continue;
-    const uint64_t t = cta_radix_select(I.keys + s.seg[b], I.kw + s.seg[b], s.seg[b + 1] - s.seg[b], budget(b),
-                                        reinterpret_cast<unsigned char*>(&f), kPxStage);
-    if (threadIdx.x == 0) thr[b] = t;
-    __syncthreads();
-  }
-}
-
-// Moves the collected items of f (local vertex ids in f.pos, local
-// from | to << 16 in f.ft) between their blocks: part, block weights and,
-// CTA-flat, Φ / Λ / Λ1 with km1Delta attribution. Returns this thread's
-// attributed delta.
-__device__ __forceinline__ int64_t px_move_items(const RoundCtx& c, const PxInst& I, PxShared& s, FlatSmem& f,
-                                                 int64_t* moved_pins, int64_t* toggles) {
-  __syncthreads();
-  const int n = f.n;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const int64_t v = I.v0 + f.pos[i];
-    const int from = f.ft[i] & 0xffff, to = f.ft[i] >> 16;
-    const int64_t wv = I.w_v[v];
-    I.part[v] = I.boff + to;
-    atomicAdd(reinterpret_cast<ull*>(&s.bw[to]), (ull)wv);
-    atomicAdd(reinterpret_cast<ull*>(&s.bw[from]), (ull)(-wv));
-  }
-  const int total = flat_scan(f, n);
-  if (moved_pins && threadIdx.x == 0) *moved_pins += total;
-  const int64_t att = flat_commit(c, f, n, total, false, toggles);
-  __syncthreads();
-  return att;
-}
-
-// Collects into f the candidates [c0, c0 + kFlatItems) of the sub-round list
-// with status `want` (0: the accepted ones), as moves from `from` to `to`
-// (back: the reverse), and sets their status to `set` (0: unchanged).
-// Returns this thread's number of collected items.
-template <bool ACCEPT>
-__device__ __forceinline__ int px_gather(const PxInst& I, PxShared& s, FlatSmem& f, int c0, int ncand, int want,
-                                         bool back, int set) {
-  constexpr int PER = kFlatItems / kPxThreads;
-  if (threadIdx.x == 0) f.n = 0;
-  __syncthreads();
-  int got = 0;
-#pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int i = c0 + q * kPxThreads + threadIdx.x;
-    bool take = false;
-    int lv = 0;
-    int4 r = make_int4(0, 0, 0, 0);
-    if (i < ncand) {
-      lv = I.cand[i];
-      r = I.rec[I.v0 + lv];
-      if constexpr (ACCEPT) {
-        const uint64_t key = move_key(r.y, lv);
-        take = key < s.thr_to[r.x] && key < s.thr_from[r.w];
-      } else {
-        take = I.status[I.v0 + lv] == want;
-      }
-    }
-    const int slot = flat_append(f, take);
-    if (take) {
-      const int64_t v = I.v0 + lv;
-      f.o0[slot] = I.vtx_off[v];
-      f.pre[slot] = (int)(I.vtx_off[v + 1] - f.o0[slot]);
-      f.ft[slot] = back ? (r.x | (r.w << 16)) : (r.w | (r.x << 16));
-      f.att[slot] = 0;
-      f.pos[slot] = lv;
-      if (set) I.status[v] = (uint8_t)set;
-      ++got;
-    }
-  }
-  return got;
-}
-
-template <int W, bool UNIT, int U>
-__device__ void px_instance_round(const PxInst& I, const PxParams& P, PxShared& s, FlatSmem& f) {
-  constexpr int PL = UNIT ? 6 : 8;
-  const RoundCtx c = px_ctx(I);
-  const int k = I.k, S = P.S;
-  const int round = P.round >= 0 ? P.round : I.round;
-  const int64_t ni = I.v1 - I.v0;
-  for (int b = threadIdx.x; b < k; b += blockDim.x) {
-    s.bw[b] = I.bw[I.boff + b];
-    s.lmax[b] = I.lmax[I.boff + b];
-    s.perf[b] = I.perfect[I.boff + b];
-  }
-  if (threadIdx.x < kStats) s.st[threadIdx.x] = 0;
-  int64_t t_active = 0, t_pins = 0, t_moved_pins = 0, t_toggles = 0;
-  __syncthreads();
-  for (int sub = 0; sub < S; ++sub) {
-    // ---- slack, feasibility masks, per-block totals
-    for (int b = threadIdx.x; b < k; b += blockDim.x) {
-      const int64_t sl = s.lmax[b] - s.bw[b];
-      s.slack[b] = sl < 0 ? -1 : (sl > INT_MAX ? INT_MAX : (int)sl);
-      s.in_w[b] = s.acc_w[b] = 0;
-      s.in_cnt[b] = s.acc_cnt[b] = 0;
-      s.thr_to[b] = s.thr_from[b] = ~0ull;
-    }
-    if (threadIdx.x == 0) {
-      s.ncand = 0;
-      s.nrev = 0;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < kLvWeights * W; i += blockDim.x) {
-      const int w = i / W + 1, t = i % W;
-      uint32_t msk = 0;
-      for (int l = 0; l < 32; ++l) {
-        const int b = 32 * t + l;
-        if (b < k && s.slack[b] >= w) msk |= 1u << l;
-      }
-      s.fmask[i] = msk;
-    }
-    __syncthreads();
-    // ---- sweep: a sub-round holds whole 32-vertex chunks; warps take the
-    // sub-round's chunks independently (no CTA barrier), a lane evaluates its
-    // own vertex, and the warp evaluates the chunk's heavy vertices together
-    {
-      const int lane = lane_id(), wid = threadIdx.x >> 5;
-      const int64_t nch = (ni + 31) >> kChunkShift;
-      for (int64_t ch = wid; ch < nch; ch += kPxWarps) {
-        if (subround_of(ch << kChunkShift, round, S) != sub) continue;
-        const int64_t lv = (ch << kChunkShift) + lane, v = I.v0 + lv;
-        bool heavy = false;
-        if (lv < ni && (I.flag[v] & 1)) {
-          I.status[v] = 0;
-          const int64_t o0 = I.vtx_off[v], dd = I.vtx_off[v + 1] - o0;
-          ++t_active;
-          t_pins += dd;
-          const int d = dd > kHighDegree ? 0 : (int)dd;  // isBorderNode is false above the threshold
-          heavy = sweep_heavy(d, W, UNIT, I.max_we);
-          if (!heavy && d > 0) {
-            const int from = I.part[v] - I.boff, wv = I.w_v[v];
-            int to = from, gain = 0;
-            bool border = false;
-            lv_vertex<W, UNIT, PL, U, false>(c, o0, d, from, wv, 0, 0, false, P.zero_gain, s.fmask, s.slack, s.bw,
-                                             s.perf, to, gain, border);
-            if (to != from) px_candidate(I, s, lv, from, to, gain, wv);
-          }
-        }
-        for (unsigned hm = __ballot_sync(FULLMASK, heavy); hm; hm &= hm - 1)
-          px_heavy<W, UNIT>(I, P, s, (ch << kChunkShift) + __ffs(hm) - 1);
-      }
-    }
-    __syncthreads();
-    const int ncand = s.ncand;
-    // ---- target side (the atomic weight check of changeNodePart, h:548-562):
-    // per block the longest (gain, vertex) prefix within L_max
-    uint64_t over = 0;
-    for (int b = 0; b < k; ++b)
-      if ((int64_t)s.in_w[b] > s.lmax[b] - s.bw[b]) over |= 1ull << b;
-    if (over)
-      px_select(I, s, f, over, s.in_cnt, s.thr_to, [](const int4& r, int) { return r.x; },
-                [&](int b) { return s.lmax[b] - s.bw[b]; });
-    // ---- source side (from_weight_after > 0, h:551): per block the longest
-    // prefix of its target-accepted moves that leaves weight >= 1
-    for (int i = threadIdx.x; i < ncand; i += blockDim.x) {
-      const int lv = I.cand[i];
-      const int4 r = I.rec[I.v0 + lv];
-      if (move_key(r.y, lv) < s.thr_to[r.x]) {
-        atomicAdd(&s.acc_w[r.w], (ull)(int64_t)I.w_v[I.v0 + lv]);
-        atomicAdd(&s.acc_cnt[r.w], 1u);
-      }
-    }
-    __syncthreads();
-    uint64_t over_from = 0;
-    for (int b = 0; b < k; ++b)
-      if (s.bw[b] - (int64_t)s.acc_w[b] < 1) over_from |= 1ull << b;
-    if (over_from)
-      px_select(I, s, f, over_from, s.acc_cnt, s.thr_from,
-                [&](const int4& r, int lv) { return move_key(r.y, lv) < s.thr_to[r.x] ? r.w : -1; },
-                [&](int b) { return s.bw[b] - 1; });
-    // ---- commit of the accepted moves
-    int64_t att = 0;
-    for (int c0 = 0; c0 < ncand; c0 += kFlatItems) {
-      px_gather<true>(I, s, f, c0, ncand, 0, false, 1);
-      att += px_move_items(c, I, s, f, &t_moved_pins, &t_toggles);
-    }
-    // ---- hindsight reverts: every committed move is evaluated on the
-    // post-commit state before any is undone (moveVertex,
-    // label_propagation_refiner.h:100-137, made deterministic)
-    if (P.revert) {
-      for (int c0 = 0; c0 < ncand; c0 += kFlatItems) {
-        px_gather<false>(I, s, f, c0, ncand, 1, false, 0);
-        __syncthreads();
-        const int n = f.n;
-        const int total = flat_scan(f, n);
-        // gain of moving back: + w(e) if Φ(e, to) > 1, - w(e) if from is in Λ(e)
-        for (int x = threadIdx.x; x < total; x += kPxThreads) {
-          const int it = flat_find(f, n, x);
-          const int64_t e = I.inets[f.o0[it] + (x - f.pre[it])];
-          const int fa = f.ft[it] & 0xffff, ta = f.ft[it] >> 16;
-          const uint32_t* rec = I.conn + e * 2 * W;
-          const int we = UNIT ? 1 : I.w_e[e];
-          const int xa = (((rec[W + (ta >> 5)] >> (ta & 31)) & 1u) ? 0 : we) -
-                         (((rec[fa >> 5] >> (fa & 31)) & 1u) ? we : 0);
-          if (xa) atomicAdd(&f.att[it], xa);
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += blockDim.x)
-          if (f.att[i] < 0) {
-            I.status[I.v0 + f.pos[i]] = 2;
-            atomicAdd(&s.nrev, 1);
-          }
-        __syncthreads();
-      }
-      if (s.nrev)
-        for (int c0 = 0; c0 < ncand; c0 += kFlatItems) {
-          px_gather<false>(I, s, f, c0, ncand, 2, true, 0);
-          att += px_move_items(c, I, s, f, nullptr, nullptr);
-        }
-    }
-    // ---- rollback of a sub-round whose summed delta is positive
-    att = block_sum_i64(att);
-    int64_t rolled = 0;
-    if (P.rollback && att > 0) {
-      for (int c0 = 0; c0 < ncand; c0 += kFlatItems) {
-        rolled += px_gather<false>(I, s, f, c0, ncand, 1, true, 3);
-        att += block_sum_i64(px_move_items(c, I, s, f, nullptr, nullptr));
-      }
-      rolled = block_sum_i64(rolled);
-    }
-    // ---- activation of the kept moves (label_propagation_refiner.h:112-128):
-    // the vertex and the pins of its nets with |e| <= threshold, once per net
-    int64_t kept = 0;
-    const int stamp = round + 1;
-    for (int c0 = 0; c0 < ncand; c0 += kFlatItems) {
-      kept += px_gather<false>(I, s, f, c0, ncand, 1, false, 0);
-      __syncthreads();
-      const int n = f.n;
-      for (int i = threadIdx.x; i < n; i += blockDim.x) I.flag[I.v0 + f.pos[i]] |= 2;
-      const int total = flat_scan(f, n);
-      for (int x = threadIdx.x; x < total; x += kPxThreads) {
-        const int it = flat_find(f, n, x);
-        const int64_t e = I.inets[f.o0[it] + (x - f.pre[it])];
-        const int64_t p0 = I.net_off[e], p1 = I.net_off[e + 1];
-        if (p1 - p0 <= P.act_threshold && atomicExch(&I.net_epoch[e], stamp) != stamp)
-          for (int64_t j = p0; j < p1; ++j) I.flag[I.pins[j]] |= 2;
-      }
-      __syncthreads();
-    }
-    kept = block_sum_i64(kept);
-    if (threadIdx.x == 0) {
-      s.st[kStCands] += ncand;
-      s.st[kStMoved] += kept;
-      s.st[kStReverted] += s.nrev + rolled;
-      s.st[kStDelta] += att;
-    }
-    __syncthreads();
-  }
-  // ---- end of the instance's round: next round's flags, weights, statistics
-  for (int64_t lv = threadIdx.x; lv < ni; lv += blockDim.x) I.flag[I.v0 + lv] >>= 1;
-  for (int b = threadIdx.x; b < k; b += blockDim.x) I.bw[I.boff + b] = s.bw[b];
-  t_active = block_sum_i64(t_active);
-  t_pins = block_sum_i64(t_pins);
-  t_moved_pins = block_sum_i64(t_moved_pins);
-  t_toggles = block_sum_i64(t_toggles);
-  if (threadIdx.x == 0) {
-    int64_t* st = I.stats + (int64_t)round * kStats;
-    s.st[kStActive] = t_active;
-    s.st[kStPins] = t_pins;
-    s.st[kStMovedPins] = t_moved_pins;
-    s.st[kStToggles] = t_toggles;
-    for (int j = 0; j < kStats; ++j)
-      if (s.st[j]) atomicAdd(reinterpret_cast<ull*>(&st[j]), (ull)s.st[j]);
-  }
-  __syncthreads();
-}
-
-template <int W, bool UNIT, int U, int MINB>
-__global__ void __launch_bounds__(kPxThreads, MINB) k_px_round(const PxInst* __restrict__ insts,
-                                                               const int32_t* __restrict__ order, int32_t count,
-                                                               PxParams P, int64_t* queue) {
-  extern __shared__ __align__(16) unsigned char px_smem[];
-  FlatSmem& f = *reinterpret_cast<FlatSmem*>(px_smem);
-  PxShared& s = *reinterpret_cast<PxShared*>(px_smem + ((sizeof(FlatSmem) + 15) & ~size_t(15)));
-  for (;;) {
-    if (threadIdx.x == 0) s.item = (int)atomicAdd(reinterpret_cast<ull*>(queue), 1ull);
-    __syncthreads();
-    const int it = s.item;
-    __syncthreads();
-    if (it >= count) break;
-    px_instance_round<W, UNIT, U>(insts[order ? order[it] : it], P, s, f);
-  }
-}
-
-constexpr size_t kPxSmem = ((sizeof(FlatSmem) + 15) & ~size_t(15)) + sizeof(PxShared);
-
-// Kernel variant: W words, unit net weights, sweep unroll 4 or 8, compiled for
-// 1 resident CTA per SM (up to 128 registers) or 2 (64 registers).
-template <int W, bool UNIT>
-static const void* px_kernel_wu(int unroll, int minb) {
-  if (minb >= 2) return unroll == 8 ? (const void*)k_px_round<W, UNIT, 8, 2> : (const void*)k_px_round<W, UNIT, 4, 2>;
-  return unroll == 8 ? (const void*)k_px_round<W, UNIT, 8, 1> : (const void*)k_px_round<W, UNIT, 4, 1>;
-}
-
-static const void* px_kernel_for(int W, bool unit, int unroll, int minb) {
-  if (W == 1) return unit ? px_kernel_wu<1, true>(unroll, minb) : px_kernel_wu<1, false>(unroll, minb);
-  return unit ? px_kernel_wu<2, true>(unroll, minb) : px_kernel_wu<2, false>(unroll, minb);
-}
-
-// Active vertices of every instance's last persistent round (its round's
-// statistics), for the host's stop rule.
-__global__ void k_px_active(const PxInst* __restrict__ insts, int32_t count, int64_t* __restrict__ out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-    const PxInst& I = insts[i];
-    out[i] = I.stats[(int64_t)I.round * kStats + kStActive];
-  }
-}
-
-cudaError_t launch_px_active(const Launch& L, const PxInst* insts, int32_t count, int64_t* out) {
-  if (count <= 0) return cudaSuccess;
-  k_px_active<<<(count + 255) / 256, 256, 0, L.st>>>(insts, count, out);
-  return launched("k_px_active");
-}
-
-cudaError_t launch_px_round(const Launch& L, const PxInst* insts, const int32_t* order, int32_t count,
-                            const PxParams& P, int W, bool unit, int ctas_per_sm, int64_t* queue) {
-  if (count <= 0) return cudaSuccess;
-  if (W != 1 && W != 2) return cudaErrorInvalidValue;
-  cudaError_t e = cudaMemsetAsync(queue, 0, sizeof(int64_t), L.st);
-  if (e != cudaSuccess) return e;
-  const int minb = ctas_per_sm >= 2 ? 2 : 1;
-  const void* kern = px_kernel_for(W, unit, P.unroll, minb);
-  allow_dyn_smem(kern, kPxSmem);
-  const int occ = std::max(1, occupancy(kern, kPxThreads, kPxSmem));
-  const int per_sm = std::min(minb, occ);
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(count, (int64_t)per_sm * L.num_sms));
-  void* args[] = {(void*)&insts, (void*)&order, (void*)&count, (void*)&P, (void*)&queue};
-  e = cudaLaunchKernel(kern, dim3(grid), dim3(kPxThreads), args, kPxSmem, L.st);
-  if (e != cudaSuccess) return e;
-  return launched("k_px_round");
 }
 
 }  // namespace lpgpu

@@ -191,6 +191,7 @@ struct lpgpu_session_s {
   DevBuf<int32_t> vinst, inst_boff, inst_k, over_ids;
   DevBuf<int64_t> inst_voff, inst_noff, inst_delta;
   DevBuf<int64_t> vout;  // result words of the device-side input checks
+  DevBuf<int64_t> team;  // per-team scratch of the team rounds
   // results of the last refine
   std::vector<lpgpu_round_stats> last_stats;
   // timing
@@ -335,6 +336,7 @@ struct lpgpu_session_s {
     saved_part.release(&mem);
     px.release(&mem);
     px_order.release(&mem);
+    team.release(&mem);
     px_key.clear();
     vinst.release(&mem);
     inst_voff.release(&mem);
@@ -943,6 +945,26 @@ static lpgpu_tuning session_tuning(const lpgpu_session* s) {
   return default_tuning();
 }
 
+// ---- one instance refined by one team (team.cu)
+//
+// CTAs of the team and of an SM by the number of vertices. Measured (GB300,
+// whole refine call in us, one CTA / cluster of 16 / one CTA per SM / two per
+// SM; multi-launch pipeline in brackets): 1,024 vertices 577 / 701 / - / -
+// [1,134]; 4,096: 979 / 915 / - / - [1,428]; 16,384: 2,462 / 995 / 966 / -
+// [1,377]; 131,071 (k = 64): - / 4,511 / 2,118 / 2,250 [3,370]; 1M (k = 32):
+// - / 25,213 / 5,195 / 4,899 [5,727]; 4.2M (k = 128): - / - / 12,145 / 11,361
+// [11,554].
+constexpr int kTeamUnroll = 4;
+struct TeamShape {
+  int per_sm;  // kernel build: resident CTAs per SM
+  int T;       // CTAs of the team (0: as many as are resident)
+};
+static TeamShape team_shape(int64_t n) {
+  if (n <= 2048) return {1, 1};
+  if (n <= 16384) return {1, kTeamMaxCluster};
+  return {n < (int64_t)1 << 19 ? 1 : 2, 0};
+}
+
 // Instance descriptors of the persistent rounds over the session's current
 // buffers, and the work order (rebuilt when a buffer or the order changed).
 static lpgpu_status build_px(lpgpu_session* s, int order) {
@@ -950,7 +972,7 @@ static lpgpu_status build_px(lpgpu_session* s, int order) {
   const std::vector<int64_t> key = {
       (int64_t)s->stats.p, (int64_t)s->part.p, (int64_t)s->phi.p,  (int64_t)s->conn.p,      (int64_t)s->bw.p,
       (int64_t)s->rec.p,   (int64_t)s->seg_key.p, (int64_t)s->revl.p, (int64_t)s->next_flag.p, (int64_t)s->net_off.p,
-      (int64_t)s->inets.p, (int64_t)s->lmax.p, order, s->kmax, s->k, s->W, s->n, s->m, I, s->max_we,
+      (int64_t)s->inets.p, (int64_t)s->lmax.p, (int64_t)s->list.p, order, s->kmax, s->k, s->W, s->n, s->m, I, s->max_we,
       s->unit_nets ? 1 : 0};
   if (s->px.p && s->px_key == key) return LPGPU_OK;
   std::vector<PxInst> h(I);
@@ -976,8 +998,11 @@ static lpgpu_status build_px(lpgpu_session* s, int order) {
     x.keys = s->seg_key.p + x.v0;
     x.kw = s->seg_w.p + x.v0;
     x.cand = s->revl.p + x.v0;
+    x.list = s->list.p + x.v0;
     x.net_epoch = s->net_epoch.p;
     x.stats = s->stats.p;
+    x.e0 = s->h_inst_noff[i];
+    x.e1 = s->h_inst_noff[i + 1];
     x.boff = s->batched ? s->h_inst_boff[i] : 0;
     x.k = s->batched ? s->h_inst_k[i] : s->k;
     x.kstride = s->batched ? s->kmax : s->k;
@@ -1089,12 +1114,21 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
   }
   if (cfg.flags & LPGPU_FLAG_MULTI_LAUNCH) use_px = false;
   use_px = use_px && px_ok;
+  // one instance whose form nobody chose: all rounds in one team launch
+  const bool use_team = !use_px && !s->batched && !s->has_tuning && !s->timing && s->k <= kTeamMaxK &&
+                        !(cfg.flags & LPGPU_FLAG_MULTI_LAUNCH);
   DeviceGuard g(s->device);
   s->gc_valid = false;  // refinement moves without gain-cache maintenance
   const int R = cfg.rounds, S = cfg.subrounds;
   Mem* fp = &s->mem;
   CK(s->stats.alloc(std::max(1, R) * kStats, fp));
-  if (use_px) {
+  TeamShape shape{1, 1};
+  if (use_team) {
+    shape = team_shape(s->n);
+    if (shape.T == 0) shape.T = team_resident(s->launch(), s->W, s->unit_nets, kTeamUnroll, shape.per_sm);
+    CK(s->team.alloc(team_scratch_words(s->k), fp));
+  }
+  if (use_px || use_team) {
     ps = build_px(s, tu.order);
     if (ps != LPGPU_OK) return ps;
   }
@@ -1104,7 +1138,9 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
   pxp.revert = cfg.revert;
   pxp.rollback = cfg.rollback;
   pxp.act_threshold = cfg.activation_threshold <= 0 ? INT64_MAX : cfg.activation_threshold;
-  pxp.unroll = tu.unroll;
+  pxp.unroll = use_team ? kTeamUnroll : tu.unroll;
+  pxp.kcap = s->batched ? s->kmax : s->k;
+  pxp.T = shape.T;
   const int32_t px_count = s->batched ? s->num_inst : 1;
   cudaStream_t st = s->st;
   int64_t km1_before = 0;
@@ -1136,11 +1172,21 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
       if (s->n > 0 && (e = cudaMemsetAsync(s->next_flag.p, 0, s->n, st)) != cudaSuccess) return e;
       if ((e = launch_mark_all(L, c, cfg.rebalancing)) != cudaSuccess) return e;
     }
-    if (use_px) {  // one persistent launch per round
-      for (int r = 0; r < R; ++r) {
+    if (use_px || use_team) {
+      pxp.round = 0;
+      if (use_team) {  // all rounds in one launch
+        pxp.rounds = R;
+        if ((e = launch_px_round(L, s->px.p, nullptr, 1, pxp, s->W, s->unit_nets, shape.per_sm, 1,
+                                 s->team.p,
+                                 s->scal.p + kPxQueue, s->scal.p + kError)) != cudaSuccess)
+          return e;
+      }
+      for (int r = 0; !use_team && r < R; ++r) {  // one persistent launch per round
         pxp.round = r;
+        pxp.rounds = 1;
+        pxp.activate_last = r + 1 < R;
         if ((e = launch_px_round(L, s->px.p, s->px_order.p, px_count, pxp, s->W, s->unit_nets, tu.ctas_per_sm,
-                                 s->scal.p + kPxQueue)) != cudaSuccess)
+                                 px_count, nullptr, s->scal.p + kPxQueue, s->scal.p + kError)) != cudaSuccess)
           return e;
       }
       if (s->n > 0 && (e = cudaMemsetAsync(s->next_flag.p, 0, s->n, st)) != cudaSuccess) return e;
@@ -1156,7 +1202,7 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
     if (s->n > 0 && (e = cudaMemsetAsync(s->next_flag.p, 0, s->n, st)) != cudaSuccess) return e;
     return cudaSuccess;
   };
-  if (num_nodes > 0 || tm || (cfg.flags & LPGPU_FLAG_NO_GRAPH)) {
+  if (num_nodes > 0 || tm || use_team || (cfg.flags & LPGPU_FLAG_NO_GRAPH)) {
     // direct launches: explicit node lists, and per-phase event timing
     if (tm) tm->reset();
     CK(enqueue());
@@ -1212,7 +1258,14 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
   }
   std::vector<int64_t> hs(std::max(1, R) * kStats);
   CK(cudaMemcpyAsync(hs.data(), s->stats.p, sizeof(int64_t) * hs.size(), cudaMemcpyDeviceToHost, st));
+  int64_t err = 0;
+  if (use_team) CK(cudaMemcpyAsync(&err, s->scal.p + kError, sizeof(err), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  if (err) {
+    s->has_part = false;  // the moves of an unfinished sub-round
+    set_error("a grid barrier of the refinement gave up");
+    return LPGPU_ERR_TIMEOUT;
+  }
   if (tm) {
     std::map<int, lpgpu_phase_time> acc;
     for (auto& rec : tm->recs) {
@@ -1289,7 +1342,7 @@ struct lpgpu_stepper_s {
   int num_sms = 1;
   Mem mem;
   DevBuf<PxInst> table;
-  DevBuf<int64_t> active, queue;
+  DevBuf<int64_t> active, queue;  // queue: work counter, error word
   cudaEvent_t ev = nullptr;
   std::vector<lpgpu_session*> pending;  // sessions of the launched round
   std::vector<int32_t> first;           // their first row of the table
@@ -1411,7 +1464,7 @@ lpgpu_status lpgpu_stepper_launch(lpgpu_stepper* t, lpgpu_session* const* sessio
     CK(t->table.alloc(rows, &t->mem));
     CK(t->active.alloc(rows, &t->mem));
   }
-  if (!t->queue.p) CK(t->queue.alloc(1, &t->mem));
+  if (!t->queue.p) CK(t->queue.alloc(2, &t->mem));
   if (rows > 0)
     CK(cudaMemcpyAsync(t->table.p, t->h.data(), sizeof(PxInst) * rows, cudaMemcpyHostToDevice, t->st));
   const Launch L{t->st, t->num_sms};
@@ -1428,9 +1481,13 @@ lpgpu_status lpgpu_stepper_launch(lpgpu_stepper* t, lpgpu_session* const* sessio
     P.rollback = k.rollback;
     P.act_threshold = k.act;
     P.round = -1;  // every instance runs its own round
+    P.rounds = 1;
+    P.activate_last = 1;
+    P.T = 1;
+    P.kcap = kTeamMaxK;
     P.unroll = tuned ? tu.unroll : 8;
     CK(launch_px_round(L, t->table.p + gr.second.first, nullptr, gr.second.second, P, k.W, k.unit != 0,
-                       tuned ? tu.ctas_per_sm : 2, t->queue.p));
+                       tuned ? tu.ctas_per_sm : 2, gr.second.second, nullptr, t->queue.p, t->queue.p + 1));
   }
   if (rows > 0) CK(launch_px_active(L, t->table.p, (int32_t)rows, t->active.p));
   // the sessions' later work (downloads, the next round's inputs) comes after this round

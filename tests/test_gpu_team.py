@@ -1,0 +1,78 @@
+"""Team rounds (all rounds of one instance in one launch: a CTA, a cluster or
+the whole cooperative grid) against the multi-launch pipeline, at the sizes
+where the team's shape, its chunk split or its selection changes."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+KEYS = ["active", "pins", "candidates", "moved", "reverted", "delta", "moved_pins"]
+
+
+def _refine(lp, hg, k, part, flags=0, nodes=None, **cfg):
+    with lp.Session(0) as s:
+        s.upload(hg)
+        s.set_partition(k, part, eps=0.03)
+        r = s.refine(lp.default_config(flags=flags, **cfg), nodes=nodes)
+        stats = [[x[q] for q in KEYS] for x in s.round_stats()]
+        return (s.partition(), s.block_weights(), s.pin_counts(), s.connectivity(), stats, s.metrics(),
+                (r.km1_before, r.km1_after, r.delta, r.moves, r.rounds))
+
+
+def _same(a, b):
+    for x, y in zip(a, b):
+        if isinstance(x, np.ndarray):
+            assert np.array_equal(x, y)
+        else:
+            assert x == y
+
+
+# vertices: no chunk, one partial chunk, whole chunks, one CTA / cluster / grid limits, fewer chunks than CTAs
+@pytest.mark.parametrize("n,k,weighted", [
+    (1, 1, False), (7, 3, True), (32, 2, False), (33, 4, True), (2048, 128, True), (2049, 65, False),
+    (2080, 2, True), (16384, 2, False), (16385, 33, True), (20000, 128, False), (70001, 64, True)])
+def test_team_equals_multi_launch(lp, n, k, weighted):
+    from lpgpu import gen
+    inst = gen.random_small(n + k, n=n, m=max(1, int(1.2 * n)), k=k, max_size=9, weighted=weighted) if n > 40 else None
+    if inst is None:
+        rng = np.random.default_rng(n)
+        off = np.arange(0, 3 * n + 1, 3, dtype=np.int64)
+        hg = gen.Hypergraph(n, n, off, rng.integers(0, n, 3 * n).astype(np.int32), np.ones(n, np.int32),
+                            rng.integers(1, 9, n).astype(np.int32))
+        part = rng.integers(0, k, n).astype(np.int32)
+    else:
+        hg, part = inst.hg, inst.part
+    _same(_refine(lp, hg, k, part), _refine(lp, hg, k, part, flags=lp.FLAG_MULTI_LAUNCH))
+
+
+@pytest.mark.parametrize("cfg", [dict(subrounds=1, rounds=3), dict(subrounds=64, rounds=2, rebalancing=0),
+                                 dict(subrounds=3, revert=0, rollback=0), dict(revert=0, activation_threshold=0),
+                                 dict(rollback=0, activation_threshold=3), dict(rounds=0), dict(rounds=40)])
+@pytest.mark.parametrize("n", [900, 9000, 40000])
+def test_team_options(lp, n, cfg):
+    from lpgpu import gen
+    inst = gen.random_small(n, n=n, m=n, k=8, max_size=12, hubs=3, vw_hi=30)
+    _same(_refine(lp, inst.hg, 8, inst.part, **cfg),
+          _refine(lp, inst.hg, 8, inst.part, flags=lp.FLAG_MULTI_LAUNCH, **cfg))
+
+
+def test_team_selection_sizes(lp, orc):
+    """Segments above one CTA's stage (2 blocks, one sub-round), of one key, and
+    overloaded target blocks (negative slack), against the oracle."""
+    from lpgpu import gen
+    for n, k, rounds in ((60000, 2, 2), (1500, 700 // 6, 3)):
+        inst = gen.random_small(5 + n, n=n, m=n, k=k, max_size=6, vw_hi=9)
+        part = inst.part.copy()
+        part[: n // 3] = 0  # block 0 far above its bound
+        got = _refine(lp, inst.hg, k, part, subrounds=1, rounds=rounds)
+        ref, _ = orc.lp_sync(inst.hg, k, inst.lmax, part, perfect=inst.perfect, rounds=rounds, subrounds=1, revert=1,
+                             rollback=1, zero_gain=1)
+        assert np.array_equal(got[0], ref)
+
+
+def test_team_node_list(lp):
+    from lpgpu import gen
+    inst = gen.random_small(77, n=30000, m=33000, k=16)
+    nodes = np.arange(0, 30000, 7, dtype=np.int32)
+    _same(_refine(lp, inst.hg, 16, inst.part, nodes=nodes),
+          _refine(lp, inst.hg, 16, inst.part, nodes=nodes, flags=lp.FLAG_MULTI_LAUNCH))
