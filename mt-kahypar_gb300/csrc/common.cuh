@@ -369,8 +369,8 @@ inline int64_t team_scratch_words(int kcap) { return 32 + 17 * (int64_t)kcap; }
 constexpr int kTeamMaxCluster = 16;
 
 // Runs LP rounds of `count` instances, taken in `order` (null: 0..count-1)
-// from the work queue counter `queue` (zeroed here) by `teams` teams of P.T
-// CTAs each. W: Λ words class of all instances (1, 2 or 4); unit: every net
+// from the work queue counter `queue` (zeroed here) by up to `teams` teams of
+// P.T CTAs each. W: Λ words class of all instances (1, 2 or 4); unit: every net
 // weight is 1; ctas_per_sm: the 1- or 2-CTA-per-SM build of the kernel.
 // `scratch`: teams * team_scratch_words(P.kcap) words (P.T > 1, zeroed here).
 // A grid barrier that gives up sets *err. More than kTeamMaxCluster CTAs per
@@ -378,6 +378,11 @@ constexpr int kTeamMaxCluster = 16;
 cudaError_t launch_px_round(const Launch& L, const PxInst* insts, const int32_t* order, int32_t count,
                             PxParams P, int W, bool unit, int ctas_per_sm, int teams, int64_t* scratch,
                             int64_t* queue, int64_t* err);
+// CTAs per team of a launch over `count` > 1 instances, the largest of max_n
+// vertices, with about `per_sm` CTAs' worth of teams per SM at most.
+int team_cluster(const Launch& L, int64_t count, int64_t max_n, int per_sm);
+// Teams of T CTAs that can be resident at once (an upper bound for clusters).
+int team_slots(const Launch& L, int64_t count, int T);
 // Largest number of CTAs of the kernel build that can be resident at once.
 int team_resident(const Launch& L, int W, bool unit, int unroll, int ctas_per_sm);
 // out[i]: active vertices of instance i's round `insts[i].round` (from its statistics).

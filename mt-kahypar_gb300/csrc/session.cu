@@ -1,5 +1,6 @@
 // Session management and the C ABI of liblpgpu (declared in include/lpgpu.h).
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -932,17 +933,27 @@ static bool valid_tuning(const lpgpu_tuning& t) {
 }
 
 // The session's tuning, else the first table row whose instance count and
-// mean instance size it meets, else the multi-launch form.
-static lpgpu_tuning session_tuning(const lpgpu_session* s) {
-  if (s->has_tuning) return s->tuning;
+// mean instance size it meets (true), else the default (false).
+static bool find_tuning(const lpgpu_session* s, lpgpu_tuning* t) {
+  *t = s->has_tuning ? s->tuning : default_tuning();
+  if (s->has_tuning) return true;
   const int64_t count = s->batched ? s->num_inst : 1;
   int64_t pins = 0;
   for (int64_t p : s->h_inst_pins) pins += p;
   const int64_t mean = count > 0 ? pins / count : 0;
   std::lock_guard<std::mutex> lock(g_tuning_mutex);
   for (const lpgpu_tuning_entry& e : g_tuning_table)
-    if (count >= e.min_instances && mean <= e.max_mean_pins) return e.tuning;
-  return default_tuning();
+    if (count >= e.min_instances && mean <= e.max_mean_pins) {
+      *t = e.tuning;
+      return true;
+    }
+  return false;
+}
+
+static lpgpu_tuning session_tuning(const lpgpu_session* s) {
+  lpgpu_tuning t;
+  find_tuning(s, &t);
+  return t;
 }
 
 // ---- one instance refined by one team (team.cu)
@@ -954,16 +965,31 @@ static lpgpu_tuning session_tuning(const lpgpu_session* s) {
 // [1,377]; 131,071 (k = 64): - / 4,511 / 2,118 / 2,250 [3,370]; 1M (k = 32):
 // - / 25,213 / 5,195 / 4,899 [5,727]; 4.2M (k = 128): - / - / 12,145 / 11,361
 // [11,554].
-constexpr int kTeamUnroll = 4;
 struct TeamShape {
   int per_sm;  // kernel build: resident CTAs per SM
+  int unroll;
   int T;       // CTAs of the team (0: as many as are resident)
 };
-static TeamShape team_shape(int64_t n) {
-  if (n <= 2048) return {1, 1};
-  if (n <= 16384) return {1, kTeamMaxCluster};
-  return {n < (int64_t)1 << 19 ? 1 : 2, 0};
+static TeamShape team_shape(int64_t n, int num_sms, int in_flight) {
+  if (n <= 2048) return {1, 4, 1};
+  if (n <= 16384) return {1, 4, kTeamMaxCluster};
+  if (in_flight > 1) return {2, 4, 2 * num_sms / std::min(in_flight, 4)};
+  return {n < (int64_t)1 << 19 ? 1 : 2, 4, 0};
 }
+
+// Refine calls in progress per device: a cooperative grid over the whole GPU
+// keeps every other session's kernels out until it ends, so sessions that are
+// refined from several threads at once take an equal share of the SMs each (64
+// registers per thread, so that two CTAs fit an SM). 131,071 vertices, k = 64,
+// 1 / 2 / 4 threads, us per refine: whole grid 2,110 / 2,034 / 2,014, shares
+// 2,110 / 1,247 / 763 (multi-launch pipeline 3,508 / 1,952 / 1,154).
+static std::atomic<int> g_in_flight[16];
+struct InFlight {
+  std::atomic<int>& c;
+  const int now;
+  explicit InFlight(int device) : c(g_in_flight[device & 15]), now(c.fetch_add(1) + 1) {}
+  ~InFlight() { c.fetch_sub(1); }
+};
 
 // Instance descriptors of the persistent rounds over the session's current
 // buffers, and the work order (rebuilt when a buffer or the order changed).
@@ -1104,31 +1130,45 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
     return invalid("LPGPU_FLAG_PERSISTENT and LPGPU_FLAG_MULTI_LAUNCH exclude each other");
   for (int64_t i = 0; i < num_nodes; ++i)
     if (nodes[i] < 0 || nodes[i] >= s->n) return invalid("refinement node out of range");
-  // persistent rounds: forced by the flag, or chosen by the tuning when eligible
-  const lpgpu_tuning tu = session_tuning(s);
-  const bool px_ok = num_nodes == 0 && (s->batched ? s->kmax : s->k) <= kPxMaxK;
-  bool use_px = tu.mode == LPGPU_MODE_PERSISTENT;
+  // the team rounds, forced by the flag, chosen by the tuning or, where no tuning
+  // applies, by default; the multi-launch pipeline otherwise (k above the team
+  // kernel's, per-phase timing, forced or tuned)
+  lpgpu_tuning tu;
+  const bool tuned = find_tuning(s, &tu);
+  const int kmax = s->batched ? s->kmax : s->k;
+  const bool px_ok = num_nodes == 0 && kmax <= kPxMaxK;
+  bool use_team = tuned ? tu.mode == LPGPU_MODE_PERSISTENT && px_ok : kmax <= kTeamMaxK && !s->timing;
   if (cfg.flags & LPGPU_FLAG_PERSISTENT) {
     if (!px_ok) return invalid("persistent rounds need every k <= 64 and no refinement node list");
-    use_px = true;
+    use_team = true;
   }
-  if (cfg.flags & LPGPU_FLAG_MULTI_LAUNCH) use_px = false;
-  use_px = use_px && px_ok;
-  // one instance whose form nobody chose: all rounds in one team launch
-  const bool use_team = !use_px && !s->batched && !s->has_tuning && !s->timing && s->k <= kTeamMaxK &&
-                        !(cfg.flags & LPGPU_FLAG_MULTI_LAUNCH);
+  if (cfg.flags & LPGPU_FLAG_MULTI_LAUNCH) use_team = false;
   DeviceGuard g(s->device);
+  const InFlight in_flight(s->device);
   s->gc_valid = false;  // refinement moves without gain-cache maintenance
   const int R = cfg.rounds, S = cfg.subrounds;
   Mem* fp = &s->mem;
   CK(s->stats.alloc(std::max(1, R) * kStats, fp));
-  TeamShape shape{1, 1};
+  const int32_t px_count = s->batched ? s->num_inst : 1;
+  TeamShape shape{2, 8, 1};
   if (use_team) {
-    shape = team_shape(s->n);
-    if (shape.T == 0) shape.T = team_resident(s->launch(), s->W, s->unit_nets, kTeamUnroll, shape.per_sm);
-    CK(s->team.alloc(team_scratch_words(s->k), fp));
-  }
-  if (use_px || use_team) {
+    const Launch L = s->launch();
+    if (px_count == 1) {
+      shape = team_shape(s->n, L.num_sms, in_flight.now);
+    } else {
+      int64_t max_n = 0;
+      for (int32_t i = 0; i < px_count; ++i) max_n = std::max(max_n, s->h_inst_voff[i + 1] - s->h_inst_voff[i]);
+      shape.T = team_cluster(L, px_count, max_n, 5);
+    }
+    if (tuned && tu.mode == LPGPU_MODE_PERSISTENT) {
+      shape.per_sm = tu.ctas_per_sm;
+      shape.unroll = tu.unroll;
+    }
+    if (shape.T == 0 || shape.T > kTeamMaxCluster) {
+      const int most = team_resident(L, s->W, s->unit_nets, shape.unroll, shape.per_sm);
+      shape.T = shape.T == 0 ? most : std::min(shape.T, most);
+    }
+    if (shape.T > 1) CK(s->team.alloc(team_scratch_words(kmax) * team_slots(L, px_count, shape.T), fp));
     ps = build_px(s, tu.order);
     if (ps != LPGPU_OK) return ps;
   }
@@ -1138,10 +1178,11 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
   pxp.revert = cfg.revert;
   pxp.rollback = cfg.rollback;
   pxp.act_threshold = cfg.activation_threshold <= 0 ? INT64_MAX : cfg.activation_threshold;
-  pxp.unroll = use_team ? kTeamUnroll : tu.unroll;
-  pxp.kcap = s->batched ? s->kmax : s->k;
+  pxp.round = 0;
+  pxp.rounds = R;
+  pxp.unroll = shape.unroll;
+  pxp.kcap = kmax;
   pxp.T = shape.T;
-  const int32_t px_count = s->batched ? s->num_inst : 1;
   cudaStream_t st = s->st;
   int64_t km1_before = 0;
   lpgpu_status ms = read_metrics(s, &km1_before, nullptr);
@@ -1155,7 +1196,8 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
   }
   PhaseTimer* tm = s->timing ? &s->timer : nullptr;
   // The whole refine is a fixed sequence of launches whose element counts live
-  // in device memory, so it is captured once as a CUDA graph and replayed.
+  // in device memory: the multi-launch form is captured once as a CUDA graph and
+  // replayed.
   auto enqueue = [&]() -> cudaError_t {
     cudaError_t e;
     if ((e = cudaMemsetAsync(s->stats.p, 0, sizeof(int64_t) * std::max(1, R) * kStats, st)) != cudaSuccess) return e;
@@ -1172,23 +1214,11 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
       if (s->n > 0 && (e = cudaMemsetAsync(s->next_flag.p, 0, s->n, st)) != cudaSuccess) return e;
       if ((e = launch_mark_all(L, c, cfg.rebalancing)) != cudaSuccess) return e;
     }
-    if (use_px || use_team) {
-      pxp.round = 0;
-      if (use_team) {  // all rounds in one launch
-        pxp.rounds = R;
-        if ((e = launch_px_round(L, s->px.p, nullptr, 1, pxp, s->W, s->unit_nets, shape.per_sm, 1,
-                                 s->team.p,
-                                 s->scal.p + kPxQueue, s->scal.p + kError)) != cudaSuccess)
-          return e;
-      }
-      for (int r = 0; !use_team && r < R; ++r) {  // one persistent launch per round
-        pxp.round = r;
-        pxp.rounds = 1;
-        pxp.activate_last = r + 1 < R;
-        if ((e = launch_px_round(L, s->px.p, s->px_order.p, px_count, pxp, s->W, s->unit_nets, tu.ctas_per_sm,
-                                 px_count, nullptr, s->scal.p + kPxQueue, s->scal.p + kError)) != cudaSuccess)
-          return e;
-      }
+    if (use_team) {  // all rounds in one launch
+      if ((e = launch_px_round(L, s->px.p, s->px_order.p, px_count, pxp, s->W, s->unit_nets, shape.per_sm,
+                               team_slots(L, px_count, shape.T), s->team.p, s->scal.p + kPxQueue,
+                               s->scal.p + kError)) != cudaSuccess)
+        return e;
       if (s->n > 0 && (e = cudaMemsetAsync(s->next_flag.p, 0, s->n, st)) != cudaSuccess) return e;
       return cudaSuccess;
     }
@@ -1203,31 +1233,20 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
     return cudaSuccess;
   };
   if (num_nodes > 0 || tm || use_team || (cfg.flags & LPGPU_FLAG_NO_GRAPH)) {
-    // direct launches: explicit node lists, and per-phase event timing
+    // direct launches: explicit node lists, per-phase event timing, and the few of the team form
     if (tm) tm->reset();
     CK(enqueue());
   } else {
     // key: every pointer and parameter baked into the captured launches
     struct Key {
       RoundCtx c;
-      int R, S, timing, px;
+      int R, S;
       int64_t* p[1];
-      lpgpu_tuning tu;
-      const void* px_ptr[2];
-      int32_t px_count;
     } key;
     std::memset(&key, 0, sizeof(key));
     key.c = c;
     key.R = R;
     key.S = S;
-    key.timing = 0;
-    key.px = use_px ? 1 : 0;
-    if (use_px) {
-      key.tu = tu;
-      key.px_ptr[0] = s->px.p;
-      key.px_ptr[1] = s->px_order.p;
-      key.px_count = px_count;
-    }
     key.p[0] = s->bin_cnt.p;
     std::vector<unsigned char> kb(reinterpret_cast<unsigned char*>(&key),
                                   reinterpret_cast<unsigned char*>(&key) + sizeof(key));
@@ -1342,7 +1361,10 @@ struct lpgpu_stepper_s {
   int num_sms = 1;
   Mem mem;
   DevBuf<PxInst> table;
-  DevBuf<int64_t> active, queue;  // queue: work counter, error word
+  DevBuf<int64_t> active, queue;  // queue: per group of a round its work counter and error word
+  DevBuf<int64_t> team;           // scratch of the teams, group after group
+  cudaStream_t side[3] = {};      // further groups of a round run beside the first
+  cudaEvent_t side_ev[3] = {};
   cudaEvent_t ev = nullptr;
   std::vector<lpgpu_session*> pending;  // sessions of the launched round
   std::vector<int32_t> first;           // their first row of the table
@@ -1392,11 +1414,18 @@ lpgpu_status lpgpu_stepper_destroy(lpgpu_stepper* t) {
   if (!t) return LPGPU_OK;
   {
     DeviceGuard g(t->device);
+    for (cudaStream_t x : t->side)
+      if (x) cudaStreamSynchronize(x);
     cudaStreamSynchronize(t->st);
     t->table.release(&t->mem);
     t->active.release(&t->mem);
     t->queue.release(&t->mem);
+    t->team.release(&t->mem);
     cudaStreamSynchronize(t->st);
+    for (int i = 0; i < 3; ++i) {
+      if (t->side[i]) cudaStreamDestroy(t->side[i]);
+      if (t->side_ev[i]) cudaEventDestroy(t->side_ev[i]);
+    }
     cudaEventDestroy(t->ev);
     cudaMemPoolDestroy(t->mem.pool);
     cudaStreamDestroy(t->st);
@@ -1446,6 +1475,9 @@ lpgpu_status lpgpu_stepper_launch(lpgpu_stepper* t, lpgpu_session* const* sessio
   std::vector<std::pair<Group, std::pair<int32_t, int32_t>>> ranges;  // group, (first row, rows)
   for (auto& kv : groups) {
     const int32_t beg = (int32_t)t->h.size();
+    // largest first: the longest jobs start first on the work queue
+    std::stable_sort(kv.second.begin(), kv.second.end(),
+                     [&](int32_t a, int32_t b) { return sessions[a]->P > sessions[b]->P; });
     for (int32_t i : kv.second) {
       lpgpu_session* s = sessions[i];
       t->first[i] = (int32_t)t->h.size();
@@ -1464,11 +1496,26 @@ lpgpu_status lpgpu_stepper_launch(lpgpu_stepper* t, lpgpu_session* const* sessio
     CK(t->table.alloc(rows, &t->mem));
     CK(t->active.alloc(rows, &t->mem));
   }
-  if (!t->queue.p) CK(t->queue.alloc(2, &t->mem));
   if (rows > 0)
     CK(cudaMemcpyAsync(t->table.p, t->h.data(), sizeof(PxInst) * rows, cudaMemcpyHostToDevice, t->st));
   const Launch L{t->st, t->num_sms};
-  for (const auto& gr : ranges) {
+  // the groups of a round run side by side, so the team size follows their total;
+  // all teams are resident at once, which leaves room for other sessions' work
+  int64_t max_n = 0;
+  for (const PxInst& x : t->h) max_n = std::max(max_n, x.v1 - x.v0);
+  const int T = rows > 0 ? team_cluster(L, (int64_t)rows, max_n, 2) : 1;
+  const int64_t words = team_scratch_words(kPxMaxK);
+  const size_t G = ranges.size();
+  if (t->queue.count < 2 * G) CK(t->queue.alloc(2 * G, &t->mem));
+  if (T > 1) {
+    int64_t need = 0;
+    for (const auto& gr : ranges) need += words * team_slots(L, gr.second.second, T);
+    if ((int64_t)t->team.count < need) CK(t->team.alloc((size_t)need, &t->mem));
+  }
+  if (G > 1) CK(cudaEventRecord(t->ev, t->st));  // the table and the sessions' work
+  int64_t used = 0;
+  for (size_t gi = 0; gi < G; ++gi) {
+    const auto& gr = ranges[gi];
     const Group& k = gr.first;
     // the kernel build of the group's first session's tuning when that is a
     // persistent one, else 2 CTAs per SM with unroll 8
@@ -1483,11 +1530,27 @@ lpgpu_status lpgpu_stepper_launch(lpgpu_stepper* t, lpgpu_session* const* sessio
     P.round = -1;  // every instance runs its own round
     P.rounds = 1;
     P.activate_last = 1;
-    P.T = 1;
-    P.kcap = kTeamMaxK;
+    P.T = T;
+    P.kcap = kPxMaxK;
     P.unroll = tuned ? tu.unroll : 8;
-    CK(launch_px_round(L, t->table.p + gr.second.first, nullptr, gr.second.second, P, k.W, k.unit != 0,
-                       tuned ? tu.ctas_per_sm : 2, gr.second.second, nullptr, t->queue.p, t->queue.p + 1));
+    Launch Lg = L;
+    const int lane = (int)(gi % 4) - 1;  // -1: the stepper's own stream
+    if (lane >= 0) {
+      if (!t->side[lane]) {
+        CK(cudaStreamCreateWithFlags(&t->side[lane], cudaStreamNonBlocking));
+        CK(cudaEventCreateWithFlags(&t->side_ev[lane], cudaEventDisableTiming));
+      }
+      Lg.st = t->side[lane];
+      CK(cudaStreamWaitEvent(Lg.st, t->ev, 0));
+    }
+    CK(launch_px_round(Lg, t->table.p + gr.second.first, nullptr, gr.second.second, P, k.W, k.unit != 0,
+                       tuned ? tu.ctas_per_sm : 2, team_slots(L, gr.second.second, T),
+                       T > 1 ? t->team.p + used : nullptr, t->queue.p + 2 * gi, t->queue.p + 2 * gi + 1));
+    if (T > 1) used += words * team_slots(L, gr.second.second, T);
+  }
+  for (size_t i = 0; i + 1 < G && i < 3; ++i) {  // the round ends with its last group
+    CK(cudaEventRecord(t->side_ev[i], t->side[i]));
+    CK(cudaStreamWaitEvent(t->st, t->side_ev[i], 0));
   }
   if (rows > 0) CK(launch_px_active(L, t->table.p, (int32_t)rows, t->active.p));
   // the sessions' later work (downloads, the next round's inputs) comes after this round
@@ -1777,6 +1840,7 @@ int64_t lpgpu_estimate_footprint(int64_t n, int64_t m, int64_t P, int32_t k, int
   b += 4 * m + 4 * n + n + n + 16 * n + 8 * n + 4 * n + 8 * n;         // epoch, list, flags, status, rec, seg, queues
   b += 8 * (2 * kMaxSubrounds + 1) + 8 * 2 * kMaxSubrounds * kDegClasses;  // sub-round bins
   b += 8 * (scan_tmp_elems(n + 1) + 1);
+  b += 8 * team_scratch_words(std::min(std::max(1, k), kTeamMaxK));
   b += 4 * n + 4 * m * (int64_t)k + 8 * m * W;                         // part, Φ, Λ + Λ1
   b += 8 * (3 * k + 7 * k + 1 + 2 * k) + 2 * k + 8 * 64 + 8 * 8;       // per-block, stats, scalars
   return b;
