@@ -359,6 +359,7 @@ struct PxParams {
   int32_t unroll;       // incidences per lane step of the sweep (4 or 8; W = 4: always 4)
   int32_t T;            // CTAs per team
   int32_t kcap;         // largest k of the launch
+  int32_t resident;     // bytes of shared memory per CTA for the instance's own arrays (set by the launch)
 };
 
 // int64 words of global scratch one team of more than one CTA needs.
@@ -374,10 +375,16 @@ constexpr int kTeamMaxCluster = 16;
 // weight is 1; ctas_per_sm: the 1- or 2-CTA-per-SM build of the kernel.
 // `scratch`: teams * team_scratch_words(P.kcap) words (P.T > 1, zeroed here).
 // A grid barrier that gives up sets *err. More than kTeamMaxCluster CTAs per
-// team need count == 1.
+// team need count == 1. `own_bytes`: shared memory a CTA's part of the largest
+// instance wants (team_own_bytes).
 cudaError_t launch_px_round(const Launch& L, const PxInst* insts, const int32_t* order, int32_t count,
                             PxParams P, int W, bool unit, int ctas_per_sm, int teams, int64_t* scratch,
-                            int64_t* queue, int64_t* err);
+                            int64_t* queue, int64_t* err, int64_t own_bytes);
+// Bytes a CTA of a team of T keeps of an instance, on average: its vertices'
+// offsets, weights, blocks and list entries and their incident nets; alone also
+// the records and pin counts.
+int64_t team_own_bytes(int64_t n, int64_t m, int64_t pins, int T, int k, int W, bool phi16,
+                       int per_sm);
 // CTAs per team of a launch over `count` > 1 instances, the largest of max_n
 // vertices, with about `per_sm` CTAs' worth of teams per SM at most.
 int team_cluster(const Launch& L, int64_t count, int64_t max_n, int per_sm);

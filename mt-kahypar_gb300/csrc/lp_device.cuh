@@ -459,9 +459,9 @@ __device__ __forceinline__ void lv_decide(const RoundCtx& c, const uint32_t (&cn
 }
 
 // Best move of one vertex by its own lane (accumulate all incidences, decide);
-// U incidences per step have their gathers in flight together, with AHEAD also
-// the next step's net ids; NC as in load_words.
-template <int W, bool UNIT, int PL, int U = LPGPU_LV_UNROLL, bool NC = true, bool AHEAD = false>
+// U incidences per step have their gathers in flight together; NC as in
+// load_words.
+template <int W, bool UNIT, int PL, int U = LPGPU_LV_UNROLL, bool NC = true>
 __device__ __forceinline__ void lv_vertex(const RoundCtx& c, int64_t o0, int d, int from, int wv, int bo,
                                           int inst, bool batched, int zero_gain,
                                           const uint32_t* __restrict__ s_fmask, const int* __restrict__ s_slack,
@@ -477,13 +477,11 @@ __device__ __forceinline__ void lv_vertex(const RoundCtx& c, int64_t o0, int d, 
   const int fw = from >> 5;
   const uint32_t fbit = 1u << (from & 31);
   int32_t ee[U];
-  if constexpr (AHEAD) lv_ids<U, NC>(c, o0, d, 0, ee);
   for (int j = 0; j < d; j += U) {
     uint32_t wd[U][W], l1[U];
     int we[U];
-    if constexpr (!AHEAD) lv_ids<U, NC>(c, o0, d, j, ee);
+    lv_ids<U, NC>(c, o0, d, j, ee);
     lv_records<W, UNIT, U, NC>(c, ee, fw, fbit, wd, l1, we);
-    if constexpr (AHEAD) lv_ids<U, NC>(c, o0, d, j + U, ee);  // in flight with the records
     lv_add<W, UNIT, PL, U>(wd, l1, we, fbit, cnt, internal);
   }
   lv_decide<W, PL>(c, cnt, internal, from, wv, bo, inst, batched, zero_gain, s_fmask, s_slack, s_bw, s_perf, to,

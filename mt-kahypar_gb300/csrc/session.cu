@@ -1151,6 +1151,7 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
   CK(s->stats.alloc(std::max(1, R) * kStats, fp));
   const int32_t px_count = s->batched ? s->num_inst : 1;
   TeamShape shape{2, 8, 1};
+  int64_t own_bytes = 0;
   if (use_team) {
     const Launch L = s->launch();
     if (px_count == 1) {
@@ -1168,6 +1169,10 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
       const int most = team_resident(L, s->W, s->unit_nets, shape.unroll, shape.per_sm);
       shape.T = shape.T == 0 ? most : std::min(shape.T, most);
     }
+    for (int32_t i = 0; i < px_count; ++i)
+      own_bytes = std::max(own_bytes, team_own_bytes(s->h_inst_voff[i + 1] - s->h_inst_voff[i],
+                                                     s->h_inst_noff[i + 1] - s->h_inst_noff[i], s->h_inst_pins[i],
+                                                     shape.T, kmax, s->W, s->phi16(), shape.per_sm));
     if (shape.T > 1) CK(s->team.alloc(team_scratch_words(kmax) * team_slots(L, px_count, shape.T), fp));
     ps = build_px(s, tu.order);
     if (ps != LPGPU_OK) return ps;
@@ -1217,7 +1222,7 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
     if (use_team) {  // all rounds in one launch
       if ((e = launch_px_round(L, s->px.p, s->px_order.p, px_count, pxp, s->W, s->unit_nets, shape.per_sm,
                                team_slots(L, px_count, shape.T), s->team.p, s->scal.p + kPxQueue,
-                               s->scal.p + kError)) != cudaSuccess)
+                               s->scal.p + kError, own_bytes)) != cudaSuccess)
         return e;
       if (s->n > 0 && (e = cudaMemsetAsync(s->next_flag.p, 0, s->n, st)) != cudaSuccess) return e;
       return cudaSuccess;
@@ -1504,6 +1509,13 @@ lpgpu_status lpgpu_stepper_launch(lpgpu_stepper* t, lpgpu_session* const* sessio
   int64_t max_n = 0;
   for (const PxInst& x : t->h) max_n = std::max(max_n, x.v1 - x.v0);
   const int T = rows > 0 ? team_cluster(L, (int64_t)rows, max_n, 2) : 1;
+  int64_t own_bytes = 0;
+  for (int32_t i = 0; i < count; ++i) {
+    const lpgpu_session* s = sessions[i];
+    for (size_t j = 0; j < s->h_px.size(); ++j)
+      own_bytes = std::max(own_bytes, team_own_bytes(s->h_px[j].v1 - s->h_px[j].v0, s->h_px[j].e1 - s->h_px[j].e0,
+                                                     s->h_inst_pins[j], T, s->h_px[j].kstride, s->W, s->phi16(), 2));
+  }
   const int64_t words = team_scratch_words(kPxMaxK);
   const size_t G = ranges.size();
   if (t->queue.count < 2 * G) CK(t->queue.alloc(2 * G, &t->mem));
@@ -1545,7 +1557,7 @@ lpgpu_status lpgpu_stepper_launch(lpgpu_stepper* t, lpgpu_session* const* sessio
     }
     CK(launch_px_round(Lg, t->table.p + gr.second.first, nullptr, gr.second.second, P, k.W, k.unit != 0,
                        tuned ? tu.ctas_per_sm : 2, team_slots(L, gr.second.second, T),
-                       T > 1 ? t->team.p + used : nullptr, t->queue.p + 2 * gi, t->queue.p + 2 * gi + 1));
+                       T > 1 ? t->team.p + used : nullptr, t->queue.p + 2 * gi, t->queue.p + 2 * gi + 1, own_bytes));
     if (T > 1) used += words * team_slots(L, gr.second.second, T);
   }
   for (size_t i = 0; i + 1 < G && i < 3; ++i) {  // the round ends with its last group

@@ -25,6 +25,8 @@
 // instance's scratch arrays. CTAs meet in per-block totals and selection
 // segments (global memory) only.
 #include <algorithm>
+#include <cstddef>
+#include <type_traits>
 
 #include "lp_device.cuh"
 
@@ -70,8 +72,32 @@ static_assert(kTeamArea >= kWarpSelArea, "every warp's selection histogram fits 
 #endif
 constexpr int kTeamWarpSelKeys = LPGPU_PX_WARP_SEL;
 
+// Candidates whose records stay in shared memory (the others in I.rec).
+constexpr int kCandCache = 512;
+
+// The 1-CTA-per-SM builds (OWN) keep a CTA's part of the instance in shared
+// memory; the 2-CTA builds have 64 registers, where the code for it costs more
+// than it gives (4.2M vertices 11,360 us without, 12,210 us with it).
+//
+// A CTA's part of the instance. Its vertices are named by their index li in
+// the CTA (32 per chunk). off / wv / part / list / inets are copies in shared
+// memory when they fit (off null: not resident): nobody else reads or changes
+// them, so a sweep's chain of dependent accesses is one L2 trip (the net's
+// record) instead of four. Whole refine, without -> with (GB300, us): 1,024
+// vertices 577 -> 544, 16,384 996 -> 912, 65,536 (k = 32) 1,810 -> 1,708,
+// 131,071 (k = 64) 2,117 -> 2,032, 262,144 1,409 -> 1,352.
+struct TeamPart {
+  int4* rec;
+  uint8_t* status;
+  int32_t *list, *heavy, *kept;
+  int32_t *off, *wv, *part;
+  int len, vbits, chunks, own_nets;  // own_nets: bit 0 the records, 1 the pin counts are in shared memory
+};
+
 struct TeamShared {
   PxInst I;
+  TeamPart V;
+  RoundCtx c;
   int64_t bw[kTeamMaxK], lmax[kTeamMaxK], perf[kTeamMaxK];
   int64_t tot_cnt[kTeamMaxK];  // candidates of the team per block
   int64_t seg[kTeamMaxK];
@@ -95,8 +121,14 @@ struct TeamShared {
   int nover, any;  // any: bit 0 a target block overflows, 1 a source block may empty, 2 a candidate exists
   int sel_bin, sel_n;
   int ncand, nrev, grev, nkept, rolled, tile, nheavy, nhuge, item, abort;
+  // builds with resident parts only (kTeamShortAt: the end for the others)
+  alignas(16) int4 crec[kCandCache];  // (li, gain, to | from << 16, weight)
+  uint8_t cst[kCandCache];            // 1 committed, 2 reverted, 3 rolled back
 };
-constexpr size_t kTeamSmem = ((kTeamArea + 15) & ~size_t(15)) + sizeof(TeamShared);
+constexpr size_t kTeamSharedAt = (kTeamArea + 15) & ~size_t(15);
+constexpr size_t kTeamOwnAt = (kTeamSharedAt + sizeof(TeamShared) + 15) & ~size_t(15);  // the CTA's part of the instance
+constexpr size_t kTeamSmem = kTeamOwnAt;
+constexpr size_t kTeamSmemShort = kTeamSharedAt + offsetof(TeamShared, crec);
 
 struct Team {
   TeamGlob G;
@@ -144,24 +176,6 @@ __device__ __forceinline__ bool team_sync(Team& tm, TeamShared& s) {
   do {                                   \
     if (!team_sync(tm, s)) return false; \
   } while (0)
-
-__device__ __forceinline__ RoundCtx team_ctx(const PxInst& I) {
-  RoundCtx c{};
-  c.vtx_off = I.vtx_off;
-  c.inets = I.inets;
-  c.w_v = I.w_v;
-  c.w_e = I.w_e;
-  c.part = I.part;
-  c.phi = I.phi;
-  c.conn = I.conn;
-  c.k = I.k;
-  c.W = I.W;
-  c.kmax = I.kstride;
-  c.unit_nets = I.unit_nets;
-  c.phi16 = I.phi16;
-  c.max_we = I.max_we;
-  return c;
-}
 
 // (gain, local vertex) as one integer in the order of move_key, without the
 // constant bits between the two fields: the selection's first pass then covers
@@ -481,17 +495,110 @@ __device__ __forceinline__ void team_select(const PxInst& I, Team& tm, TeamShare
   }
 }
 
+__device__ __forceinline__ int team_lv(const Team& tm, int li) {
+  return (((li >> kChunkShift) * tm.T + tm.rank) << kChunkShift) | (li & 31);
+}
+template <bool OWN>
+__device__ __forceinline__ void team_degree(const Team& tm, const TeamShared& s, int li, int64_t& o0, int64_t& d) {
+  if (OWN && s.V.off) {
+    o0 = s.V.off[li];
+    d = s.V.off[li + 1] - o0;
+  } else {
+    const int64_t v = s.I.v0 + team_lv(tm, li);
+    o0 = s.I.vtx_off[v];
+    d = s.I.vtx_off[v + 1] - o0;
+  }
+}
+template <bool OWN>
+__device__ __forceinline__ void team_vertex(const Team& tm, const TeamShared& s, int li, int64_t& o0, int64_t& d,
+                                            int& from, int& wv) {
+  team_degree<OWN>(tm, s, li, o0, d);
+  if (OWN && s.V.off) {
+    from = s.V.part[li];
+    wv = s.V.wv[li];
+  } else {
+    const int64_t v = s.I.v0 + team_lv(tm, li);
+    from = s.I.part[v] - s.I.boff;
+    wv = s.I.w_v[v];
+  }
+}
+
+// Candidate i of the CTA's list and its status.
+template <bool OWN>
+__device__ __forceinline__ int4 team_rec(const TeamShared& s, int i) { return OWN && i < kCandCache ? s.crec[i] : s.V.rec[i]; }
+template <bool OWN>
+__device__ __forceinline__ int team_status(const TeamShared& s, int i) {
+  return OWN && i < kCandCache ? s.cst[i] : s.V.status[i];
+}
+template <bool OWN>
+__device__ __forceinline__ void team_set_status(TeamShared& s, int i, int x) {
+  (OWN && i < kCandCache ? s.cst : s.V.status)[i] = (uint8_t)x;
+}
+
 // Appends the warp's candidate moves (lanes with `has`) to the CTA's list and
 // adds them to its per-block totals.
-__device__ __forceinline__ void team_candidates(TeamShared& s, int4* rec, bool has, int lv, int gain, int from, int to,
-                                                int wv) {
+template <bool OWN>
+__device__ __forceinline__ void team_candidates(TeamShared& s, bool has, int li, int gain, int from, int to, int wv) {
   const int slot = flat_append_to(&s.ncand, has);
   if (has) {
-    rec[slot] = make_int4(lv, gain, to | (from << 16), wv);
+    (OWN && slot < kCandCache ? s.crec : s.V.rec)[slot] = make_int4(li, gain, to | (from << 16), wv);
     atomicAdd(&s.in_w[to], (ull)(int64_t)wv);
     atomicAdd(&s.in_cnt[to], 1u);
     atomicAdd(&s.out_w[from], (ull)(int64_t)wv);
   }
+}
+
+// cnt += x (bit-sliced).
+template <int PL>
+__device__ __forceinline__ void lv_add_counters(uint32_t (&cnt)[PL], const uint32_t (&x)[PL]) {
+  uint32_t cy = 0;
+#pragma unroll
+  for (int p = 0; p < PL; ++p) {
+    const uint32_t t = cnt[p];
+    cnt[p] = t ^ x[p] ^ cy;
+    cy = (t & x[p]) | (cy & (t ^ x[p]));
+  }
+}
+
+// Best move of a vertex by the G = 1, 2 or 4 lanes of its group (lane `sub`
+// takes every G-th step of U incidences; the counters are summed over the
+// group, so every lane decides alike). All lanes of the warp take part; d = 0:
+// nothing to evaluate.
+template <int W, bool UNIT, int PL, int U>
+__device__ __forceinline__ void team_lv_vertex(const RoundCtx& c, const TeamShared& s, int64_t o0, int d, int from,
+                                               int wv, int G, int sub, int zero_gain, int& to, int& gain) {
+  uint32_t cnt[W][PL];
+#pragma unroll
+  for (int t = 0; t < W; ++t)
+#pragma unroll
+    for (int p = 0; p < PL; ++p) cnt[t][p] = 0;
+  int internal = 0;
+  const int fw = from >> 5;
+  const uint32_t fbit = 1u << (from & 31);
+  int32_t ee[U];
+  lv_ids<U, false>(c, o0, d, U * sub, ee);
+  for (int j = U * sub; j < d; j += U * G) {
+    uint32_t wd[U][W], l1[U];
+    int we[U];
+    lv_records<W, UNIT, U, false>(c, ee, fw, fbit, wd, l1, we);
+    lv_ids<U, false>(c, o0, d, j + U * G, ee);  // in flight with the records
+    lv_add<W, UNIT, PL, U>(wd, l1, we, fbit, cnt, internal);
+  }
+  __syncwarp();
+  for (int g = 1; g < G; g <<= 1) {
+#pragma unroll
+    for (int t = 0; t < W; ++t) {
+      uint32_t x[PL];
+#pragma unroll
+      for (int p = 0; p < PL; ++p) x[p] = __shfl_xor_sync(FULLMASK, cnt[t][p], g);
+      lv_add_counters<PL>(cnt[t], x);
+    }
+    internal += __shfl_xor_sync(FULLMASK, internal, g);
+  }
+  bool border = false;
+  if (d > 0)
+    lv_decide<W, PL>(c, cnt, internal, from, wv, 0, 0, false, zero_gain, s.fmask, s.slack, s.bw, s.perf, to, gain,
+                     border);
 }
 
 // Penalties of the blocks 32 t + lane over the 32-incidence windows start,
@@ -530,40 +637,39 @@ __device__ __forceinline__ void team_windows(const RoundCtx& c, int64_t o0, int 
   }
 }
 
-template <int W, bool UNIT>
-__device__ __forceinline__ void team_heavy_decide(const PxInst& I, const PxParams& P, TeamShared& s, int4* rec, int lv,
-                                                  int from, int wv, int internal, const int (&pen)[W]) {
-  const int lane = lane_id();
+template <int W, bool UNIT, bool OWN>
+__device__ __forceinline__ void team_heavy_decide(const PxParams& P, TeamShared& s, int li, int from, int wv,
+                                                  int internal, const int (&pen)[W]) {
+  const int lane = lane_id(), k = s.I.k;
   int sl[W];
 #pragma unroll
-  for (int t = 0; t < W; ++t) sl[t] = 32 * t + lane < I.k ? s.slack[32 * t + lane] : -1;
+  for (int t = 0; t < W; ++t) sl[t] = 32 * t + lane < k ? s.slack[32 * t + lane] : -1;
   int to = from, gain = 0;
-  decide<W, UNIT>(I.k, from, wv, internal, P.zero_gain, pen, sl, s.bw, s.perf, to, gain);
-  team_candidates(s, rec, lane == 0 && to != from, lv, gain, from, to, wv);
+  decide<W, UNIT>(k, from, wv, internal, P.zero_gain, pen, sl, s.bw, s.perf, to, gain);
+  team_candidates<OWN>(s, lane == 0 && to != from, li, gain, from, to, wv);
 }
 
 // Heavy vertices (summed net weight beyond the lane counters): a warp each up
 // to kTeamHuge incidences, the whole CTA above.
 constexpr int kTeamHuge = 1024;
-template <int W, bool UNIT>
-__device__ void team_heavy(const PxInst& I, const PxParams& P, const RoundCtx& c, TeamShared& s, int4* rec,
-                           const int32_t* heavy, int len) {
+template <int W, bool UNIT, bool OWN>
+__device__ void team_heavy(const PxParams& P, const RoundCtx& c, const Team& tm, TeamShared& s) {
   const int lane = lane_id(), wid = threadIdx.x >> 5;
   const int nheavy = s.nheavy, nhuge = s.nhuge;
+  int64_t o0, d;
+  int from, wv;
   for (int i = wid; i < nheavy; i += kTeamWarps) {
-    const int lv = heavy[i];
-    const int64_t v = I.v0 + lv, o0 = I.vtx_off[v];
-    const int d = (int)(I.vtx_off[v + 1] - o0), from = I.part[v] - I.boff, wv = I.w_v[v];
+    const int li = s.V.heavy[i];
+    team_vertex<OWN>(tm, s, li, o0, d, from, wv);
     int pen[W], internal = 0;
     bool border = false;
-    team_windows<W, UNIT>(c, o0, d, from, 0, 32, pen, internal, border);
+    team_windows<W, UNIT>(c, o0, (int)d, from, 0, 32, pen, internal, border);
     internal = warp_sum(internal);
-    if (border) team_heavy_decide<W, UNIT>(I, P, s, rec, lv, from, wv, internal, pen);
+    if (border) team_heavy_decide<W, UNIT, OWN>(P, s, li, from, wv, internal, pen);
   }
   for (int i = 0; i < nhuge; ++i) {
-    const int lv = heavy[len - 1 - i];
-    const int64_t v = I.v0 + lv, o0 = I.vtx_off[v];
-    const int d = (int)(I.vtx_off[v + 1] - o0), from = I.part[v] - I.boff, wv = I.w_v[v];
+    const int li = s.V.heavy[s.V.len - 1 - i];
+    team_vertex<OWN>(tm, s, li, o0, d, from, wv);
     __syncthreads();  // the previous vertex's sums are read
     for (int b = threadIdx.x; b < kTeamMaxK; b += blockDim.x) s.pen[b] = 0;
     if (threadIdx.x == 0) {
@@ -573,7 +679,7 @@ __device__ void team_heavy(const PxInst& I, const PxParams& P, const RoundCtx& c
     __syncthreads();
     int pen[W], internal = 0;
     bool border = false;
-    team_windows<W, UNIT>(c, o0, d, from, 32 * wid, 32 * kTeamWarps, pen, internal, border);
+    team_windows<W, UNIT>(c, o0, (int)d, from, 32 * wid, 32 * kTeamWarps, pen, internal, border);
     internal = warp_sum(internal);
     if (lane == 0) {
       if (internal) atomicAdd(&s.hint, (ull)internal);
@@ -586,7 +692,7 @@ __device__ void team_heavy(const PxInst& I, const PxParams& P, const RoundCtx& c
     if (wid == 0 && s.hborder) {
 #pragma unroll
       for (int t = 0; t < W; ++t) pen[t] = s.pen[32 * t + lane];
-      team_heavy_decide<W, UNIT>(I, P, s, rec, lv, from, wv, (int)s.hint, pen);
+      team_heavy_decide<W, UNIT, OWN>(P, s, li, from, wv, (int)s.hint, pen);
     }
   }
 }
@@ -599,10 +705,9 @@ constexpr int kTeamGroup = 4;
 // pass `take(i, rec)`, as moves from `from` to `to` (back: the reverse), and
 // sets their status to `set` (0: unchanged); with `move`, their part and the
 // CTA's block-weight deltas follow.
-template <typename Take>
-__device__ __forceinline__ void team_gather(const PxInst& I, TeamShared& s, FlatSmem& f, const int4* rec,
-                                            uint8_t* status, int c0, int ncand, bool back, int set, bool move,
-                                            Take take) {
+template <bool OWN, typename Take>
+__device__ __forceinline__ void team_gather(const Team& tm, TeamShared& s, FlatSmem& f, int c0, int ncand, bool back,
+                                            int set, bool move, Take take) {
   constexpr int PER = kFlatItems / kTeamThreads;
   if (threadIdx.x == 0) f.n = 0;
   __syncthreads();
@@ -612,23 +717,24 @@ __device__ __forceinline__ void team_gather(const PxInst& I, TeamShared& s, Flat
     bool sel = false;
     int4 r = make_int4(0, 0, 0, 0);
     if (i < ncand) {
-      r = rec[i];
+      r = team_rec<OWN>(s, i);
       sel = take(i, r);
     }
     const int slot = flat_append(f, sel);
     if (sel) {
-      const int64_t v = I.v0 + r.x;
       const int to = r.z & 0xffff, from = r.z >> 16;
-      const int64_t o0 = I.vtx_off[v];
+      int64_t o0, d;
+      team_degree<OWN>(tm, s, r.x, o0, d);
       f.o0[slot] = o0;
-      f.pre[slot] = (int)(I.vtx_off[v + 1] - o0);
+      f.pre[slot] = (int)d;
       f.ft[slot] = back ? r.z : (from | (to << 16));  // low half: the block left
       f.att[slot] = 0;
       f.pos[slot] = i;
-      if (set) status[i] = (uint8_t)set;
+      if (set) team_set_status<OWN>(s, i, set);
       if (move) {
         const int a = back ? to : from, b = back ? from : to;
-        I.part[v] = I.boff + b;
+        s.I.part[s.I.v0 + team_lv(tm, r.x)] = s.I.boff + b;
+        if (OWN && s.V.off) s.V.part[r.x] = b;
         atomicAdd(&s.dw[b], (ull)(int64_t)r.w);
         atomicAdd(&s.dw[a], (ull)(-(int64_t)r.w));
       }
@@ -680,8 +786,10 @@ __device__ __forceinline__ void team_state(const PxInst& I, const Team& tm, Team
 // The CTA's active vertices of the round, grouped by sub-round, from the
 // flags (which are cleared): list[s.off[j] .. s.off[j + 1]) is sub-round j.
 // Returns their number.
-__device__ int team_build_list(const PxInst& I, const PxParams& P, Team& tm, TeamShared& s, int32_t* list,
-                               uint32_t* masks, int chunks, int round) {
+__device__ int team_build_list(const PxInst& I, const PxParams& P, Team& tm, TeamShared& s, int round) {
+  int32_t* list = s.V.list;
+  uint32_t* masks = reinterpret_cast<uint32_t*>(s.V.kept);  // free until the round's first kept move
+  const int chunks = s.V.chunks;
   const int lane = lane_id(), wid = threadIdx.x >> 5, S = P.S;
   const int ni = (int)(I.v1 - I.v0);
   for (int j = threadIdx.x; j < S; j += blockDim.x) s.fill[j] = 0;
@@ -715,11 +823,11 @@ __device__ int team_build_list(const PxInst& I, const PxParams& P, Team& tm, Tea
   for (int i = wid; i < chunks; i += kTeamWarps) {
     const unsigned m = masks[i];
     if (!m) continue;
-    const int lv = ((i * tm.T + tm.rank) << kChunkShift) + lane;
+    const int lv = (i * tm.T + tm.rank) << kChunkShift;
     int at = 0;
     if (lane == 0) at = atomicAdd(&s.fill[subround_of(lv, round, S)], __popc(m));
     at = __shfl_sync(FULLMASK, at, 0);
-    if ((m >> lane) & 1u) list[at + __popc(m & lanemask_lt())] = lv;
+    if ((m >> lane) & 1u) list[at + __popc(m & lanemask_lt())] = (i << kChunkShift) + lane;
   }
   __syncthreads();
   return s.off[S];
@@ -727,14 +835,13 @@ __device__ int team_build_list(const PxInst& I, const PxParams& P, Team& tm, Tea
 
 // One sub-round; `q` is its slot of the team's totals. False: aborted or, with
 // *idle set, the round has no active vertex in the whole team.
-template <int W, bool UNIT, int U, bool AHEAD>
+template <int W, bool UNIT, int U, bool OWN>
 __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx& c, Team& tm, TeamShared& s,
-                              unsigned char* area, int4* rec, uint8_t* status, const int32_t* list, int32_t* heavy,
-                              int32_t* kept, int len, int sub, int q, int vbits, int64_t& t_pins, int64_t& t_moved_pins, int64_t& t_toggles,
-                              bool* idle) {
+                              unsigned char* area, int sub, int q, int64_t& t_pins, int64_t& t_moved_pins,
+                              int64_t& t_toggles, bool* idle) {
   constexpr int PL = UNIT ? 6 : 8;
   FlatSmem& f = *reinterpret_cast<FlatSmem*>(area);
-  const int lane = lane_id(), k = I.k, T = tm.T;
+  const int lane = lane_id(), k = I.k, T = tm.T, vbits = s.V.vbits;
   const TeamGlob& G = tm.G;
   // ---- slack, feasibility masks, per-block totals
   for (int b = threadIdx.x; b < k; b += blockDim.x) {
@@ -756,40 +863,52 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
     if (lane == 0) s.fmask[i] = m;
   }
   __syncthreads();
-  // ---- sweep: warps take tiles of 32 vertices, a lane evaluates its own;
-  // heavy vertices are set aside and evaluated by a warp or the CTA
+  // ---- sweep: warps take tiles of 32 / G vertices, G lanes evaluate one: few
+  // vertices leave warps idle, which then shorten the longest incidence walk
+  // (131,071 vertices on 152 CTAs, 123 per CTA and sub-round: sweep 6.8 -> 5.6
+  // us together with the resident part, the wait for its slowest CTA 4.7 -> 4.2
+  // us); heavy vertices are set aside and evaluated by a warp or the CTA
   {
     const int beg = s.off[sub], cnt = s.off[sub + 1] - beg;
+    const int gs = !OWN ? 0 : cnt <= 8 * kTeamWarps ? 2 : cnt <= 16 * kTeamWarps ? 1 : 0;  // log2 G
+    const int vi = OWN ? lane >> gs : lane, part_of = lane & ((1 << gs) - 1);
     for (;;) {
       int tile = 0;
-      if (lane == 0) tile = atomicAdd(&s.tile, 32);
+      if (lane == 0) tile = atomicAdd(&s.tile, 32 >> gs);
       tile = __shfl_sync(FULLMASK, tile, 0);
       if (tile >= cnt) break;
-      int lv = 0, from = 0, to = 0, gain = 0, wv = 0;
-      if (tile + lane < cnt) {
-        lv = list[beg + tile + lane];
-        const int64_t v = I.v0 + lv;
-        const int64_t o0 = I.vtx_off[v], dd = I.vtx_off[v + 1] - o0;
-        t_pins += dd;
-        const int d = dd > kHighDegree ? 0 : (int)dd;  // isBorderNode is false above the threshold
+      int li = 0, from = 0, to = 0, gain = 0, wv = 0, d = 0;
+      int64_t o0 = 0;
+      if (tile + vi < cnt) {
+        li = s.V.list[beg + tile + vi];
+        int64_t dd;
+        team_vertex<OWN>(tm, s, li, o0, dd, from, wv);
+        to = from;
+        if (!OWN || part_of == 0) t_pins += dd;
+        d = dd > kHighDegree ? 0 : (int)dd;  // isBorderNode is false above the threshold
         if (sweep_heavy(d, W, UNIT, I.max_we)) {
-          if (d <= kTeamHuge)
-            heavy[atomicAdd(&s.nheavy, 1)] = lv;
-          else
-            heavy[len - 1 - atomicAdd(&s.nhuge, 1)] = lv;
-        } else if (d > 0) {
-          from = to = I.part[v] - I.boff;
-          wv = I.w_v[v];
+          if (!OWN || part_of == 0) {
+            if (d <= kTeamHuge)
+              s.V.heavy[atomicAdd(&s.nheavy, 1)] = li;
+            else
+              s.V.heavy[s.V.len - 1 - atomicAdd(&s.nhuge, 1)] = li;
+          }
+          d = 0;
+        }
+        if constexpr (!OWN) {
           bool border = false;
-          lv_vertex<W, UNIT, PL, U, false, AHEAD>(c, o0, d, from, wv, 0, 0, false, P.zero_gain, s.fmask, s.slack,
-                                                  s.bw, s.perf, to, gain, border);
+          if (d > 0)
+            lv_vertex<W, UNIT, PL, U, false>(c, o0, d, from, wv, 0, 0, false, P.zero_gain, s.fmask, s.slack, s.bw,
+                                             s.perf, to, gain, border);
         }
       }
-      team_candidates(s, rec, to != from, lv, gain, from, to, wv);
+      if constexpr (OWN)
+        team_lv_vertex<W, UNIT, PL, U>(c, s, o0, d, from, wv, 1 << gs, part_of, P.zero_gain, to, gain);
+      team_candidates<OWN>(s, (!OWN || part_of == 0) && to != from, li, gain, from, to, wv);
     }
     __syncthreads();
     if (s.nheavy | s.nhuge) {
-      team_heavy<W, UNIT>(I, P, c, s, rec, heavy, len);
+      team_heavy<W, UNIT, OWN>(P, c, tm, s);
       __syncthreads();
     }
   }
@@ -837,11 +956,11 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
   if (flags & 1) {
     team_plan(I, s);
     for (int i = threadIdx.x; i < ncand; i += blockDim.x) {
-      const int4 r = rec[i];
+      const int4 r = team_rec<OWN>(s, i);
       const int b = r.z & 0xffff;
       if (s.over[b]) {
         const int64_t slot = s.seg[b] + s.base[b] + atomicAdd(&s.cur[b], 1u);
-        I.keys[slot] = team_key(r.y, r.x, vbits);
+        I.keys[slot] = team_key(r.y, team_lv(tm, r.x), vbits);
         I.kw[slot] = r.w;
       }
     }
@@ -863,8 +982,8 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
     }
     __syncthreads();
     for (int i = threadIdx.x; i < ncand; i += blockDim.x) {
-      const int4 r = rec[i];
-      if (team_key(r.y, r.x, vbits) < s.thr_to[r.z & 0xffff]) {
+      const int4 r = team_rec<OWN>(s, i);
+      if (team_key(r.y, team_lv(tm, r.x), vbits) < s.thr_to[r.z & 0xffff]) {
         atomicAdd(&s.in_w[r.z >> 16], (ull)(int64_t)r.w);
         atomicAdd(&s.in_cnt[r.z >> 16], 1u);
       }
@@ -889,9 +1008,9 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
     if (__syncthreads_or(any)) {
       team_plan(I, s);
       for (int i = threadIdx.x; i < ncand; i += blockDim.x) {
-        const int4 r = rec[i];
+        const int4 r = team_rec<OWN>(s, i);
         const int b = r.z >> 16;
-        const uint64_t key = team_key(r.y, r.x, vbits);
+        const uint64_t key = team_key(r.y, team_lv(tm, r.x), vbits);
         if (s.over[b] && key < s.thr_to[r.z & 0xffff]) {
           const int64_t slot = s.seg[b] + s.base[b] + atomicAdd(&s.cur[b], 1u);
           I.keys[slot] = key;
@@ -912,10 +1031,10 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
   int64_t att = 0;
   int total = 0, n = 0;
   for (int c0 = 0; c0 < ncand; c0 += kFlatItems) {
-    team_gather(I, s, f, rec, status, c0, ncand, false, 0, true, [&](int i, const int4& r) {
-      const uint64_t key = team_key(r.y, r.x, vbits);
+    team_gather<OWN>(tm, s, f, c0, ncand, false, 0, true, [&](int i, const int4& r) {
+      const uint64_t key = team_key(r.y, team_lv(tm, r.x), vbits);
       const bool acc = key < s.thr_to[r.z & 0xffff] && key < s.thr_from[r.z >> 16];
-      status[i] = acc ? 1 : 0;
+      team_set_status<OWN>(s, i, acc ? 1 : 0);
       return acc;
     });
     n = f.n;
@@ -932,8 +1051,8 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
   if (P.revert) {
     for (int c0 = 0; c0 < ncand; c0 += kFlatItems) {
       if (ncand > kFlatItems) {  // otherwise the commit's items are still there
-        team_gather(I, s, f, rec, status, c0, ncand, false, 0, false,
-                    [&](int i, const int4&) { return status[i] == 1; });
+        team_gather<OWN>(tm, s, f, c0, ncand, false, 0, false,
+                    [&](int i, const int4&) { return team_status<OWN>(s, i) == 1; });
         n = f.n;
         total = flat_scan(f, n);
       }
@@ -967,7 +1086,7 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
       __syncthreads();
       for (int i = threadIdx.x; i < n; i += blockDim.x)
         if (f.att[i] < 0) {
-          status[f.pos[i]] = 2;
+          team_set_status<OWN>(s, f.pos[i], 2);
           atomicAdd(&s.nrev, 1);
         }
       __syncthreads();
@@ -981,8 +1100,8 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
       att = 0;
       if (s.nrev)
         for (int c0 = 0; c0 < ncand; c0 += kFlatItems) {
-          team_gather(I, s, f, rec, status, c0, ncand, true, 0, true,
-                      [&](int i, const int4&) { return status[i] == 2; });
+          team_gather<OWN>(tm, s, f, c0, ncand, true, 0, true,
+                      [&](int i, const int4&) { return team_status<OWN>(s, i) == 2; });
           const int nu = f.n, tu = flat_scan(f, nu);
           att += flat_commit<kTeamGroup>(c, f, nu, tu, false);
           __syncthreads();
@@ -997,8 +1116,8 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
     TEAM_SYNC();
     att = 0;
     for (int c0 = 0; c0 < ncand; c0 += kFlatItems) {
-      team_gather(I, s, f, rec, status, c0, ncand, true, 3, true,
-                  [&](int i, const int4&) { return status[i] == 1; });
+      team_gather<OWN>(tm, s, f, c0, ncand, true, 3, true,
+                  [&](int i, const int4&) { return team_status<OWN>(s, i) == 1; });
       const int nu = f.n, tu = flat_scan(f, nu);
       if (threadIdx.x == 0) s.rolled += nu;
       att += flat_commit<kTeamGroup>(c, f, nu, tu, false);
@@ -1010,9 +1129,9 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
   // ---- kept moves (they activate the next round's vertices), statistics
   for (int i0 = 0; i0 < ncand; i0 += blockDim.x) {
     const int i = i0 + threadIdx.x;
-    const bool keep = i < ncand && status[i] == 1;
+    const bool keep = i < ncand && team_status<OWN>(s, i) == 1;
     const int slot = flat_append_to(&s.nkept, keep);
-    if (keep) kept[slot] = rec[i].x;
+    if (keep) s.V.kept[slot] = team_rec<OWN>(s, i).x;
   }
   if (threadIdx.x == 0) {
     s.st[kStCands] += ncand;
@@ -1025,28 +1144,139 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
 
 constexpr int kTeamBigNet = 65536;
 
-// All rounds of one instance (P.rounds, fewer when no vertex is active). `q`
-// continues over instances. False: aborted.
-template <int W, bool UNIT, int U, bool AHEAD>
-__device__ bool team_instance(const PxInst& I, const PxParams& P, Team& tm, TeamShared& s, unsigned char* area,
-                              int& q) {
-  FlatSmem& f = *reinterpret_cast<FlatSmem*>(area);
-  const RoundCtx c = team_ctx(I);
-  const int k = I.k, T = tm.T, lane = lane_id();
-  const int ni = (int)(I.v1 - I.v0);
-  const int vbits = 32 - __clz(ni > 1 ? ni - 1 : 1);
-  // this CTA's part of the scratch arrays: 32 entries per chunk. The CTA that
-  // holds the last, possibly partial chunk comes last.
+// Copies `words` 32-bit words from src to dst (whole CTA).
+__device__ __forceinline__ void team_copy(uint32_t* dst, const uint32_t* src, int64_t words) {
+#pragma unroll 4
+  for (int64_t i = threadIdx.x; i < words; i += kTeamThreads) dst[i] = src[i];
+}
+
+// This CTA's part of the instance (s.V) and the pointers its phases use (s.c).
+// The scratch arrays hold 32 entries per chunk; the CTA with the last,
+// possibly partial chunk comes last. What fits into the launch's P.resident
+// bytes of shared memory at `own` is copied there: the vertices' arrays, and
+// for a team of one CTA whose arrays start at net 0 also the nets' records and
+// pin counts.
+__device__ void team_part(const PxInst& I, int resident, const Team& tm, TeamShared& s, unsigned char* own) {
+  const int T = tm.T, ni = (int)(I.v1 - I.v0), lane = lane_id(), wid = threadIdx.x >> 5;
   const int nch = (ni + 31) >> kChunkShift, base = nch / T, rem = nch % T;
   const int chunks = base + (tm.rank < rem ? 1 : 0);
   const int last = rem ? rem - 1 : T - 1;
   const int64_t r0 = 32ll * (tm.rank > last ? (int64_t)(tm.rank - last - 1) * base
                                             : (int64_t)(T - 1 - last) * base + (int64_t)tm.rank * (base + (rem ? 1 : 0)));
   const int len = chunks == 0 ? 0 : (tm.rank == last ? ni - (int)r0 : 32 * chunks);
-  int4* rec = I.rec + I.v0 + r0;
-  uint8_t* status = I.status + I.v0 + r0;
-  int32_t* list = I.list + r0;
-  int32_t* cand = I.cand + r0;
+  int32_t* off = reinterpret_cast<int32_t*>(own);
+  int32_t *wv = off + len + 1, *part = wv + len, *list = part + len, *inets = list + len;
+  int64_t left = (int64_t)resident - 4 * (4 * (int64_t)len + 1);
+  // incidences per chunk, then the chunks' starts
+  int64_t run = 0;
+  const bool room = left > 0;
+  if (room)
+    for (int c0 = 0; c0 < chunks; c0 += kTeamThreads) {
+      const int i = c0 + threadIdx.x;
+      int64_t size = 0;
+      if (i < chunks) {
+        const int v = team_lv(tm, i << kChunkShift);
+        size = I.vtx_off[I.v0 + min(v + 32, ni)] - I.vtx_off[I.v0 + v];
+      }
+      int64_t total;
+      const int64_t at = run + block_scan_excl_i64(size, &total);
+      if (i < chunks) off[i << kChunkShift] = (int)min(at, (int64_t)INT_MAX);
+      run += total;
+    }
+  left -= 4 * run;
+  const bool res = room && left >= 0;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    RoundCtx c{};
+    c.inets = res ? inets : I.inets;
+    c.w_e = I.w_e;
+    c.phi = I.phi;
+    c.conn = I.conn;
+    c.k = I.k;
+    c.W = I.W;
+    c.kmax = I.kstride;
+    c.unit_nets = I.unit_nets;
+    c.phi16 = I.phi16;
+    c.max_we = I.max_we;
+    s.c = c;
+    s.V.rec = I.rec + I.v0 + r0;
+    s.V.status = I.status + I.v0 + r0;
+    s.V.list = res ? list : I.list + r0;
+    s.V.heavy = I.kw + r0;
+    s.V.kept = I.cand + r0;
+    s.V.off = res ? off : nullptr;
+    s.V.wv = wv;
+    s.V.part = part;
+    s.V.len = len;
+    s.V.chunks = chunks;
+    s.V.vbits = 32 - __clz(ni > 1 ? ni - 1 : 1);
+    s.V.own_nets = 0;
+  }
+  if (res) {
+    for (int i = wid; i < chunks; i += kTeamWarps) {
+      const int lv = team_lv(tm, i << kChunkShift) + lane, li = (i << kChunkShift) + lane;
+      const int64_t v = I.v0 + min(lv, ni - 1);
+      const int at = off[i << kChunkShift];
+      const int64_t g = I.vtx_off[v], g0 = __shfl_sync(FULLMASK, g, 0);
+      const int64_t size = __shfl_sync(FULLMASK, I.vtx_off[v + 1], 31) - g0;
+      __syncwarp();
+      if (lv < ni) {
+        off[li] = at + (int)(g - g0);
+        wv[li] = I.w_v[v];
+        part[li] = I.part[v] - I.boff;
+      }
+      for (int64_t x = lane; x < size; x += 32) inets[at + x] = I.inets[g0 + x];
+    }
+    if (threadIdx.x == 0) off[len] = (int)run;
+  }
+  __syncthreads();
+  if (T == 1 && res && I.e0 == 0) {
+    // 16-byte boundary for the record loads
+    uint32_t* at = reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(inets + run) + 15) & ~(uintptr_t)15);
+    left -= 16;
+    const int64_t cw = I.e1 * 2 * I.W, pe = I.e1 * I.kstride, pw = I.phi16 ? (pe + 1) / 2 : pe;
+    int nets = 0;
+    if (left >= 4 * cw) {
+      left -= 4 * cw;
+      team_copy(at, I.conn, cw);
+      if (threadIdx.x == 0) s.c.conn = at;
+      at += cw;
+      nets |= 1;
+    }
+    if (left >= 4 * pw) {
+      team_copy(at, reinterpret_cast<const uint32_t*>(I.phi), pw);
+      if (threadIdx.x == 0) s.c.phi = reinterpret_cast<int32_t*>(at);
+      nets |= 2;
+    }
+    if (threadIdx.x == 0) s.V.own_nets = nets;
+    __syncthreads();
+  }
+}
+
+// Writes the nets' records and pin counts back.
+__device__ void team_put_back(const PxInst& I, const TeamShared& s) {
+  if (s.V.own_nets & 1) team_copy(I.conn, s.c.conn, I.e1 * 2 * I.W);
+  if (s.V.own_nets & 2) {
+    const int64_t pe = I.e1 * I.kstride;
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(s.c.phi);
+    team_copy(reinterpret_cast<uint32_t*>(I.phi), src, I.phi16 ? pe / 2 : pe);
+    if (I.phi16 && (pe & 1) && threadIdx.x == 0)  // the last word's other half may be another instance's
+      reinterpret_cast<uint16_t*>(I.phi)[pe - 1] = reinterpret_cast<const uint16_t*>(src)[pe - 1];
+  }
+}
+
+// All rounds of one instance (P.rounds, fewer when no vertex is active). `q`
+// continues over instances. False: aborted.
+template <int W, bool UNIT, int U, bool OWN>
+__device__ bool team_instance(const PxInst& I, const PxParams& P, Team& tm, TeamShared& s, unsigned char* area,
+                              int& q) {
+  FlatSmem& f = *reinterpret_cast<FlatSmem*>(area);
+  const int k = I.k, T = tm.T, lane = lane_id();
+  team_part(I, OWN ? P.resident : 0, tm, s, area + kTeamOwnAt);
+  // with 64 registers and 4-word records the pointers are better re-read from
+  // shared memory than spilled (4.2M vertices 11,880 -> 11,270 us)
+  typename std::conditional<(OWN || W < 4), const RoundCtx, const RoundCtx&>::type c = s.c;
+  const int32_t* kept = s.V.kept;
   for (int b = threadIdx.x; b < k; b += blockDim.x) {
     s.bw[b] = I.bw[I.boff + b];
     s.lmax[b] = I.lmax[I.boff + b];
@@ -1057,13 +1287,12 @@ __device__ bool team_instance(const PxInst& I, const PxParams& P, Team& tm, Team
   for (int round = first; round < first + P.rounds; ++round) {
     if (threadIdx.x < kStats) s.st[threadIdx.x] = 0;
     if (threadIdx.x == 0) s.nkept = 0;
-    const int active = team_build_list(I, P, tm, s, list, reinterpret_cast<uint32_t*>(cand), chunks, round);
+    const int active = team_build_list(I, P, tm, s, round);
     int64_t t_pins = 0, t_moved_pins = 0, t_toggles = 0;
     bool idle = false;
     for (int sub = 0; sub < P.S; ++sub) {
-      const bool ok = team_subround<W, UNIT, U, AHEAD>(I, P, c, tm, s, area, rec, status, list, I.kw + r0, cand, len, sub, q,
-                                                vbits,
-                                                t_pins, t_moved_pins, t_toggles, &idle);
+      const bool ok = team_subround<W, UNIT, U, OWN>(I, P, c, tm, s, area, sub, q, t_pins, t_moved_pins, t_toggles,
+                                                       &idle);
       q = q == 2 ? 0 : q + 1;
       if (idle) break;
       if (!ok) return false;
@@ -1091,11 +1320,12 @@ __device__ bool team_instance(const PxInst& I, const PxParams& P, Team& tm, Team
     for (int c0 = 0; c0 < nkept; c0 += kFlatItems) {
       const int n = min(kFlatItems, nkept - c0);
       for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int64_t v = I.v0 + cand[c0 + i];
-        const int64_t o0 = I.vtx_off[v];
+        const int li = kept[c0 + i];
+        int64_t o0, d;
+        team_degree<OWN>(tm, s, li, o0, d);
         f.o0[i] = o0;
-        f.pre[i] = (int)(I.vtx_off[v + 1] - o0);
-        I.flag[v] = 1;
+        f.pre[i] = (int)d;
+        I.flag[I.v0 + team_lv(tm, li)] = 1;
       }
       __syncthreads();
       const int total = flat_scan(f, n);
@@ -1166,8 +1396,10 @@ __device__ bool team_instance(const PxInst& I, const PxParams& P, Team& tm, Team
     TEAM_SYNC();
   }
   __syncthreads();
-  if (T == 1)
+  if (T == 1) {
     for (int b = threadIdx.x; b < k; b += blockDim.x) I.bw[I.boff + b] = s.bw[b];
+    if (OWN) team_put_back(I, s);
+  }
   return true;
 }
 
@@ -1177,7 +1409,7 @@ __global__ void __launch_bounds__(kTeamThreads, MINB) k_team(const PxInst* __res
                                                              PxParams P, int sync, int64_t* scratch, int64_t* queue,
                                                              int64_t* err) {
   extern __shared__ __align__(16) unsigned char team_smem[];
-  TeamShared& s = *reinterpret_cast<TeamShared*>(team_smem + ((kTeamArea + 15) & ~size_t(15)));
+  TeamShared& s = *reinterpret_cast<TeamShared*>(team_smem + kTeamSharedAt);
   Team tm;
   tm.T = P.T;
   tm.rank = blockIdx.x % P.T;
@@ -1235,11 +1467,37 @@ static const void* team_kernel_for(int W, bool unit, int unroll, int minb) {
   return unit ? team_kernel_wu<4, true>(unroll, minb) : team_kernel_wu<4, false>(unroll, minb);
 }
 
-static int team_occupancy(const void* kern, int minb) {
-  allow_dyn_smem_of(kern, kTeamSmem);
+static int team_occupancy(const void* kern, int minb, size_t smem) {
+  allow_dyn_smem_of(kern, smem);
   int blocks = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, kTeamThreads, kTeamSmem) != cudaSuccess) return 1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, kTeamThreads, smem) != cudaSuccess) return 1;
   return std::max(1, std::min(blocks, minb));
+}
+
+// Shared memory for a CTA's part of the instance. A team of several CTAs leaves
+// half of the SM's memory to the L1 cache, which holds the record gathers in
+// flight (400K vertices with 170 KB of parts: 3,030 -> 3,690 us).
+static int64_t team_own_most(int per_sm, int T) {
+  return per_sm >= 2 ? 0 : (T == 1 ? 224 : 128) * 1024 - (int64_t)kTeamSmem;
+}
+
+// Shared memory of a launch: what a CTA's part of the instance wants with a
+// quarter to spare (the CTAs' shares differ), if an SM holds it; a part that
+// does not fit stays in global memory and leaves the SM's memory to the L1
+// cache.
+static size_t team_smem_bytes(int minb, int T, int64_t own_bytes) {
+  if (minb >= 2) return kTeamSmemShort;
+  const int64_t most = team_own_most(minb, T);
+  if (own_bytes <= 0 || own_bytes > most) return kTeamSmem;
+  return kTeamSmem + (size_t)std::min(most, own_bytes + own_bytes / 4 + 1024);
+}
+
+int64_t team_own_bytes(int64_t n, int64_t m, int64_t pins, int T, int k, int W, bool phi16, int per_sm) {
+  const int64_t own = 4 * (pins / T) + 16 * (n / T + 32);
+  if (T > 1) return own;
+  const int64_t nets = own + 16 + 8 * m * W, all = nets + (phi16 ? 2 : 4) * m * k;
+  const int64_t most = team_own_most(per_sm, T);
+  return all <= most ? all : nets <= most ? nets : own;
 }
 
 // Larger teams finish the largest instance sooner, more of them keep the SMs
@@ -1263,7 +1521,8 @@ int team_slots(const Launch& L, int64_t count, int T) {
 
 int team_resident(const Launch& L, int W, bool unit, int unroll, int ctas_per_sm) {
   const int minb = ctas_per_sm >= 2 ? 2 : 1;
-  return L.num_sms * team_occupancy(team_kernel_for(W, unit, unroll, minb), minb);
+  return L.num_sms * team_occupancy(team_kernel_for(W, unit, unroll, minb), minb,
+                                       minb >= 2 ? kTeamSmemShort : kTeamSmem);
 }
 
 // Active vertices of every instance's last persistent round (its round's
@@ -1283,7 +1542,7 @@ cudaError_t launch_px_active(const Launch& L, const PxInst* insts, int32_t count
 
 cudaError_t launch_px_round(const Launch& L, const PxInst* insts, const int32_t* order, int32_t count, PxParams P,
                             int W, bool unit, int ctas_per_sm, int teams, int64_t* scratch, int64_t* queue,
-                            int64_t* err) {
+                            int64_t* err, int64_t own_bytes) {
   if (count <= 0 || P.rounds <= 0) return cudaSuccess;
   if ((W != 1 && W != 2 && W != 4) || P.T < 1 || P.kcap > kTeamMaxK) return cudaErrorInvalidValue;
   const bool grid = P.T > kTeamMaxCluster;
@@ -1299,14 +1558,16 @@ cudaError_t launch_px_round(const Launch& L, const PxInst* insts, const int32_t*
   }
   const int minb = ctas_per_sm >= 2 ? 2 : 1;
   const void* kern = team_kernel_for(W, unit, P.unroll, minb);
-  const int resident = L.num_sms * team_occupancy(kern, minb);
+  const size_t smem = team_smem_bytes(minb, P.T, own_bytes);
+  P.resident = smem > kTeamSmem ? (int32_t)(smem - kTeamSmem) : 0;
+  const int resident = L.num_sms * team_occupancy(kern, minb, smem);
   if (grid && P.T > resident) return cudaErrorCooperativeLaunchTooLarge;
   teams = std::max(1, std::min(teams, std::min<int>(count, std::max(1, resident / P.T))));
   int sync = P.T == 1 ? kSyncCta : grid ? kSyncGrid : kSyncCluster;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(teams * P.T));
   cfg.blockDim = dim3(kTeamThreads);
-  cfg.dynamicSmemBytes = kTeamSmem;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = L.st;
   cudaLaunchAttribute at[1];
   cfg.attrs = at;

@@ -76,3 +76,23 @@ def test_team_node_list(lp):
     nodes = np.arange(0, 30000, 7, dtype=np.int32)
     _same(_refine(lp, inst.hg, 16, inst.part, nodes=nodes),
           _refine(lp, inst.hg, 16, inst.part, nodes=nodes, flags=lp.FLAG_MULTI_LAUNCH))
+
+
+@pytest.mark.parametrize("n,size,skew", [(16384, 40, 0.0), (16384, 12, 0.6), (1800, 30, 0.0), (2048, 7, 0.0)])
+def test_team_resident_part(lp, n, size, skew):
+    """Instances whose arrays do not fit a CTA's shared memory, that fit in all
+    but one CTA of the team (its chunks hold most incidences), or in part."""
+    from lpgpu import gen
+    rng = np.random.default_rng(n + size)
+    m = n
+    net = np.repeat(np.arange(m), size)
+    v = rng.integers(0, n, m * size)
+    hot = rng.random(m * size) < skew  # chunks 0, 16, 32, ... all belong to the first CTA of 16
+    v = np.where(hot, (v // 32 // 16 * 16) * 32 + v % 32, v)
+    key = np.unique(net.astype(np.int64) * n + v)
+    off = np.zeros(m + 1, np.int64)
+    np.cumsum(np.bincount(key // n, minlength=m), out=off[1:])
+    hg = gen.Hypergraph(n, m, off, (key % n).astype(np.int32), rng.integers(1, 4, n).astype(np.int32),
+                        np.ones(m, np.int32))
+    part = rng.integers(0, 61, n).astype(np.int32)
+    _same(_refine(lp, hg, 61, part, rounds=3), _refine(lp, hg, 61, part, rounds=3, flags=lp.FLAG_MULTI_LAUNCH))
