@@ -56,7 +56,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if force or _stale(obj, [src] + headers):
             jobs.append([cc] + ARCH + NVCC_FLAGS + ["-c", src, "-o", obj])
     if jobs:
-        with cf.ThreadPoolExecutor(max_workers=min(8, len(jobs))) as ex:
+        with cf.ThreadPoolExecutor(max_workers=min(os.cpu_count() or 8, len(jobs))) as ex:
             futs = [ex.submit(subprocess.run, j, capture_output=True, text=True) for j in jobs]
             for j, f in zip(jobs, futs):
                 r = f.result()

@@ -310,9 +310,9 @@ cudaError_t launch_repair_candidates(const Launch& L, const RoundCtx& c, int blk
 
 // ---- team rounds (LP rounds of whole instances inside one launch)
 
-// Largest k of an instance the team kernel takes (Λ records of at most 4
-// words), and the largest one the persistent form of the API accepts.
-constexpr int kTeamMaxK = 128;
+// Largest k of an instance the team kernel takes, and the largest one the
+// persistent form of the API accepts.
+constexpr int kTeamMaxK = LPGPU_MAX_K;
 constexpr int kPxMaxK = 64;
 
 // One instance of a team launch. Arrays are indexed by the ids the instance's
@@ -345,7 +345,7 @@ struct PxInst {
   int64_t e0, e1;       // the instance's nets
   int32_t boff, k;
   int32_t kstride;      // Φ row length
-  int32_t W;            // Λ words per record half (1, 2 or 4)
+  int32_t W;            // Λ words per record half (1, 2, 4, ..., 32)
   int32_t unit_nets, phi16, max_we;
   int32_t round;        // first round of this instance (when the launch does not set one)
 };
@@ -356,7 +356,7 @@ struct PxParams {
   int32_t round;        // >= 0: every instance starts at this round; < 0: at its own `round`
   int32_t rounds;       // rounds to run (an instance without active vertices stops earlier)
   int32_t activate_last;  // 1: the last of them also activates its successor's vertices
-  int32_t unroll;       // incidences per lane step of the sweep (4 or 8; W = 4: always 4)
+  int32_t unroll;       // incidences per lane step of the sweep (8: in the 2-CTA builds for k <= 64)
   int32_t T;            // CTAs per team
   int32_t kcap;         // largest k of the launch
   int32_t resident;     // bytes of shared memory per CTA for the instance's own arrays (set by the launch)
@@ -371,7 +371,7 @@ constexpr int kTeamMaxCluster = 16;
 
 // Runs LP rounds of `count` instances, taken in `order` (null: 0..count-1)
 // from the work queue counter `queue` (zeroed here) by up to `teams` teams of
-// P.T CTAs each. W: Λ words class of all instances (1, 2 or 4); unit: every net
+// P.T CTAs each. W: Λ words class of all instances; unit: every net
 // weight is 1; ctas_per_sm: the 1- or 2-CTA-per-SM build of the kernel.
 // `scratch`: teams * team_scratch_words(P.kcap) words (P.T > 1, zeroed here).
 // A grid barrier that gives up sets *err. More than kTeamMaxCluster CTAs per

@@ -30,7 +30,10 @@ def _same(a, b):
 # vertices: no chunk, one partial chunk, whole chunks, one CTA / cluster / grid limits, fewer chunks than CTAs
 @pytest.mark.parametrize("n,k,weighted", [
     (1, 1, False), (7, 3, True), (32, 2, False), (33, 4, True), (2048, 128, True), (2049, 65, False),
-    (2080, 2, True), (16384, 2, False), (16385, 33, True), (20000, 128, False), (70001, 64, True)])
+    (2080, 2, True), (16384, 2, False), (16385, 33, True), (20000, 128, False), (70001, 64, True),
+    # more than 128 blocks: two, four or eight lanes per vertex
+    (1000, 129, True), (1500, 1024, False), (9000, 300, False), (30000, 300, True), (40000, 1024, True),
+    (50000, 513, False), (300, 256, False)])
 def test_team_equals_multi_launch(lp, n, k, weighted):
     from lpgpu import gen
     inst = gen.random_small(n + k, n=n, m=max(1, int(1.2 * n)), k=k, max_size=9, weighted=weighted) if n > 40 else None
@@ -68,6 +71,18 @@ def test_team_selection_sizes(lp, orc):
         ref, _ = orc.lp_sync(inst.hg, k, inst.lmax, part, perfect=inst.perfect, rounds=rounds, subrounds=1, revert=1,
                              rollback=1, zero_gain=1)
         assert np.array_equal(got[0], ref)
+
+
+@pytest.mark.parametrize("k", [200, 1000])
+def test_team_wide_hubs_and_weights(lp, orc, k):
+    """k > 128 with heavy vertices (warp and CTA) and vertex weights above the
+    precomputed feasibility masks, against the oracle."""
+    from lpgpu import gen
+    inst = gen.random_small(k, n=6000, m=9000, k=k, max_size=14, hubs=3, hub_frac=0.2, vw_hi=40)
+    got = _refine(lp, inst.hg, k, inst.part, rounds=3)
+    ref, _ = orc.lp_sync(inst.hg, k, inst.lmax, inst.part, perfect=inst.perfect, rounds=3, subrounds=7, revert=1,
+                         rollback=1, zero_gain=1)
+    assert np.array_equal(got[0], ref)
 
 
 def test_team_node_list(lp):
