@@ -363,7 +363,9 @@ struct PxParams {
 };
 
 // int64 words of global scratch one team of more than one CTA needs.
-inline int64_t team_scratch_words(int kcap) { return 32 + 17 * (int64_t)kcap; }
+__host__ __device__ inline int64_t team_scratch_words(int kcap) {
+  return 32 + 17 * (int64_t)kcap + 3 * kMaxSubrounds;
+}
 
 // CTAs per team of a launch over one instance of n vertices (1: a CTA; up to
 // kTeamMaxCluster: a thread-block cluster; more: the whole cooperative grid).

@@ -19,11 +19,15 @@
 // 1,280-instance batch from 55.7 to 39.0 ms end to end and 24 stepped sessions
 // from 38.1 to 20.2 ms.
 //
-// Vertices are dealt to the team's CTAs in 32-vertex chunks (chunk c to CTA
-// c mod T), so a vertex is swept, selected, moved and undone by one CTA, whose
-// candidate list, kept moves and active list live in its own part of the
-// instance's scratch arrays. CTAs meet in per-block totals and selection
-// segments (global memory) only.
+// A vertex is swept, selected, moved and undone by one CTA per sub-round, whose
+// candidate and kept-move lists live in its own part of the instance's scratch
+// arrays; CTAs meet in per-block totals and selection segments (global memory)
+// only. The 1-CTA-per-SM builds deal the vertices out once, in 32-vertex chunks
+// (chunk c to CTA c mod T), and so can keep them in shared memory. The others
+// list a round's active vertices per sub-round for the whole team and cut each
+// sub-round's list into equal parts: a CTA's chunks fall into a sub-round by a
+// hash, 15 +- 4 of them where 304 CTAs share a million vertices, and the
+// slowest CTA had 1.7 times the mean.
 #pragma once
 
 #include <cstddef>
@@ -60,6 +64,8 @@ struct TeamGlob {
   __device__ ull* active(int q) const { return in_w(q) + 5 * K + 2; }
   __device__ uint64_t* thr_to() const { return reinterpret_cast<uint64_t*>(g + 32 + 15 * (int64_t)K); }
   __device__ uint64_t* thr_from() const { return thr_to() + K; }
+  // active vertices per sub-round, for three rounds in turn
+  __device__ ull* count(int r) const { return reinterpret_cast<ull*>(thr_from() + K) + r * kMaxSubrounds; }
 };
 
 constexpr int kTeamStage = 2048;  // selection keys a CTA holds in registers and shared memory
@@ -92,6 +98,8 @@ struct TeamPart {
   uint8_t* status;
   int32_t *list, *heavy, *kept;
   int32_t *off, *wv, *part;
+  uint32_t* masks;  // active vertices per chunk while the list is built (free until the round's first kept move)
+  int beg, cnt;     // this CTA's part of the sub-round's list
   int len, vbits, chunks, own_nets;  // own_nets: bit 0 the records, 1 the pin counts are in shared memory
 };
 
@@ -115,6 +123,7 @@ struct TeamShared {
   uint32_t fmask[kLvWeights * KM / 32];
   uint8_t over[KM];
   int off[kMaxSubrounds + 1], fill[kMaxSubrounds];
+  int kbeg[kMaxSubrounds], kpre[kMaxSubrounds + 1];  // kept moves of the round's sub-rounds: place, count before
   long long st[kStats];
   uint64_t red_and[kTeamWarps], red_or[kTeamWarps];
   unsigned wsum[kTeamWarps];
@@ -139,6 +148,7 @@ struct Team {
   TeamGlob G;
   int T, rank, sync;
   ull arrivals;  // barrier arrivals expected so far (grid barrier, thread 0)
+  int builds;    // active lists built so far
 };
 
 // Barrier of the team: everything its CTAs wrote before is visible after. The
@@ -504,8 +514,9 @@ __device__ __forceinline__ void team_select(const PxInst& I, Team& tm, TS& s, un
   }
 }
 
+template <bool OWN>
 __device__ __forceinline__ int team_lv(const Team& tm, int li) {
-  return (((li >> kChunkShift) * tm.T + tm.rank) << kChunkShift) | (li & 31);
+  return !OWN ? li : (((li >> kChunkShift) * tm.T + tm.rank) << kChunkShift) | (li & 31);
 }
 template <bool OWN, typename TS>
 __device__ __forceinline__ void team_degree(const Team& tm, const TS& s, int li, int64_t& o0, int64_t& d) {
@@ -513,7 +524,7 @@ __device__ __forceinline__ void team_degree(const Team& tm, const TS& s, int li,
     o0 = s.V.off[li];
     d = s.V.off[li + 1] - o0;
   } else {
-    const int64_t v = s.I.v0 + team_lv(tm, li);
+    const int64_t v = s.I.v0 + team_lv<OWN>(tm, li);
     o0 = s.I.vtx_off[v];
     d = s.I.vtx_off[v + 1] - o0;
   }
@@ -526,7 +537,7 @@ __device__ __forceinline__ void team_vertex(const Team& tm, const TS& s, int li,
     from = s.V.part[li];
     wv = s.V.wv[li];
   } else {
-    const int64_t v = s.I.v0 + team_lv(tm, li);
+    const int64_t v = s.I.v0 + team_lv<OWN>(tm, li);
     from = s.I.part[v] - s.I.boff;
     wv = s.I.w_v[v];
   }
@@ -849,7 +860,7 @@ __device__ __forceinline__ void team_gather(const Team& tm, TS& s, FlatSmem& f, 
       if (set) team_set_status<OWN>(s, i, set);
       if (move) {
         const int a = back ? to : from, b = back ? from : to;
-        s.I.part[s.I.v0 + team_lv(tm, r.x)] = s.I.boff + b;
+        s.I.part[s.I.v0 + team_lv<OWN>(tm, r.x)] = s.I.boff + b;
         if (OWN && s.V.off) s.V.part[r.x] = b;
         atomicAdd(&s.dw[b], (ull)(int64_t)r.w);
         atomicAdd(&s.dw[a], (ull)(-(int64_t)r.w));
@@ -901,13 +912,15 @@ __device__ __forceinline__ void team_state(const PxInst& I, const Team& tm, TS& 
   __syncthreads();
 }
 
-// The CTA's active vertices of the round, grouped by sub-round, from the
-// flags (which are cleared): list[s.off[j] .. s.off[j + 1]) is sub-round j.
-// Returns their number.
-template <typename TS>
+// The round's active vertices grouped by sub-round, from the flags (which are
+// cleared): sub-round j is list[s.off[j] .. s.off[j + 1]), of the CTA's own
+// vertices (by their index in the CTA) or, for a team that shares its list, of
+// all of the team's. Returns their number, -1: aborted.
+template <bool OWN, typename TS>
 __device__ int team_build_list(const PxInst& I, const PxParams& P, Team& tm, TS& s, int round) {
+  const bool shared = !OWN && tm.T > 1;
   int32_t* list = s.V.list;
-  uint32_t* masks = reinterpret_cast<uint32_t*>(s.V.kept);  // free until the round's first kept move
+  uint32_t* masks = s.V.masks;
   const int chunks = s.V.chunks;
   const int lane = lane_id(), wid = threadIdx.x >> 5, S = P.S;
   const int ni = (int)(I.v1 - I.v0);
@@ -924,6 +937,17 @@ __device__ int team_build_list(const PxInst& I, const PxParams& P, Team& tm, TS&
     }
   }
   __syncthreads();
+  if (shared) {
+    const int r = tm.builds % 3;
+    for (int j = threadIdx.x; j < S; j += blockDim.x)
+      s.kbeg[j] = s.fill[j] ? (int)atomicAdd(tm.G.count(r) + j, (ull)s.fill[j]) : 0;
+    if (!team_sync(tm, s)) return -1;
+    if (tm.rank == 0)  // nobody reads the counts of the round before last any more
+      for (int j = threadIdx.x; j < kMaxSubrounds; j += blockDim.x) tm.G.count(r == 2 ? 0 : r + 1)[j] = 0;
+    for (int j = threadIdx.x; j < S; j += blockDim.x) s.fill[j] = (int)tm.G.count(r)[j];
+    __syncthreads();
+  }
+  ++tm.builds;
   if (threadIdx.x < 32) {  // S <= 64: two bins per lane
     const int a = 2 * lane < S ? s.fill[2 * lane] : 0, b = 2 * lane + 1 < S ? s.fill[2 * lane + 1] : 0;
     int incl = a + b;
@@ -934,8 +958,14 @@ __device__ int team_build_list(const PxInst& I, const PxParams& P, Team& tm, TS&
     }
     const int excl = incl - a - b;
     __syncwarp();
-    if (2 * lane < S) s.off[2 * lane] = s.fill[2 * lane] = excl;
-    if (2 * lane + 1 < S) s.off[2 * lane + 1] = s.fill[2 * lane + 1] = excl + a;
+    if (2 * lane < S) {
+      s.off[2 * lane] = excl;
+      s.fill[2 * lane] = excl + (shared ? s.kbeg[2 * lane] : 0);
+    }
+    if (2 * lane + 1 < S) {
+      s.off[2 * lane + 1] = excl + a;
+      s.fill[2 * lane + 1] = excl + a + (shared ? s.kbeg[2 * lane + 1] : 0);
+    }
     if (lane == 31) s.off[S] = incl;
   }
   __syncthreads();
@@ -946,9 +976,13 @@ __device__ int team_build_list(const PxInst& I, const PxParams& P, Team& tm, TS&
     int at = 0;
     if (lane == 0) at = atomicAdd(&s.fill[subround_of(lv, round, S)], __popc(m));
     at = __shfl_sync(FULLMASK, at, 0);
-    if ((m >> lane) & 1u) list[at + __popc(m & lanemask_lt())] = (i << kChunkShift) + lane;
+    if ((m >> lane) & 1u) list[at + __popc(m & lanemask_lt())] = (OWN ? i << kChunkShift : lv) + lane;
   }
-  __syncthreads();
+  if (shared) {
+    if (!team_sync(tm, s)) return -1;
+  } else {
+    __syncthreads();
+  }
   return s.off[S];
 }
 
@@ -974,6 +1008,18 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
     s.ncand = s.nrev = s.rolled = s.tile = s.nheavy = s.nhuge = 0;
     s.any = 0;
     s.delta = s.gdelta = 0;
+    const int beg = s.off[sub], cnt = s.off[sub + 1] - beg;
+    s.V.beg = beg;
+    s.V.cnt = cnt;
+    if (!OWN && T > 1) {  // an equal part of the team's list, and of the scratch arrays at its place
+      const int lo = (int)((int64_t)cnt * tm.rank / T), hi = (int)((int64_t)cnt * (tm.rank + 1) / T);
+      s.V.beg = beg + lo;
+      s.V.cnt = s.V.len = hi - lo;
+      s.V.rec = I.rec + I.v0 + beg + lo;
+      s.V.status = I.status + I.v0 + beg + lo;
+      s.V.heavy = I.kw + beg + lo;
+      s.V.kept = I.cand + beg + lo;
+    }
   }
   __syncthreads();
   for (int i = threadIdx.x >> 5; i < kLvWeights * W; i += kTeamWarps) {
@@ -988,7 +1034,7 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
   // us together with the resident part, the wait for its slowest CTA 4.7 -> 4.2
   // us); heavy vertices are set aside and evaluated by a warp or the CTA
   {
-    const int beg = s.off[sub], cnt = s.off[sub + 1] - beg;
+    const int beg = s.V.beg, cnt = s.V.cnt;
     constexpr int wide = W <= 4 ? 0 : W == 8 ? 1 : W == 16 ? 2 : 3;  // k > 128: log2 of the W / 4 lanes per vertex
     const int gs = wide ? wide : !OWN ? 0 : cnt <= 8 * kTeamWarps ? 2 : cnt <= 16 * kTeamWarps ? 1 : 0;  // log2 G
     const int vi = OWN ? lane >> gs : lane, part_of = lane & ((1 << gs) - 1);
@@ -1043,7 +1089,7 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
       }
       if (s.out_w[b]) atomicAdd(G.out_w(q) + b, s.out_w[b]);
     }
-    if (sub == 0 && threadIdx.x == 0 && s.off[P.S]) atomicAdd(G.active(q), (ull)s.off[P.S]);
+    if (OWN && sub == 0 && threadIdx.x == 0 && s.off[P.S]) atomicAdd(G.active(q), (ull)s.off[P.S]);
   }
   TEAM_SYNC();
   // ---- plan: target blocks whose candidates weigh more than the slack, and
@@ -1063,7 +1109,7 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
     if (bits) atomicOr(&s.any, bits);
   }
   if (sub == 0) {
-    const int64_t act = T > 1 ? (int64_t)*(G.active(q)) : (int64_t)s.off[P.S];
+    const int64_t act = OWN && T > 1 ? (int64_t)*(G.active(q)) : (int64_t)s.off[P.S];
     if (act == 0) {  // the same in every CTA
       *idle = true;
       __syncthreads();
@@ -1072,7 +1118,11 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
   }
   __syncthreads();
   const int flags = s.any;
-  if (!(flags & 4)) return true;  // no candidate in the team
+  if (!(flags & 4)) {  // no candidate in the team
+    if (threadIdx.x == 0) s.kpre[sub] = s.nkept;
+    __syncthreads();
+    return true;
+  }
   // ---- target side (the atomic weight check of changeNodePart, h:548-562):
   // per block the longest (gain, vertex) prefix within L_max
   if (flags & 1) {
@@ -1082,7 +1132,7 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
       const int b = r.z & 0xffff;
       if (s.over[b]) {
         const int64_t slot = s.seg[b] + s.base[b] + atomicAdd(&s.cur[b], 1u);
-        I.keys[slot] = team_key(r.y, team_lv(tm, r.x), vbits);
+        I.keys[slot] = team_key(r.y, team_lv<OWN>(tm, r.x), vbits);
         I.kw[slot] = r.w;
       }
     }
@@ -1105,7 +1155,7 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
     __syncthreads();
     for (int i = threadIdx.x; i < ncand; i += blockDim.x) {
       const int4 r = team_rec<OWN>(s, i);
-      if (team_key(r.y, team_lv(tm, r.x), vbits) < s.thr_to[r.z & 0xffff]) {
+      if (team_key(r.y, team_lv<OWN>(tm, r.x), vbits) < s.thr_to[r.z & 0xffff]) {
         atomicAdd(&s.in_w[r.z >> 16], (ull)(int64_t)r.w);
         atomicAdd(&s.in_cnt[r.z >> 16], 1u);
       }
@@ -1132,7 +1182,7 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
       for (int i = threadIdx.x; i < ncand; i += blockDim.x) {
         const int4 r = team_rec<OWN>(s, i);
         const int b = r.z >> 16;
-        const uint64_t key = team_key(r.y, team_lv(tm, r.x), vbits);
+        const uint64_t key = team_key(r.y, team_lv<OWN>(tm, r.x), vbits);
         if (s.over[b] && key < s.thr_to[r.z & 0xffff]) {
           const int64_t slot = s.seg[b] + s.base[b] + atomicAdd(&s.cur[b], 1u);
           I.keys[slot] = key;
@@ -1154,7 +1204,7 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
   int total = 0, n = 0;
   for (int c0 = 0; c0 < ncand; c0 += kFlatItems) {
     team_gather<OWN>(tm, s, f, c0, ncand, false, 0, true, [&](int i, const int4& r) {
-      const uint64_t key = team_key(r.y, team_lv(tm, r.x), vbits);
+      const uint64_t key = team_key(r.y, team_lv<OWN>(tm, r.x), vbits);
       const bool acc = key < s.thr_to[r.z & 0xffff] && key < s.thr_from[r.z >> 16];
       team_set_status<OWN>(s, i, acc ? 1 : 0);
       return acc;
@@ -1249,16 +1299,23 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
     team_state(I, tm, s, q);
   }
   // ---- kept moves (they activate the next round's vertices), statistics
+  const bool shared = !OWN && T > 1;
+  const int at0 = s.nkept;
+  __syncthreads();
   for (int i0 = 0; i0 < ncand; i0 += blockDim.x) {
     const int i = i0 + threadIdx.x;
     const bool keep = i < ncand && team_status<OWN>(s, i) == 1;
     const int slot = flat_append_to(&s.nkept, keep);
-    if (keep) s.V.kept[slot] = team_rec<OWN>(s, i).x;
+    if (keep) s.V.kept[shared ? slot - at0 : slot] = team_rec<OWN>(s, i).x;
   }
   if (threadIdx.x == 0) {
     s.st[kStCands] += ncand;
     s.st[kStReverted] += s.nrev + s.rolled;
     s.st[kStDelta] += s.delta;
+    if (shared) {
+      s.kbeg[sub] = s.V.beg;
+      s.kpre[sub] = at0;
+    }
   }
   __syncthreads();
   return true;
@@ -1279,7 +1336,7 @@ __device__ __forceinline__ void team_copy(uint32_t* dst, const uint32_t* src, in
 // for a team of one CTA whose arrays start at net 0 also the nets' records and
 // pin counts.
 template <typename TS>
-__device__ void team_part(const PxInst& I, int resident, const Team& tm, TS& s, unsigned char* own) {
+__device__ void team_part(const PxInst& I, int resident, bool shared, const Team& tm, TS& s, unsigned char* own) {
   const int T = tm.T, ni = (int)(I.v1 - I.v0), lane = lane_id(), wid = threadIdx.x >> 5;
   const int nch = (ni + 31) >> kChunkShift, base = nch / T, rem = nch % T;
   const int chunks = base + (tm.rank < rem ? 1 : 0);
@@ -1298,7 +1355,7 @@ __device__ void team_part(const PxInst& I, int resident, const Team& tm, TS& s, 
       const int i = c0 + threadIdx.x;
       int64_t size = 0;
       if (i < chunks) {
-        const int v = team_lv(tm, i << kChunkShift);
+        const int v = team_lv<true>(tm, i << kChunkShift);
         size = I.vtx_off[I.v0 + min(v + 32, ni)] - I.vtx_off[I.v0 + v];
       }
       int64_t total;
@@ -1324,9 +1381,10 @@ __device__ void team_part(const PxInst& I, int resident, const Team& tm, TS& s, 
     s.c = c;
     s.V.rec = I.rec + I.v0 + r0;
     s.V.status = I.status + I.v0 + r0;
-    s.V.list = res ? list : I.list + r0;
+    s.V.list = res ? list : shared ? I.list : I.list + r0;  // a shared list holds the whole team's vertices
     s.V.heavy = I.kw + r0;
     s.V.kept = I.cand + r0;
+    s.V.masks = reinterpret_cast<uint32_t*>(I.cand + r0);
     s.V.off = res ? off : nullptr;
     s.V.wv = wv;
     s.V.part = part;
@@ -1337,7 +1395,7 @@ __device__ void team_part(const PxInst& I, int resident, const Team& tm, TS& s, 
   }
   if (res) {
     for (int i = wid; i < chunks; i += kTeamWarps) {
-      const int lv = team_lv(tm, i << kChunkShift) + lane, li = (i << kChunkShift) + lane;
+      const int lv = team_lv<true>(tm, i << kChunkShift) + lane, li = (i << kChunkShift) + lane;
       const int64_t v = I.v0 + min(lv, ni - 1);
       const int at = off[i << kChunkShift];
       const int64_t g = I.vtx_off[v], g0 = __shfl_sync(FULLMASK, g, 0);
@@ -1396,7 +1454,8 @@ __device__ bool team_instance(const PxInst& I, const PxParams& P, Team& tm, TS& 
                               int& q) {
   FlatSmem& f = *reinterpret_cast<FlatSmem*>(area);
   const int k = I.k, T = tm.T, lane = lane_id();
-  team_part(I, OWN ? P.resident : 0, tm, s, area + kTeamOwnAt<TS::kBlocks>);
+  const bool shared = !OWN && T > 1;
+  team_part(I, OWN ? P.resident : 0, shared, tm, s, area + kTeamOwnAt<TS::kBlocks>);
   // with 64 registers and 4-word records the pointers are better re-read from
   // shared memory than spilled (4.2M vertices 11,880 -> 11,270 us)
   typename std::conditional<(OWN || W < 4), const RoundCtx, const RoundCtx&>::type c = s.c;
@@ -1411,7 +1470,8 @@ __device__ bool team_instance(const PxInst& I, const PxParams& P, Team& tm, TS& 
   for (int round = first; round < first + P.rounds; ++round) {
     if (threadIdx.x < kStats) s.st[threadIdx.x] = 0;
     if (threadIdx.x == 0) s.nkept = 0;
-    const int active = team_build_list(I, P, tm, s, round);
+    const int active = team_build_list<OWN>(I, P, tm, s, round);
+    if (active < 0) return false;
     int64_t t_pins = 0, t_moved_pins = 0, t_toggles = 0;
     bool idle = false;
     for (int sub = 0; sub < P.S; ++sub) {
@@ -1430,7 +1490,8 @@ __device__ bool team_instance(const PxInst& I, const PxParams& P, Team& tm, TS& 
       atomicAdd(reinterpret_cast<ull*>(&s.st[kStToggles]), (ull)t_toggles);
     }
     if (threadIdx.x == 0) {
-      s.st[kStActive] = active;
+      s.st[kStActive] = !shared || tm.rank == 0 ? active : 0;
+      s.kpre[P.S] = s.nkept;
       s.st[kStMoved] = s.nkept;
       s.st[kStMovedPins] = t_moved_pins;
     }
@@ -1444,12 +1505,19 @@ __device__ bool team_instance(const PxInst& I, const PxParams& P, Team& tm, TS& 
     for (int c0 = 0; c0 < nkept; c0 += kFlatItems) {
       const int n = min(kFlatItems, nkept - c0);
       for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int li = kept[c0 + i];
+        int li;
+        if (shared) {  // the sub-rounds' kept moves lie apart
+          int j = 0;
+          while (s.kpre[j + 1] <= c0 + i) ++j;
+          li = I.cand[s.kbeg[j] + c0 + i - s.kpre[j]];
+        } else {
+          li = kept[c0 + i];
+        }
         int64_t o0, d;
         team_degree<OWN>(tm, s, li, o0, d);
         f.o0[i] = o0;
         f.pre[i] = (int)d;
-        I.flag[I.v0 + team_lv(tm, li)] = 1;
+        I.flag[I.v0 + team_lv<OWN>(tm, li)] = 1;
       }
       __syncthreads();
       const int total = flat_scan(f, n);
@@ -1539,8 +1607,9 @@ __global__ void __launch_bounds__(kTeamThreads, MINB) k_team(const PxInst* __res
   tm.rank = blockIdx.x % P.T;
   tm.sync = sync;
   tm.arrivals = 0;
+  tm.builds = 0;
   tm.G.K = P.kcap;
-  tm.G.g = scratch ? scratch + (int64_t)(blockIdx.x / P.T) * (32 + 17 * (int64_t)P.kcap) : nullptr;
+  tm.G.g = scratch ? scratch + (int64_t)(blockIdx.x / P.T) * team_scratch_words(P.kcap) : nullptr;
   if (threadIdx.x == 0) s.abort = 0;
   __syncthreads();
   int q = 0;
