@@ -83,6 +83,7 @@ enum Scalar : int {
   kHeavyCount = 11, // heavy vertices a per-vertex query deferred to k_sweep_heavy
   kRevCount = 12,  // moves marked for revert in the current sub-round
   kPxQueue = 13,   // work queue counter of a persistent round
+  kStepKm1 = 14,   // km1 and cut at the start of a stepped refinement
   kScalars = 16
 };
 
@@ -237,7 +238,10 @@ cudaError_t launch_build_incidence(const Launch& L, int64_t n, int64_t m, int64_
                                    int32_t* rank, int64_t* scan_tmp, int64_t scan_tmp_elems,
                                    int64_t* deg_hist);
 cudaError_t launch_init_partition(const Launch& L, const RoundCtx& c);
-cudaError_t launch_metrics(const Launch& L, const RoundCtx& c);
+// Adds km1 and cut to out[0] and out[1] (zeroed by the caller).
+cudaError_t launch_metrics(const Launch& L, const RoundCtx& c, int64_t* out);
+// dst = a[0 .. na) followed by b[0 .. nb): what the host reads after a call, in one copy.
+cudaError_t launch_report(const Launch& L, int64_t* dst, const int64_t* a, int64_t na, const int64_t* b, int64_t nb);
 cudaError_t launch_instance_metrics(const Launch& L, const RoundCtx& c, int64_t* km1_inst);
 cudaError_t launch_best_moves(const Launch& L, const RoundCtx& c, int32_t* to, int32_t* gain,
                               uint8_t* border);

@@ -393,7 +393,7 @@ cudaError_t launch_init_partition(const Launch& L, const RoundCtx& c) {
 }
 
 // metrics::km1 / hyperedgeCut (metrics.cpp:29-65): thread per net.
-__global__ void k_metrics(RoundCtx c) {
+__global__ void k_metrics(RoundCtx c, int64_t* out) {
   int64_t km1 = 0, cut = 0;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < c.m;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -406,8 +406,8 @@ __global__ void k_metrics(RoundCtx c) {
   km1 = block_sum_i64(km1);
   cut = block_sum_i64(cut);
   if (threadIdx.x == 0) {
-    atomicAdd(reinterpret_cast<ull*>(&c.scal[kKm1]), (ull)km1);
-    atomicAdd(reinterpret_cast<ull*>(&c.scal[kCut]), (ull)cut);
+    atomicAdd(reinterpret_cast<ull*>(&out[0]), (ull)km1);
+    atomicAdd(reinterpret_cast<ull*>(&out[1]), (ull)cut);
   }
 }
 
@@ -434,13 +434,22 @@ cudaError_t launch_instance_metrics(const Launch& L, const RoundCtx& c, int64_t*
   return cudaSuccess;
 }
 
-cudaError_t launch_metrics(const Launch& L, const RoundCtx& c) {
-  cudaError_t e = cudaMemsetAsync(c.scal + kKm1, 0, sizeof(int64_t) * 2, L.st);
-  if (e != cudaSuccess) return e;
+cudaError_t launch_metrics(const Launch& L, const RoundCtx& c, int64_t* out) {
   if (c.m > 0) {
-    k_metrics<<<grid_for(L, c.m, 256), 256, 0, L.st>>>(c);
+    k_metrics<<<grid_for(L, c.m, 256), 256, 0, L.st>>>(c, out);
     LAUNCHED("k_metrics");
   }
+  return cudaGetLastError();
+}
+
+__global__ void k_report(int64_t* dst, const int64_t* a, int64_t na, const int64_t* b, int64_t nb) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < na + nb; i += (int64_t)gridDim.x * blockDim.x)
+    dst[i] = i < na ? a[i] : b[i - na];
+}
+
+cudaError_t launch_report(const Launch& L, int64_t* dst, const int64_t* a, int64_t na, const int64_t* b, int64_t nb) {
+  k_report<<<grid_for(L, na + nb, 256), 256, 0, L.st>>>(dst, a, na, b, nb);
+  LAUNCHED("k_report");
   return cudaGetLastError();
 }
 

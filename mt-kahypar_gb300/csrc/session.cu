@@ -129,6 +129,9 @@ using namespace lpgpu;
     if (_e != cudaSuccess) return cuda_fail(_e, #expr); \
   } while (0)
 
+// Head of a session's report: km1 and cut before and after, the team kernel's error word.
+enum ReportWord : int { kRepBefore = 0, kRepAfter = 2, kRepErr = 4, kRepHead = 8 };
+
 struct lpgpu_session_s {
   int device = 0;
   cudaStream_t st = nullptr;
@@ -187,12 +190,18 @@ struct lpgpu_session_s {
   bool stepping = false, step_done = false;
   lpgpu_config step_cfg{};
   int32_t step_round = 0;
-  int64_t step_km1_before = 0;
   cudaEvent_t step_ev = nullptr;
   DevBuf<int32_t> vinst, inst_boff, inst_k, over_ids;
   DevBuf<int64_t> inst_voff, inst_noff, inst_delta;
   DevBuf<int64_t> vout;  // result words of the device-side input checks
   DevBuf<int64_t> team;  // per-team scratch of the team rounds
+  // what the host reads back after a call, in one copy (ReportWord, then round
+  // statistics and the block weights)
+  DevBuf<int64_t> rep;
+  std::vector<int64_t> h_lmax;
+  cudaError_t reserve_report(int64_t words) {
+    return (int64_t)rep.count >= words ? cudaSuccess : rep.alloc((size_t)words, &mem);
+  }
   // results of the last refine
   std::vector<lpgpu_round_stats> last_stats;
   // timing
@@ -338,6 +347,7 @@ struct lpgpu_session_s {
     px.release(&mem);
     px_order.release(&mem);
     team.release(&mem);
+    rep.release(&mem);
     px_key.clear();
     vinst.release(&mem);
     inst_voff.release(&mem);
@@ -433,11 +443,11 @@ lpgpu_status lpgpu_session_create(int32_t device, lpgpu_session** out) {
   }
   if (device < 0 || device >= count) return invalid("device index out of range");
   DeviceGuard g(device);
-  cudaDeviceProp prop;
-  CK(cudaGetDeviceProperties(&prop, device));
+  int sms = 0;
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   auto* s = new lpgpu_session_s();
   s->device = device;
-  s->num_sms = prop.multiProcessorCount;
+  s->num_sms = sms;
   e = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
     delete s;
@@ -746,18 +756,20 @@ static lpgpu_status set_partition_impl(lpgpu_session* s, int32_t K, int32_t kmax
   } else if (s->n > 0) {
     CK(cudaMemcpyAsync(s->part.p, part, sizeof(int32_t) * s->n, cudaMemcpyHostToDevice, st));
   }
-  CK(launch_check_partition(s->launch(), s->n, s->part.p, K, s->batched ? s->vinst.p : nullptr,
-                            s->inst_boff.p, s->inst_k.p, s->vout.p));
-  int64_t check = 0;
-  CK(cudaMemcpyAsync(&check, s->vout.p + kVErr, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   CK(cudaMemcpyAsync(s->lmax.p, hl.data(), sizeof(int64_t) * K, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(s->perfect.p, hp.data(), sizeof(int64_t) * K, cudaMemcpyHostToDevice, st));
-  CK(cudaStreamSynchronize(st));
-  if (check != kVOk) return invalid("block id out of range");
   CK(cudaMemsetAsync(s->blk64.p, 0, sizeof(int64_t) * (7 * (size_t)K + 1), st));
+  // the check replaces block ids out of range, so the state is built right
+  // behind it and one round trip brings the verdict
+  CK(launch_check_partition(s->launch(), s->n, s->part.p, K, s->batched ? s->vinst.p : nullptr,
+                            s->inst_boff.p, s->inst_k.p, s->vout.p));
   RoundCtx c = s->ctx();
   CK(launch_init_partition(s->launch(), c));
+  int64_t check = 0;
+  CK(cudaMemcpyAsync(&check, s->vout.p + kVErr, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  if (check != kVOk) return invalid("block id out of range");
+  s->h_lmax = hl;
   s->h_perfect = hp;
   s->has_part = true;
   s->trim();
@@ -875,28 +887,33 @@ lpgpu_status lpgpu_session_project_partition(lpgpu_session* fine, const lpgpu_se
   return set_partition_impl(fine, coarse->k, coarse->k, nullptr, hl, hp, nullptr, proj.p());
 }
 
-static lpgpu_status read_metrics(lpgpu_session* s, int64_t* km1, int64_t* cut);
-static lpgpu_status read_imbalance(lpgpu_session* s, double* imb);
-
-static lpgpu_status read_metrics(lpgpu_session* s, int64_t* km1, int64_t* cut) {
-  RoundCtx c = s->ctx();
-  CK(launch_metrics(s->launch(), c));
-  int64_t h[2];
-  CK(cudaMemcpyAsync(h, s->scal.p + kKm1, sizeof(h), cudaMemcpyDeviceToHost, s->st));
+// Reads the report back: its head, `nstats` words of statistics and the block
+// weights, in one copy (the caller has reserved it and written its head).
+static lpgpu_status fetch_report(lpgpu_session* s, const int64_t* stats, int64_t nstats, std::vector<int64_t>* h) {
+  CK(launch_report(s->launch(), s->rep.p + kRepHead, stats, nstats, s->bw.p, s->k));
+  h->resize(kRepHead + nstats + s->k);
+  CK(cudaMemcpyAsync(h->data(), s->rep.p, sizeof(int64_t) * h->size(), cudaMemcpyDeviceToHost, s->st));
   CK(cudaStreamSynchronize(s->st));
-  if (km1) *km1 = h[0];
-  if (cut) *cut = h[1];
   return LPGPU_OK;
 }
 
-static lpgpu_status read_imbalance(lpgpu_session* s, double* imb) {
-  std::vector<int64_t> w(s->k);
-  CK(cudaMemcpyAsync(w.data(), s->bw.p, sizeof(int64_t) * s->k, cudaMemcpyDeviceToHost, s->st));
-  CK(cudaStreamSynchronize(s->st));
-  // metrics::imbalance (metrics.cpp:114-128)
+// metrics::imbalance (metrics.cpp:114-128) from the block weights
+static double imbalance_of(const lpgpu_session* s, const int64_t* w) {
   double mx = (double)w[0] / (double)s->h_perfect[0];
   for (int b = 1; b < s->k; ++b) mx = std::max(mx, (double)w[b] / (double)s->h_perfect[b]);
-  *imb = mx - 1.0;
+  return mx - 1.0;
+}
+
+static lpgpu_status read_metrics(lpgpu_session* s, int64_t* km1, int64_t* cut, double* imbalance) {
+  CK(s->reserve_report(kRepHead + s->k));
+  CK(cudaMemsetAsync(s->rep.p, 0, sizeof(int64_t) * kRepHead, s->st));
+  CK(launch_metrics(s->launch(), s->ctx(), s->rep.p + kRepAfter));
+  std::vector<int64_t> h;
+  const lpgpu_status st = fetch_report(s, nullptr, 0, &h);
+  if (st != LPGPU_OK) return st;
+  if (km1) *km1 = h[kRepAfter];
+  if (cut) *cut = h[kRepAfter + 1];
+  if (imbalance) *imbalance = imbalance_of(s, h.data() + kRepHead);
   return LPGPU_OK;
 }
 
@@ -1077,17 +1094,16 @@ lpgpu_status lpgpu_session_tuning(lpgpu_session* s, lpgpu_tuning* out) {
   return LPGPU_OK;
 }
 
-// Statistics of R rounds (hs: R x kStats, rounds after the first one without
+// A report with the statistics of R rounds (rounds after the first one without
 // an active vertex did not run) into last_stats and the refine result
 // (IRefiner::refine's metrics update, label_propagation_refiner.cpp:48-67).
-static lpgpu_status book_rounds(lpgpu_session* s, const std::vector<int64_t>& hs, int R, int64_t km1_before,
-                                lpgpu_result* result) {
+static void book_rounds(lpgpu_session* s, const std::vector<int64_t>& h, int R, lpgpu_result* result) {
   s->last_stats.clear();
   int executed = 0;
   bool stopped = false;
   int64_t delta = 0, moves = 0, pins = 0;
   for (int r = 0; r < R; ++r) {
-    const int64_t* x = &hs[(size_t)r * kStats];
+    const int64_t* x = &h[kRepHead + (size_t)r * kStats];
     if (x[kStActive] == 0) stopped = true;
     if (stopped) continue;
     lpgpu_round_stats rs{x[kStActive], x[kStPins],  x[kStCands],     x[kStMoved],
@@ -1099,22 +1115,15 @@ static lpgpu_status book_rounds(lpgpu_session* s, const std::vector<int64_t>& hs
     pins += rs.pins;
   }
   if (result) {
-    int64_t km1_after = 0;
-    lpgpu_status ms = read_metrics(s, &km1_after, nullptr);
-    if (ms != LPGPU_OK) return ms;
-    double imb = 0;
-    ms = read_imbalance(s, &imb);
-    if (ms != LPGPU_OK) return ms;
-    result->km1_before = km1_before;
-    result->km1_after = km1_after;
+    result->km1_before = h[kRepBefore];
+    result->km1_after = h[kRepAfter];
     result->delta = delta;
     result->moves = moves;
     result->pins_processed = pins;
     result->rounds = executed;
     result->improved = delta < 0;
-    result->imbalance = imb;
+    result->imbalance = imbalance_of(s, h.data() + kRepHead + (size_t)std::max(1, R) * kStats);
   }
-  return LPGPU_OK;
 }
 
 lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
@@ -1189,11 +1198,12 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
   pxp.kcap = kmax;
   pxp.T = shape.T;
   cudaStream_t st = s->st;
-  int64_t km1_before = 0;
-  lpgpu_status ms = read_metrics(s, &km1_before, nullptr);
-  if (ms != LPGPU_OK) return ms;
   RoundCtx c = s->ctx(&cfg);
   const Launch L = s->launch();
+  const int64_t nstats = (int64_t)std::max(1, R) * kStats;
+  CK(s->reserve_report(kRepHead + nstats + s->k));
+  CK(cudaMemsetAsync(s->rep.p, 0, sizeof(int64_t) * kRepHead, st));
+  CK(launch_metrics(L, c, s->rep.p + kRepBefore));
   TmpBuf<int32_t> dnodes(s->mem);
   if (num_nodes > 0) {
     CK(dnodes.alloc(num_nodes));
@@ -1206,23 +1216,24 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
   auto enqueue = [&]() -> cudaError_t {
     cudaError_t e;
     if ((e = cudaMemsetAsync(s->stats.p, 0, sizeof(int64_t) * std::max(1, R) * kStats, st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(s->blk64.p, 0, sizeof(int64_t) * (7 * s->k + 1), st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(s->scal.p, 0, sizeof(int64_t) * kScalars, st)) != cudaSuccess) return e;
     if (s->m > 0 && (e = cudaMemsetAsync(s->net_epoch.p, 0, sizeof(int32_t) * s->m, st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(s->bin_cnt.p, 0, sizeof(int64_t) * kMaxSubrounds * kDegClasses, st)) != cudaSuccess)
-      return e;
-    if (s->batched && (e = cudaMemsetAsync(s->inst_delta.p, 0, sizeof(int64_t) * s->num_inst, st)) != cudaSuccess)
-      return e;
+    if (!use_team) {  // accumulators of the multi-launch kernels
+      if ((e = cudaMemsetAsync(s->blk64.p, 0, sizeof(int64_t) * (7 * s->k + 1), st)) != cudaSuccess) return e;
+      if ((e = cudaMemsetAsync(s->scal.p, 0, sizeof(int64_t) * kScalars, st)) != cudaSuccess) return e;
+      if ((e = cudaMemsetAsync(s->bin_cnt.p, 0, sizeof(int64_t) * kMaxSubrounds * kDegClasses, st)) != cudaSuccess)
+        return e;
+      if (s->batched && (e = cudaMemsetAsync(s->inst_delta.p, 0, sizeof(int64_t) * s->num_inst, st)) != cudaSuccess)
+        return e;
+    }
     if (num_nodes > 0) {
       if ((e = launch_mark_list(L, c, dnodes.p(), num_nodes)) != cudaSuccess) return e;
-    } else {
-      if (s->n > 0 && (e = cudaMemsetAsync(s->next_flag.p, 0, s->n, st)) != cudaSuccess) return e;
-      if ((e = launch_mark_all(L, c, cfg.rebalancing)) != cudaSuccess) return e;
+    } else if ((e = launch_mark_all(L, c, cfg.rebalancing)) != cudaSuccess) {  // sets every vertex's flag
+      return e;
     }
     if (use_team) {  // all rounds in one launch
       if ((e = launch_px_round(L, s->px.p, s->px_order.p, px_count, pxp, s->W, s->unit_nets, shape.per_sm,
                                team_slots(L, px_count, shape.T), s->team.p, s->scal.p + kPxQueue,
-                               s->scal.p + kError, own_bytes)) != cudaSuccess)
+                               s->rep.p + kRepErr, own_bytes)) != cudaSuccess)
         return e;
       if (s->n > 0 && (e = cudaMemsetAsync(s->next_flag.p, 0, s->n, st)) != cudaSuccess) return e;
       return cudaSuccess;
@@ -1280,12 +1291,11 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
     CK(cudaGraphLaunch(s->graph, st));
     add_kernel_launches(s->graph_kernels);
   }
-  std::vector<int64_t> hs(std::max(1, R) * kStats);
-  CK(cudaMemcpyAsync(hs.data(), s->stats.p, sizeof(int64_t) * hs.size(), cudaMemcpyDeviceToHost, st));
-  int64_t err = 0;
-  if (use_team) CK(cudaMemcpyAsync(&err, s->scal.p + kError, sizeof(err), cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
-  if (err) {
+  if (result) CK(launch_metrics(L, c, s->rep.p + kRepAfter));
+  std::vector<int64_t> h;
+  ps = fetch_report(s, s->stats.p, nstats, &h);
+  if (ps != LPGPU_OK) return ps;
+  if (h[kRepErr]) {
     s->has_part = false;  // the moves of an unfinished sub-round
     set_error("a grid barrier of the refinement gave up");
     return LPGPU_ERR_TIMEOUT;
@@ -1307,7 +1317,8 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
       s->phase_times.push_back(t);
     }
   }
-  return book_rounds(s, hs, R, km1_before, result);
+  book_rounds(s, h, R, result);
+  return LPGPU_OK;
 }
 
 // ---- stepped refinement: one persistent round of many sessions per launch
@@ -1327,13 +1338,12 @@ lpgpu_status lpgpu_session_begin_rounds(lpgpu_session* s, const lpgpu_config* cf
   CK(s->stats.alloc(std::max(1, R) * kStats, &s->mem));
   ps = build_px(s, 0);
   if (ps != LPGPU_OK) return ps;
-  ps = read_metrics(s, &s->step_km1_before, nullptr);
-  if (ps != LPGPU_OK) return ps;
   if (!s->step_ev) CK(cudaEventCreateWithFlags(&s->step_ev, cudaEventDisableTiming));
   RoundCtx c = s->ctx(&cfg);
+  CK(cudaMemsetAsync(s->scal.p + kStepKm1, 0, sizeof(int64_t) * 2, st));
+  CK(launch_metrics(s->launch(), c, s->scal.p + kStepKm1));
   CK(cudaMemsetAsync(s->stats.p, 0, sizeof(int64_t) * std::max(1, R) * kStats, st));
   if (s->m > 0) CK(cudaMemsetAsync(s->net_epoch.p, 0, sizeof(int32_t) * s->m, st));
-  if (s->n > 0) CK(cudaMemsetAsync(s->next_flag.p, 0, s->n, st));
   CK(launch_mark_all(s->launch(), c, cfg.rebalancing));
   s->step_cfg = cfg;
   s->step_round = 0;
@@ -1350,12 +1360,18 @@ lpgpu_status lpgpu_session_end_rounds(lpgpu_session* s, lpgpu_result* result) {
   }
   DeviceGuard g(s->device);
   const int R = s->step_cfg.rounds;
-  std::vector<int64_t> hs((size_t)std::max(1, R) * kStats);
-  CK(cudaMemcpyAsync(hs.data(), s->stats.p, sizeof(int64_t) * hs.size(), cudaMemcpyDeviceToHost, s->st));
+  const int64_t nstats = (int64_t)std::max(1, R) * kStats;
+  CK(s->reserve_report(kRepHead + nstats + s->k));
+  CK(cudaMemsetAsync(s->rep.p, 0, sizeof(int64_t) * kRepHead, s->st));
+  CK(cudaMemcpyAsync(s->rep.p + kRepBefore, s->scal.p + kStepKm1, sizeof(int64_t) * 2, cudaMemcpyDeviceToDevice, s->st));
+  if (result) CK(launch_metrics(s->launch(), s->ctx(), s->rep.p + kRepAfter));
   if (s->n > 0) CK(cudaMemsetAsync(s->next_flag.p, 0, s->n, s->st));
-  CK(cudaStreamSynchronize(s->st));
+  std::vector<int64_t> h;
+  const lpgpu_status ps = fetch_report(s, s->stats.p, nstats, &h);
+  if (ps != LPGPU_OK) return ps;
   s->stepping = false;
-  return book_rounds(s, hs, R, s->step_km1_before, result);
+  book_rounds(s, h, R, result);
+  return LPGPU_OK;
 }
 
 }  // extern "C"
@@ -1392,13 +1408,11 @@ lpgpu_status lpgpu_stepper_create(int32_t device, lpgpu_stepper** out) {
   DeviceGuard g(device);
   auto* t = new lpgpu_stepper_s();
   t->device = device;
-  cudaDeviceProp prop;
-  if ((e = cudaGetDeviceProperties(&prop, device)) != cudaSuccess ||
+  if ((e = cudaDeviceGetAttribute(&t->num_sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess ||
       (e = cudaStreamCreateWithFlags(&t->st, cudaStreamNonBlocking)) != cudaSuccess) {
     delete t;
     return cuda_fail(e, "stepper stream");
   }
-  t->num_sms = prop.multiProcessorCount;
   cudaMemPoolProps props{};
   props.allocType = cudaMemAllocationTypePinned;
   props.location.type = cudaMemLocationTypeDevice;
@@ -1642,7 +1656,7 @@ lpgpu_status lpgpu_session_instance_km1(lpgpu_session* s, int64_t* km1) {
   if (!km1) return invalid("null output");
   DeviceGuard g(s->device);
   if (!s->batched) {
-    return read_metrics(s, km1, nullptr);
+    return read_metrics(s, km1, nullptr, nullptr);
   }
   TmpBuf<int64_t> d(s->mem);
   CK(d.alloc(s->num_inst));
@@ -1657,10 +1671,7 @@ lpgpu_status lpgpu_session_metrics(lpgpu_session* s, int64_t* km1, int64_t* cut,
   lpgpu_status ps = need_part(s);
   if (ps != LPGPU_OK) return ps;
   DeviceGuard g(s->device);
-  ps = read_metrics(s, km1, cut);
-  if (ps != LPGPU_OK) return ps;
-  if (imbalance) return read_imbalance(s, imbalance);
-  return LPGPU_OK;
+  return read_metrics(s, km1, cut, imbalance);
 }
 
 lpgpu_status lpgpu_session_get_block_weights(lpgpu_session* s, int64_t* weights) {
@@ -1978,15 +1989,24 @@ lpgpu_status lpgpu_session_rebalance(lpgpu_session* s, int32_t max_rounds, lpgpu
   CK(cudaMemsetAsync(s->stats.p, 0, sizeof(int64_t) * std::max(1, R) * kStats, st));
   TmpBuf<int64_t> rb(s->mem);
   CK(rb.alloc(5 * (size_t)k + 1));
-  int64_t km1_before = 0;
-  ps = read_metrics(s, &km1_before, nullptr);
-  if (ps != LPGPU_OK) return ps;
-  std::vector<int64_t> hl(k), hb(k), hs(kStats);
-  CK(cudaMemcpyAsync(hl.data(), s->lmax.p, sizeof(int64_t) * k, cudaMemcpyDeviceToHost, st));
+  CK(s->reserve_report(kRepHead + kStats + k));
   const int64_t sub[2] = {0, s->n};
   RoundCtx c = s->ctx();
   c.revert = 0;
   c.rollback = 0;
+  // km1 and the block weights before, in one round trip; every round brings its
+  // statistics, the new weights and the new km1 in another
+  CK(cudaMemsetAsync(s->rep.p, 0, sizeof(int64_t) * kRepHead, st));
+  CK(launch_metrics(s->launch(), c, s->rep.p + kRepAfter));
+  CK(cudaMemcpyAsync(s->sub_off.p, sub, sizeof(sub), cudaMemcpyHostToDevice, st));
+  std::vector<int64_t> h;
+  ps = fetch_report(s, nullptr, 0, &h);
+  if (ps != LPGPU_OK) return ps;
+  const int64_t km1_before = h[kRepAfter];
+  const std::vector<int64_t>& hl = s->h_lmax;
+  std::vector<int64_t> hb(h.begin() + kRepHead, h.end());
+  int64_t km1_after = km1_before;
+  bool moved_before = false;  // the repair moved vertices: weights and km1 are read again
   s->last_stats.clear();
   int64_t delta = 0, moves = 0, pins = 0;
   {
@@ -1994,8 +2014,6 @@ lpgpu_status lpgpu_session_rebalance(lpgpu_session* s, int32_t max_rounds, lpgpu
     // repairEmptyBlocks come first, each applied as moveVertex does
     // (rebalancer.h:84-103: the target stays within L_max, the source keeps
     // weight > 0); they form the first statistics record
-    CK(cudaMemcpyAsync(hb.data(), s->bw.p, sizeof(int64_t) * k, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
     bool over = false, empty = false;
     for (int b = 0; b < k; ++b) {
       over = over || hb[b] > hl[b];
@@ -2018,6 +2036,7 @@ lpgpu_status lpgpu_session_rebalance(lpgpu_session* s, int32_t max_rounds, lpgpu
       }
       int64_t d = 0;
       if (!av.empty()) {
+        moved_before = true;
         const size_t cnt = av.size();
         TmpBuf<int32_t> dv(s->mem), df(s->mem), dt(s->mem);
         CK(dv.alloc(cnt));
@@ -2037,19 +2056,27 @@ lpgpu_status lpgpu_session_rebalance(lpgpu_session* s, int32_t max_rounds, lpgpu
       pins += rs.pins;
     }
   }
-  for (int r = 0; r < R; ++r) {
+  if (moved_before) {
+    double unused = 0;
+    ps = read_metrics(s, &km1_after, nullptr, &unused);
+    if (ps != LPGPU_OK) return ps;
     CK(cudaMemcpyAsync(hb.data(), s->bw.p, sizeof(int64_t) * k, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+  }
+  for (int r = 0; r < R; ++r) {
     bool over = false;
     for (int b = 0; b < k; ++b) over = over || hb[b] > hl[b];
     if (!over) break;
     // one sub-round over all vertices (rec and status per vertex id)
-    CK(cudaMemcpyAsync(s->sub_off.p, sub, sizeof(sub), cudaMemcpyHostToDevice, st));
     CK(cudaMemsetAsync(s->blk64.p, 0, sizeof(int64_t) * 3 * k, st));  // in_w, in_cnt, cand_out
+    CK(cudaMemsetAsync(s->rep.p, 0, sizeof(int64_t) * kRepHead, st));
     CK(launch_rebalance_round(s->launch(), c, r, s->heavy.p, s->revl.p, rb.p()));
-    CK(cudaMemcpyAsync(hs.data(), s->stats.p + (int64_t)r * kStats, sizeof(int64_t) * kStats,
-                       cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    CK(launch_metrics(s->launch(), c, s->rep.p + kRepAfter));
+    ps = fetch_report(s, s->stats.p + (int64_t)r * kStats, kStats, &h);
+    if (ps != LPGPU_OK) return ps;
+    km1_after = h[kRepAfter];
+    const int64_t* hs = h.data() + kRepHead;
+    hb.assign(h.begin() + kRepHead + kStats, h.end());
     lpgpu_round_stats rs{hs[kStActive],   hs[kStPins],  hs[kStCands],     hs[kStMoved],
                          hs[kStReverted], hs[kStDelta], hs[kStMovedPins], hs[kStToggles]};
     s->last_stats.push_back(rs);
@@ -2059,12 +2086,6 @@ lpgpu_status lpgpu_session_rebalance(lpgpu_session* s, int32_t max_rounds, lpgpu
     if (rs.moved == 0) break;
   }
   if (result) {
-    int64_t km1_after = 0;
-    ps = read_metrics(s, &km1_after, nullptr);
-    if (ps != LPGPU_OK) return ps;
-    double imb = 0;
-    ps = read_imbalance(s, &imb);
-    if (ps != LPGPU_OK) return ps;
     result->km1_before = km1_before;
     result->km1_after = km1_after;
     result->delta = delta;
@@ -2072,7 +2093,7 @@ lpgpu_status lpgpu_session_rebalance(lpgpu_session* s, int32_t max_rounds, lpgpu
     result->pins_processed = pins;
     result->rounds = (int32_t)s->last_stats.size();
     result->improved = delta < 0;
-    result->imbalance = imb;
+    result->imbalance = imbalance_of(s, hb.data());
   }
   return LPGPU_OK;
 }

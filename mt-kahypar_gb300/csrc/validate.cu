@@ -222,7 +222,7 @@ __global__ void k_check_partition(int64_t n, int32_t* __restrict__ part, int k, 
       const int i = vinst[v];
       if (p < 0 || p >= inst_k[i]) {
         fail(out, kVBlockRange);
-        part[v] = 0;  // keeps later indexing in range; the call fails anyway
+        part[v] = inst_boff[i];  // keeps the state built from it in range; the call fails anyway
       } else {
         part[v] = p + inst_boff[i];
       }
