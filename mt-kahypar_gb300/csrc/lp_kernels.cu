@@ -2445,86 +2445,226 @@ cudaError_t launch_expand_nets(const Launch& L, const RoundCtx& c, int S, PhaseT
 
 // Best move with rebalance = true of every border vertex of an overloaded
 // block (Km1Policy::computeMaxGainMoveImpl, gain_policy.h:108-167): minimum
-// score over feasible blocks, any sign, lowest id on ties. Warp per vertex,
-// penalties summed per block in shared memory.
+// score over feasible blocks, any sign, lowest id on ties. For k <= 128 a lane
+// evaluates its own vertex with the sweep's bit-sliced counters; vertices beyond
+// them (and all for k > 128) take the warp. Per-block sums are privatized per CTA: thousands of
+// candidates leave a few overloaded blocks. 200,003 vertices, k = 32, 87,000 of
+// them in overloaded blocks: 234 -> 66 us (and k_rb_emit 85 -> 14).
+template <int W, bool UNIT>
 __global__ void __launch_bounds__(256) k_rb_candidates(RoundCtx c, int round, int32_t* __restrict__ rb_to,
                                                        int32_t* __restrict__ rb_score, int64_t* __restrict__ rb) {
-  extern __shared__ int s_rbagg[];
-  const int k = c.k, W = c.W, lane = lane_id();
-  int* agg = s_rbagg + (threadIdx.x >> 5) * k;
-  for (int b = lane; b < k; b += 32) agg[b] = 0;
-  __syncwarp();
+  constexpr bool kLv = W <= 4;
+  constexpr int PL = UNIT ? 6 : 8, WL = kLv ? W : 1;
+  extern __shared__ ull s_rb[];  // per block: non-worsening weight, worsening count; then the masks and the warps' rows
+  const int k = c.k, lane = lane_id();
+  ull *s_w0 = s_rb, *s_cnt = s_rb + k;
+  uint32_t* s_fm = reinterpret_cast<uint32_t*>(s_cnt + k);  // feasible blocks by vertex weight
+  const int nfm = kLv ? kLvWeights * W : 0;
+  int* agg = reinterpret_cast<int*>(s_fm + nfm) + (threadIdx.x >> 5) * k;
+  for (int b = threadIdx.x; b < k; b += blockDim.x) s_w0[b] = s_cnt[b] = 0;
+  if constexpr (!kLv)
+    for (int b = lane; b < k; b += 32) agg[b] = 0;
+  for (int i = threadIdx.x >> 5; i < nfm; i += blockDim.x >> 5) {
+    const int b = 32 * (i % W) + lane;
+    const unsigned m = __ballot_sync(FULLMASK, b < k && c.bw[b] + i / W + 1 <= c.lmax[b]);
+    if (lane == 0) s_fm[i] = m;
+  }
+  __syncthreads();
   int64_t active = 0, pins = 0, cands = 0;
-  const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t v = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; v < c.n; v += warps) {
-    const int from = c.part[v];
-    if (c.bw[from] <= c.lmax[from]) {
-      if (lane == 0) rb_to[v] = -1;
-      continue;
+  for (int64_t base = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; base < c.n;
+       base += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t v = base + lane;
+    int from = 0, d = 0, wv = 0, to = -1, score = 0;
+    int64_t o0 = 0;
+    bool mine = false, heavy = false;
+    if (v < c.n) {
+      from = c.part[v];
+      if (c.bw[from] > c.lmax[from]) {
+        o0 = c.vtx_off[v];
+        const int64_t dd = c.vtx_off[v + 1] - o0;
+        ++active;
+        pins += dd;
+        d = dd > kHighDegree ? 0 : (int)dd;  // isBorderNode is false above the threshold
+        wv = c.w_v[v];
+        heavy = d > 0 && (!kLv || (int64_t)d * c.max_we >= (1 << PL));
+        mine = d > 0 && !heavy;
+      }
     }
-    const int64_t o0 = c.vtx_off[v], o1 = c.vtx_off[v + 1];
-    ++active;
-    pins += o1 - o0;
-    int internal = 0;
-    bool border = false;
-    if (o1 - o0 <= kHighDegree) {  // isBorderNode is false above the threshold
-      for (int64_t j = o0 + lane; j < o1; j += 32) {
-        const int64_t e = c.inets[j];
-        const int we = c.w_e[e];
-        const uint32_t* rec = c.conn + e * 2 * W;
-        if (!((rec[W + (from >> 5)] >> (from & 31)) & 1u)) internal += we;  // Φ(e, from) > 1
-        int lam = 0;
-        for (int w = 0; w < W; ++w) {
-          uint32_t bits = rec[w];
-          lam += __popc(bits);
-          while (bits) {
-            const int b = 32 * w + __ffs(bits) - 1;
-            bits &= bits - 1;
-            if (b != from) atomicAdd(&agg[b], we);
+    if constexpr (kLv) {
+      if (mine) {
+        uint32_t cnt[WL][PL], cand[WL];
+#pragma unroll
+        for (int t = 0; t < WL; ++t)
+#pragma unroll
+          for (int p = 0; p < PL; ++p) cnt[t][p] = 0;
+        int internal = 0;
+        const int fw = from >> 5;
+        const uint32_t fbit = 1u << (from & 31);
+        for (int j = 0; j < d; j += 4) {
+          int32_t ee[4];
+          uint32_t wd[4][WL], l1[4];
+          int we[4];
+          lv_ids<4, true>(c, o0, d, j, ee);
+          lv_records<WL, UNIT, 4, true>(c, ee, fw, fbit, wd, l1, we);
+          lv_add<WL, UNIT, PL, 4>(wd, l1, we, fbit, cnt, internal);
+        }
+        uint32_t other = 0, anyc = 0;
+#pragma unroll
+        for (int t = 0; t < WL; ++t) {
+          if (wv >= 1 && wv <= kLvWeights) {
+            cand[t] = s_fm[(wv - 1) * W + t];
+          } else {
+            cand[t] = 0;
+            for (int l = 0; l < 32; ++l) {
+              const int b = 32 * t + l;
+              if (b < k && c.bw[b] + wv <= c.lmax[b]) cand[t] |= 1u << l;
+            }
+          }
+          const uint32_t fm = t == fw ? ~fbit : ~0u;
+          uint32_t o = 0;
+#pragma unroll
+          for (int p = 0; p < PL; ++p) o |= cnt[t][p];
+          other |= o & fm;
+          cand[t] &= fm;
+          anyc |= cand[t];
+        }
+        if (other && anyc) {
+          int val = 0;  // largest penalty of a feasible block, plane by plane from the top
+#pragma unroll
+          for (int p = PL - 1; p >= 0; --p) {
+            uint32_t tt[WL], o = 0;
+#pragma unroll
+            for (int t = 0; t < WL; ++t) {
+              tt[t] = cand[t] & cnt[t][p];
+              o |= tt[t];
+            }
+            if (o) {
+#pragma unroll
+              for (int t = 0; t < WL; ++t) cand[t] = tt[t];
+              val |= 1 << p;
+            }
+          }
+#pragma unroll
+          for (int t = WL - 1; t >= 0; --t)
+            if (cand[t]) to = 32 * t + __ffs(cand[t]) - 1;
+          score = internal - val;
+        }
+      }
+    }
+    for (unsigned hm = __ballot_sync(FULLMASK, heavy); hm; hm &= hm - 1) {
+      const int q = __ffs(hm) - 1;
+      const int64_t oq = __shfl_sync(FULLMASK, o0, q);
+      const int dq = __shfl_sync(FULLMASK, d, q), fq = __shfl_sync(FULLMASK, from, q);
+      const int64_t wq = __shfl_sync(FULLMASK, wv, q);
+      int internal = 0;
+      bool border = false;
+      unsigned long long best = ~0ull;
+      auto offer = [&](int b, int pen) {  // lowest score, then lowest block
+        if (b < k && b != fq && c.bw[b] + wq <= c.lmax[b]) {
+          const unsigned long long key =
+              ((unsigned long long)((uint32_t)(internal - pen) ^ 0x80000000u) << 32) | (uint32_t)b;
+          best = key < best ? key : best;
+        }
+      };
+      if constexpr (kLv) {
+        // lane = incidence, Λ words transposed: lane l counts the blocks 32 t + l
+        int pen[WL];
+#pragma unroll
+        for (int t = 0; t < WL; ++t) pen[t] = 0;
+        for (int w0 = 0; w0 < dq; w0 += 64) {
+          uint32_t wd[2][WL];
+          int we[2], lam[2];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int j = w0 + 32 * u + lane;
+#pragma unroll
+            for (int t = 0; t < WL; ++t) wd[u][t] = 0;
+            we[u] = lam[u] = 0;
+            if (j < dq) {
+              const int64_t e = c.inets[oq + j];
+              we[u] = UNIT ? 1 : c.w_e[e];
+              const uint32_t* rec = c.conn + e * 2 * WL;
+              load_words<WL>(rec, wd[u]);
+              internal += (rec[WL + (fq >> 5)] >> (fq & 31)) & 1u ? 0 : we[u];  // Φ(e, from) > 1
+#pragma unroll
+              for (int t = 0; t < WL; ++t) lam[u] += __popc(wd[u][t]);
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            border = __any_sync(FULLMASK, lam[u] > 1) || border;
+            const Planes wp = make_planes(we[u], 32 - __clz(__reduce_or_sync(FULLMASK, (unsigned)we[u])));
+#pragma unroll
+            for (int t = 0; t < WL; ++t) pen[t] += plane_sum(wp, transpose32(wd[u][t]), we[u]);
           }
         }
-        border = border || lam > 1;
-      }
-    }
-    internal = warp_sum(internal);
-    border = __any_sync(FULLMASK, border);
-    __syncwarp();
-    const int64_t wv = c.w_v[v];
-    unsigned long long best = ~0ull;
-    for (int b = lane; b < k; b += 32) {
-      if (border && b != from && c.bw[b] + wv <= c.lmax[b]) {
-        const int sc = internal - agg[b];
-        const unsigned long long key = ((unsigned long long)((uint32_t)sc ^ 0x80000000u) << 32) | (uint32_t)b;
-        best = key < best ? key : best;
-      }
-      agg[b] = 0;
-    }
+        internal = warp_sum(internal);
+        if (border) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long y = __shfl_xor_sync(FULLMASK, best, o);
-      best = y < best ? y : best;
-    }
-    __syncwarp();
-    if (lane == 0) {
-      if (best == ~0ull) {
-        rb_to[v] = -1;
+          for (int t = 0; t < WL; ++t) offer(32 * t + lane, pen[t]);
+        }
       } else {
-        const int sc = (int)((uint32_t)(best >> 32) ^ 0x80000000u);
-        rb_to[v] = (int)(best & 0xffffffffu);
-        rb_score[v] = sc;
-        if (sc <= 0)
-          atomicAdd(reinterpret_cast<ull*>(&rb[from]), (ull)wv);
+        for (int64_t j = oq + lane; j < oq + dq; j += 32) {
+          const int64_t e = c.inets[j];
+          const int we = c.w_e[e];
+          const uint32_t* rec = c.conn + e * 2 * c.W;
+          if (!((rec[c.W + (fq >> 5)] >> (fq & 31)) & 1u)) internal += we;  // Φ(e, from) > 1
+          int lam = 0;
+          for (int w = 0; w < c.W; ++w) {
+            uint32_t bits = rec[w];
+            lam += __popc(bits);
+            while (bits) {
+              const int b = 32 * w + __ffs(bits) - 1;
+              bits &= bits - 1;
+              if (b != fq) atomicAdd(&agg[b], we);
+            }
+          }
+          border = border || lam > 1;
+        }
+        internal = warp_sum(internal);
+        border = __any_sync(FULLMASK, border);
+        __syncwarp();
+        for (int b = lane; b < k; b += 32) {
+          if (border) offer(b, agg[b]);
+          agg[b] = 0;
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long y = __shfl_xor_sync(FULLMASK, best, o);
+        best = y < best ? y : best;
+      }
+      __syncwarp();
+      if (lane == q && best != ~0ull) {
+        to = (int)(best & 0xffffffffu);
+        score = (int)((uint32_t)(best >> 32) ^ 0x80000000u);
+      }
+    }
+    if (v < c.n) {
+      rb_to[v] = to;
+      if (to >= 0) {
+        rb_score[v] = score;
+        if (score <= 0)
+          atomicAdd(&s_w0[from], (ull)(int64_t)wv);
         else
-          atomicAdd(reinterpret_cast<ull*>(&rb[k + from]), 1ull);
+          atomicAdd(&s_cnt[from], 1ull);
         ++cands;
       }
     }
   }
-  if (lane == 0) {
+  active = block_sum_i64(active);
+  pins = block_sum_i64(pins);
+  cands = block_sum_i64(cands);
+  if (threadIdx.x == 0) {
     int64_t* st = c.stats + (int64_t)round * kStats;
     if (active) atomicAdd(reinterpret_cast<ull*>(&st[kStActive]), (ull)active);
     if (pins) atomicAdd(reinterpret_cast<ull*>(&st[kStPins]), (ull)pins);
     if (cands) atomicAdd(reinterpret_cast<ull*>(&st[kStCands]), (ull)cands);
+  }
+  __syncthreads();
+  for (int b = threadIdx.x; b < k; b += blockDim.x) {
+    if (s_w0[b]) atomicAdd(reinterpret_cast<ull*>(&rb[b]), s_w0[b]);
+    if (s_cnt[b]) atomicAdd(reinterpret_cast<ull*>(&rb[k + b]), s_cnt[b]);
   }
 }
 
@@ -2586,7 +2726,11 @@ __global__ void __launch_bounds__(kSelThreads) k_rb_src_select(RoundCtx c, int64
 // totals); the last CTA plans the target-side selection.
 __global__ void k_rb_emit(RoundCtx c, const int32_t* __restrict__ rb_to, const int32_t* __restrict__ rb_score,
                           const int64_t* __restrict__ rb) {
+  extern __shared__ ull s_emit[];  // this CTA's candidate weight and count by target, weight by source
   const int k = c.k;
+  ull *s_in = s_emit, *s_cnt = s_emit + k, *s_out = s_emit + 2 * k;
+  for (int b = threadIdx.x; b < 3 * k; b += blockDim.x) s_emit[b] = 0;
+  __syncthreads();
   const uint64_t* thr = reinterpret_cast<const uint64_t*>(rb + 4 * k + 1);
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < c.n; v += (int64_t)gridDim.x * blockDim.x) {
     const int from = c.part[v];
@@ -2600,12 +2744,20 @@ __global__ void k_rb_emit(RoundCtx c, const int32_t* __restrict__ rb_to, const i
         r.x = to;
         r.y = sc;
         const int64_t wv = c.w_v[v];
-        atomicAdd(reinterpret_cast<ull*>(&c.in_w[to]), (ull)wv);
-        atomicAdd(reinterpret_cast<ull*>(&c.in_cnt[to]), 1ull);
-        atomicAdd(reinterpret_cast<ull*>(&c.cand_out[from]), (ull)wv);
+        atomicAdd(&s_in[to], (ull)wv);
+        atomicAdd(&s_cnt[to], 1ull);
+        atomicAdd(&s_out[from], (ull)wv);
       }
     }
     c.rec[v] = r;
+  }
+  __syncthreads();
+  for (int b = threadIdx.x; b < k; b += blockDim.x) {
+    if (s_cnt[b]) {
+      atomicAdd(reinterpret_cast<ull*>(&c.in_w[b]), s_in[b]);
+      atomicAdd(reinterpret_cast<ull*>(&c.in_cnt[b]), s_cnt[b]);
+    }
+    if (s_out[b]) atomicAdd(reinterpret_cast<ull*>(&c.cand_out[b]), s_out[b]);
   }
   if (last_cta(&c.scal[kDone])) plan_to(c);
 }
@@ -2690,10 +2842,14 @@ cudaError_t launch_rebalance_round(const Launch& L, const RoundCtx& c, int round
   const int k = c.k;
   cudaError_t e = cudaMemsetAsync(rb, 0, sizeof(int64_t) * 2 * k, L.st);
   if (e != cudaSuccess) return e;
-  const size_t smem = sizeof(int) * k * 8;
-  allow_dyn_smem(k_rb_candidates, smem);
-  k_rb_candidates<<<grid_for(L, c.n * 32, 256), 256, smem, L.st>>>(c, round, rb_to, rb_score, rb);
-  LAUNCHED("k_rb_candidates");
+  LPGPU_DISPATCH_W(c.W, {
+    const size_t smem = sizeof(ull) * 2 * k + (kW <= 4 ? sizeof(uint32_t) * kLvWeights * kW : 0) + (kW <= 4 ? 0 : sizeof(int) * k * 8);
+    auto kern = c.unit_nets ? k_rb_candidates<kW, true> : k_rb_candidates<kW, false>;
+    allow_dyn_smem(kern, smem);
+    kern<<<grid_for(L, c.n, 256, occupancy((const void*)kern, 256, smem)), 256, smem, L.st>>>(c, round, rb_to, rb_score,
+                                                                                           rb);
+    LAUNCHED("k_rb_candidates");
+  });
   k_rb_src_plan<<<1, 1024, 0, L.st>>>(c, rb);
   LAUNCHED("k_rb_src_plan");
   const int g = grid_for(L, c.n, 256);
@@ -2702,7 +2858,7 @@ cudaError_t launch_rebalance_round(const Launch& L, const RoundCtx& c, int round
   allow_dyn_smem(k_rb_src_select, kSelSmem);
   k_rb_src_select<<<(unsigned)std::min<int64_t>(k, 4 * (int64_t)L.num_sms), kSelThreads, kSelSmem, L.st>>>(c, rb);
   LAUNCHED("k_rb_src_select");
-  k_rb_emit<<<g, 256, 0, L.st>>>(c, rb_to, rb_score, rb);
+  k_rb_emit<<<g, 256, sizeof(ull) * 3 * k, L.st>>>(c, rb_to, rb_score, rb);
   LAUNCHED("k_rb_emit");
   // the LP target-side selection, source floor and commit of one sub-round
   k_bin_moves<<<grid_for(L, c.n, kBinThreads), kBinThreads, 0, L.st>>>(c, 0);
