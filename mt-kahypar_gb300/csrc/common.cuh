@@ -74,7 +74,7 @@ enum Scalar : int {
   kAnyOverFrom = 2,
   kKm1 = 3,        // km1 accumulator (metrics)
   kCut = 4,        // cut accumulator (metrics)
-  kError = 5,      // device-side error flag
+  kPinTiles = 5,   // tile counter of the pin counts
   kApplyDelta = 6, // apply_moves delta
   kDeltaRb = 7,    // delta of a sub-round rollback
   kEpoch = 8,      // activation stamp of the current round

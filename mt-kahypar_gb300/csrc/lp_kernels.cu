@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <type_traits>
 #include <utility>
 
 #include "lp_device.cuh"
@@ -165,34 +166,57 @@ __global__ void k_degree_hist(int64_t n, const int64_t* __restrict__ cnt, int64_
 }
 
 // Every pin writes its net id into its slot of its vertex's incident-net list
-// (list start + the rank k_count_pins returned). A warp takes the next 32 nets
-// from a counter and walks their pins in packed 32-pin groups (nets of more
-// than 32 pins alone, 32 pins at a time), so small nets keep every lane busy.
-// Taking nets in order keeps the nets in flight close together, so where a
-// hypergraph's pins are local, the partly written 32-byte sectors of their
-// vertices' lists stay in L2 until they are complete (a grid-stride loop lets
-// warps drift apart over nets of uneven size).
+// (list start + the rank k_count_pins returned). A CTA takes the next kScatterNets
+// nets from a counter; their pins are one contiguous range, over which its
+// threads spread (the net of a pin by binary search in the tile's offsets), four
+// pins in flight each. Taking tiles in order keeps the nets in flight close
+// together, so where a hypergraph's pins are local, the partly written 32-byte
+// sectors of their vertices' lists stay in L2 until they are complete (a
+// grid-stride loop lets CTAs drift apart over nets of uneven size). A warp per 32
+// nets walked its pins in dependent 32-pin groups: 400K vertices 99 -> 43 us,
+// row-net 4.2M 917 -> 680 us.
+constexpr int kScatterNets = 128;
 __global__ void __launch_bounds__(256) k_scatter_incidence(int64_t m, const int64_t* __restrict__ net_off,
                                                            const int32_t* __restrict__ pins,
                                                            const int64_t* __restrict__ vtx_off,
                                                            const int32_t* __restrict__ rank,
                                                            int32_t* __restrict__ inets, ull* next_net) {
-  __shared__ unsigned char s_own[256];
-  const int lane = lane_id();
-  unsigned char* own = s_own + (threadIdx.x & ~31);
+  __shared__ int64_t s_off[kScatterNets + 1];
+  __shared__ ull s_next;
   for (;;) {
-    ull b = 0;
-    if (lane == 0) b = atomicAdd(next_net, 32ull);
-    const int64_t base = (int64_t)__shfl_sync(FULLMASK, b, 0);
-    if (base >= m) break;
-    const int64_t e = base + lane;
-    const bool sel = e < m;
-    const int64_t o0 = sel ? net_off[e] : 0;
-    const int deg = sel ? (int)(net_off[e + 1] - o0) : 0;
-    packed_incidences(sel, o0, deg, own, [&](bool has, int ow, int64_t j) -> int {
-      if (has) inets[vtx_off[pins[j]] + rank[j]] = (int32_t)(base + ow);
-      return 0;
-    });
+    if (threadIdx.x == 0) s_next = atomicAdd(next_net, (ull)kScatterNets);
+    __syncthreads();
+    const int64_t e0 = (int64_t)s_next;
+    if (e0 >= m) break;
+    const int nets = (int)(m - e0 < kScatterNets ? m - e0 : kScatterNets);
+    for (int i = threadIdx.x; i <= nets; i += blockDim.x) s_off[i] = net_off[e0 + i];
+    __syncthreads();
+    const int64_t p1 = s_off[nets];
+    for (int64_t j0 = s_off[0] + threadIdx.x; j0 < p1; j0 += 4 * (int64_t)blockDim.x) {
+      int64_t at[4];
+      int r[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int64_t j = j0 + u * (int64_t)blockDim.x;
+        at[u] = j < p1 ? pins[j] : -1;
+        r[u] = j < p1 ? rank[j] : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (at[u] >= 0) at[u] = vtx_off[at[u]] + r[u];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (at[u] < 0) continue;
+        const int64_t j = j0 + u * (int64_t)blockDim.x;
+        int lo = 0, hi = nets - 1;  // the last net that starts at or before j
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (s_off[mid] <= j) lo = mid; else hi = mid - 1;
+        }
+        inets[at[u]] = (int32_t)(e0 + lo);
+      }
+    }
+    __syncthreads();  // the tile's offsets are read
   }
 }
 
@@ -218,7 +242,8 @@ cudaError_t launch_build_incidence(const Launch& L, int64_t n, int64_t m, int64_
   if (m > 0) {
     ull* next_net = reinterpret_cast<ull*>(scan_tmp);  // free again after the scan
     if ((e = cudaMemsetAsync(next_net, 0, sizeof(ull), L.st)) != cudaSuccess) return e;
-    k_scatter_incidence<<<grid_for(L, m, 256, 8), 256, 0, L.st>>>(m, net_off, pins, vtx_off, rank, inets, next_net);
+    k_scatter_incidence<<<grid_for(L, (m + kScatterNets - 1) / kScatterNets, 1, 8), 256, 0, L.st>>>(
+        m, net_off, pins, vtx_off, rank, inets, next_net);
     LAUNCHED("k_scatter_incidence");
   }
   return cudaGetLastError();
@@ -264,129 +289,146 @@ __global__ void k_block_weights(RoundCtx c) {
 
 
 // Φ, Λ and Λ1 (blocks holding exactly one pin of the net) from scratch
-// (initializePinCountInPart, h:1086-1110), fused with the km1 / cut sums. A
-// warp takes 32 nets and zeroes their Φ rows and records before filling them. Nets of up to 32 pins are packed
-// into 32-pin groups (lane = pin): lanes with the same (net, block) find each
-// other with a match, and the lowest writes Φ(e, b) and sets the Λ / Λ1 bits;
-// λ(e) is the number of such lanes. Larger nets are counted one at a time in a
-// per-warp shared k-bin histogram. Net e's record is conn[e * 2W .. e * 2W + 2W):
-// W words of Λ(e), then W words of Λ1(e).
-__global__ void __launch_bounds__(256) k_pin_counts(RoundCtx c) {
-  extern __shared__ int s_hist[];
-  __shared__ unsigned char s_own[256];
+// (initializePinCountInPart, h:1086-1110), fused with the km1 / cut sums. A CTA
+// takes `tn` consecutive nets, whose pins, Φ rows and records are one contiguous
+// range each: the threads spread over the pins (the net of a pin by binary
+// search in the tile's offsets), count in an image of the Φ rows in shared
+// memory, and the image and the records are then written in whole lines, zeros
+// included. The count an atomic returns drives the bits as in the commit: Λ when
+// it leaves 0, Λ1 whenever it enters or leaves 1. Four pins per thread are in
+// flight and a large net keeps the whole CTA busy; one warp per 32 nets walked
+// about ten dependent 32-pin groups one after another and wrote single entries.
+// initializePartition, before -> after: 1M vertices k = 32 153 -> 130 us, row-net
+// 1M k = 61 143 -> 129, 250,007 k = 300 93 -> 81, 16,384 21.5 -> 17.3; row-net
+// 4.2M k = 128 527 -> 552 (1.1 GB of Φ rows, mostly zeros). Net e's record is conn[e * 2W .. e * 2W + 2W): W words of Λ(e),
+// then W words of Λ1(e).
+constexpr int kPinTile = 256;  // threads per CTA
+constexpr int kPinNets = 256;  // most nets per tile
+template <bool PHI16, bool BATCHED>
+__global__ void __launch_bounds__(kPinTile) k_pin_counts(RoundCtx c, int tn) {
+  extern __shared__ __align__(16) unsigned char s_pin[];
+  // offsets inside a tile: 16-bit entries mean nets of fewer than 2^16 pins
+  using Off = typename std::conditional<PHI16, int32_t, int64_t>::type;
+  constexpr int esz = PHI16 ? 2 : 4;
   const int k = c.kmax, W = c.W;
-  int* hist = s_hist + (threadIdx.x >> 5) * k;
-  unsigned char* own = s_own + (threadIdx.x & ~31);
-  const int lane = lane_id();
-  for (int b = lane; b < k; b += 32) hist[b] = 0;
-  __syncwarp();
+  const int row_words = (tn * k * esz + 15) >> 4 << 2;  // the image, in whole 16-byte units
+  uint32_t* s_phi = reinterpret_cast<uint32_t*>(s_pin);
+  uint32_t* s_rec = s_phi + row_words;
+  Off* s_off = reinterpret_cast<Off*>(s_rec + ((tn * 2 * W + 3) & ~3));
+  int* s_bo = reinterpret_cast<int*>(s_off + tn + 1);
   int64_t km1 = 0, cut = 0;
-  for (int64_t base = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; base < c.m;
-       base += (int64_t)gridDim.x * blockDim.x) {
-    // The warp first zeroes the Φ rows and Λ records of its 32 nets (one
-    // contiguous range each), so every sector it then changes is complete in
-    // L2 and no partly written sector is read back from DRAM.
-    {
-      const int64_t e_end = base + 32 < c.m ? base + 32 : c.m;
-      const int esz = c.phi16 ? 2 : 4;
-      unsigned char* p0 = reinterpret_cast<unsigned char*>(c.phi) + base * k * esz;
-      const int64_t bytes = ((e_end - base) * k * esz + 3) & ~(int64_t)3;  // Φ is allocated in whole words
-      const int64_t n16 = bytes >> 4;
-      for (int64_t i = lane; i < n16; i += 32) reinterpret_cast<uint4*>(p0)[i] = make_uint4(0, 0, 0, 0);
-      for (int64_t i = (n16 << 2) + lane; i < (bytes >> 2); i += 32) reinterpret_cast<uint32_t*>(p0)[i] = 0;
-      for (int64_t i = base * 2 * W + lane; i < e_end * 2 * W; i += 32) c.conn[i] = 0;
-      __syncwarp();
+  __shared__ int64_t s_tile;
+  // tiles from a counter: power-law nets make them uneven
+  for (;;) {
+    if (threadIdx.x == 0) s_tile = (int64_t)atomicAdd(reinterpret_cast<ull*>(&c.scal[kPinTiles]), 1ull) * tn;
+    __syncthreads();
+    const int64_t e0 = s_tile;
+    if (e0 >= c.m) break;
+    const int nets = (int)(c.m - e0 < tn ? c.m - e0 : tn);
+    for (int i = threadIdx.x; i < (row_words >> 2); i += kPinTile) reinterpret_cast<uint4*>(s_phi)[i] = make_uint4(0, 0, 0, 0);
+    const int64_t p0 = c.net_off[e0];
+    for (int i = threadIdx.x; i < nets * 2 * W; i += kPinTile) s_rec[i] = 0;
+    for (int i = threadIdx.x; i <= nets; i += kPinTile) {
+      const int64_t o = c.net_off[e0 + i];
+      s_off[i] = (Off)(o - p0);
+      if (BATCHED && i < nets) s_bo[i] = c.net_off[e0 + i + 1] > o ? block_offset(c, c.pins[o]) : 0;
     }
-    const int64_t e = base + lane;
-    int64_t b0 = 0;
-    int deg = 0, bo = 0;
-    if (e < c.m) {
-      b0 = c.net_off[e];
-      const int64_t d = c.net_off[e + 1] - b0;
-      deg = d > INT32_MAX ? INT32_MAX : (int)d;
-      if (c.batched && d > 0) bo = block_offset(c, c.pins[b0]);
-    }
-    const bool small = deg >= 1 && deg <= 32;
-    const int lam = packed_incidences(small, b0, deg, own, [&](bool has, int ow, int64_t j) -> int {
-      const int64_t e_ow = __shfl_sync(FULLMASK, e, ow);
-      const int bo_ow = __shfl_sync(FULLMASK, bo, ow);
-      int b = 0;
-      unsigned key = 0x80000000u | (unsigned)lane;  // lanes without a pin match nobody
-      if (has) {
-        b = c.part[c.pins[j]] - bo_ow;
-        key = ((unsigned)ow << 11) | (unsigned)b;
-      }
-      const unsigned peers = __match_any_sync(FULLMASK, key);
-      const bool leader = has && __ffs(peers) - 1 == lane;
-      if (leader) {
-        const int cnt = __popc(peers);
-        phi_set(c, e_ow * k + b, cnt);
-        uint32_t* rec = c.conn + e_ow * 2 * W;
-        atomicOr(&rec[b >> 5], 1u << (b & 31));
-        if (cnt == 1) atomicOr(&rec[W + (b >> 5)], 1u << (b & 31));
-      }
-      return leader ? 1 : 0;
-    });
-    if (small) {
-      const int64_t we = c.w_e[e];
-      km1 += (int64_t)(lam > 1 ? lam - 1 : 0) * we;
-      cut += lam > 1 ? we : 0;
-    }
-    unsigned bigm = __ballot_sync(FULLMASK, deg > 32);
-    while (bigm) {
-      const int q = __ffs(bigm) - 1;
-      bigm &= bigm - 1;
-      const int64_t eq = __shfl_sync(FULLMASK, e, q);
-      const int64_t bq = __shfl_sync(FULLMASK, b0, q);
-      const int dq = __shfl_sync(FULLMASK, deg, q);
-      const int boq = __shfl_sync(FULLMASK, bo, q);
-      for (int64_t i = bq + lane; i < bq + dq; i += 32) atomicAdd(&hist[c.part[c.pins[i]] - boq], 1);
-      __syncwarp();
-      int lq = 0;
-      for (int w = 0; w < W; ++w) {
-        const int b = w * 32 + lane;
-        int cnt = 0;
-        if (b < k) {
-          cnt = hist[b];
-          hist[b] = 0;
-          if (cnt) phi_set(c, eq * k + b, cnt);
+    __syncthreads();
+    const Off p1 = s_off[nets];
+    const int32_t* pins = c.pins + p0;
+    for (Off j0 = threadIdx.x; j0 < p1; j0 += 4 * kPinTile) {
+      int b[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) b[u] = j0 + u * kPinTile < p1 ? pins[j0 + u * kPinTile] : -1;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (b[u] >= 0) b[u] = c.part[b[u]];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (b[u] < 0) continue;
+        const Off j = j0 + u * kPinTile;
+        int lo = 0, hi = nets - 1;  // the last net that starts at or before j
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (s_off[mid] <= j) lo = mid; else hi = mid - 1;
         }
-        const unsigned bits = __ballot_sync(FULLMASK, cnt > 0);
-        const unsigned ones = __ballot_sync(FULLMASK, cnt == 1);
-        if (lane == 0) {
-          c.conn[eq * 2 * W + w] = bits;
-          c.conn[eq * 2 * W + W + w] = ones;
+        const int blk = BATCHED ? b[u] - s_bo[lo] : b[u], i = lo * k + blk;
+        unsigned old;
+        if constexpr (PHI16) {
+          const int sh = (i & 1) * 16;
+          old = (atomicAdd(&s_phi[i >> 1], 1u << sh) >> sh) & 0xFFFFu;
+        } else {
+          old = atomicAdd(&s_phi[i], 1u);
         }
-        lq += __popc(bits);
-      }
-      __syncwarp();
-      if (lane == 0) {
-        const int64_t we = c.w_e[eq];
-        km1 += (int64_t)(lq > 1 ? lq - 1 : 0) * we;
-        cut += lq > 1 ? we : 0;
+        if (old <= 1) {
+          uint32_t* rec = s_rec + lo * 2 * W + (blk >> 5);
+          if (old == 0) atomicOr(rec, 1u << (blk & 31));
+          atomicXor(rec + W, 1u << (blk & 31));
+        }
       }
     }
+    __syncthreads();
+    // whole lines out: Φ is allocated in whole words, a tile starts on a word
+    unsigned char* out = reinterpret_cast<unsigned char*>(c.phi) + e0 * k * esz;
+    const int64_t words = ((int64_t)nets * k * esz + 3) >> 2;
+    if ((reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+      for (int i = threadIdx.x; i < (words >> 2); i += kPinTile)
+        reinterpret_cast<uint4*>(out)[i] = reinterpret_cast<const uint4*>(s_phi)[i];
+      for (int i = (int)(words & ~(int64_t)3) + threadIdx.x; i < words; i += kPinTile)
+        reinterpret_cast<uint32_t*>(out)[i] = s_phi[i];
+    } else {
+      for (int i = threadIdx.x; i < words; i += kPinTile) reinterpret_cast<uint32_t*>(out)[i] = s_phi[i];
+    }
+    for (int i = threadIdx.x; i < nets * 2 * W; i += kPinTile) c.conn[e0 * 2 * W + i] = s_rec[i];
+    for (int i = threadIdx.x; i < nets; i += kPinTile) {
+      int lam = 0;
+      for (int w = 0; w < W; ++w) lam += __popc(s_rec[i * 2 * W + w]);
+      if (lam > 1) {
+        const int64_t we = c.w_e[e0 + i];
+        km1 += (int64_t)(lam - 1) * we;
+        cut += we;
+      }
+    }
+    __syncthreads();  // the image is cleared for the next tile
   }
   km1 = block_sum_i64(km1);
   cut = block_sum_i64(cut);
   if (threadIdx.x == 0) {
-    atomicAdd(reinterpret_cast<ull*>(&c.scal[kKm1]), (ull)km1);
-    atomicAdd(reinterpret_cast<ull*>(&c.scal[kCut]), (ull)cut);
+    if (km1) atomicAdd(reinterpret_cast<ull*>(&c.scal[kKm1]), (ull)km1);
+    if (cut) atomicAdd(reinterpret_cast<ull*>(&c.scal[kCut]), (ull)cut);
   }
+}
+
+// Nets per tile: an image of at most 24 KB (initializePartition of row-net 4.2M,
+// k = 128 / geometric 250,007, k = 300: 8 KB 722 / 124 us, 16 KB 544 / 91, 24 KB
+// 552 / 81, 32 KB 554 / 82), an even number so that every tile starts on a word
+// of 16-bit entries, and at least two tiles per SM where the nets allow it.
+static int pin_tile(const Launch& L, const RoundCtx& c) {
+  const int64_t row = (int64_t)c.kmax * (c.phi16 ? 2 : 4);
+  int64_t tn = std::min<int64_t>(kPinNets, std::max<int64_t>(2, 24576 / row));
+  tn = std::min(tn, std::max<int64_t>(8, c.m / (2 * (int64_t)L.num_sms)));
+  return (int)(tn & ~(int64_t)1);
 }
 
 cudaError_t launch_init_partition(const Launch& L, const RoundCtx& c) {
   cudaError_t e;
   if ((e = cudaMemsetAsync(c.bw, 0, sizeof(int64_t) * c.k, L.st)) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(c.scal + kKm1, 0, sizeof(int64_t) * 2, L.st)) != cudaSuccess) return e;
+  // km1, cut and the tile counter
+  static_assert(kCut == kKm1 + 1 && kPinTiles == kKm1 + 2, "cleared together");
+  if ((e = cudaMemsetAsync(c.scal + kKm1, 0, sizeof(int64_t) * 3, L.st)) != cudaSuccess) return e;
   if (c.n > 0) {
-    k_block_weights<<<grid_for(L, c.n, 256), 256, c.batched ? 0 : sizeof(ull) * c.k, L.st>>>(c);
+    k_block_weights<<<grid_for(L, c.n, 256, 8), 256, c.batched ? 0 : sizeof(ull) * c.k, L.st>>>(c);
     LAUNCHED("k_block_weights");
   }
   if (c.m > 0) {
     // k_pin_counts writes all of Φ and the Λ records, zeros included
-    const size_t smem = sizeof(int) * c.kmax * 8;
-    k_pin_counts<<<grid_for(L, c.m, 256, occupancy((const void*)k_pin_counts, 256, smem)), 256, smem, L.st>>>(c);
+    const int tn = pin_tile(L, c);
+    const size_t smem = (((size_t)tn * c.kmax * (c.phi16 ? 2 : 4) + 15) & ~size_t(15)) +
+                        4 * (((size_t)tn * 2 * c.W + 3) & ~size_t(3)) + sizeof(int64_t) * (tn + 1) + sizeof(int) * tn;
+    auto kern = c.phi16 ? (c.batched ? k_pin_counts<true, true> : k_pin_counts<true, false>)
+                        : (c.batched ? k_pin_counts<false, true> : k_pin_counts<false, false>);
+    kern<<<grid_for(L, (c.m + tn - 1) / tn, 1, occupancy((const void*)kern, kPinTile, smem)), kPinTile, smem, L.st>>>(
+        c, tn);
     LAUNCHED("k_pin_counts");
   }
   return cudaSuccess;
