@@ -977,11 +977,13 @@ static lpgpu_tuning session_tuning(const lpgpu_session* s) {
 //
 // CTAs of the team and of an SM by the number of vertices. Measured (GB300,
 // whole refine call in us, one CTA / cluster of 16 / one CTA per SM / two per
-// SM; multi-launch pipeline in brackets): 1,024 vertices 577 / 701 / - / -
-// [1,134]; 4,096: 979 / 915 / - / - [1,428]; 16,384: 2,462 / 995 / 966 / -
-// [1,377]; 131,071 (k = 64): - / 4,511 / 2,118 / 2,250 [3,370]; 1M (k = 32):
-// - / 25,213 / 5,195 / 4,899 [5,727]; 4.2M (k = 128): - / - / 12,145 / 11,361
-// [11,554].
+// SM; multi-launch pipeline in brackets): 1,024 vertices (k = 2) 467 / 556 / - /
+// - [1,094]; 2,048 (k = 4) 608 / 617 / - / -; 4,096 (k = 2) 976 / 681 / - / -;
+// 10,007 (k = 8) 1,634 / 797 / 888 / -; 16,384 (k = 64, weighted) 5,508 / 1,852 /
+// 1,660 / - [2,917]; 65,536 (k = 32) - / 2,678 / 1,703 / 2,015; 262,144 (k = 16)
+// - / 5,877 / 2,184 / 2,242 [3,203]; 524,288 (k = 32) - / 11,319 / 2,924 / 2,887,
+// unweighted k = 8 1,777 / 1,903; 1M (k = 32) - / - / 5,195 / 4,641 [5,563]; 4.2M
+// (k = 128) - / - / 12,145 / 11,015 [11,371].
 struct TeamShape {
   int per_sm;  // kernel build: resident CTAs per SM
   int unroll;
@@ -989,9 +991,9 @@ struct TeamShape {
 };
 static TeamShape team_shape(int64_t n, int num_sms, int in_flight) {
   if (n <= 2048) return {1, 4, 1};
-  if (n <= 16384) return {1, 4, kTeamMaxCluster};
+  if (n <= 12288) return {1, 4, kTeamMaxCluster};
   if (in_flight > 1) return {2, 4, 2 * num_sms / std::min(in_flight, 4)};
-  return {n < (int64_t)1 << 19 ? 1 : 2, 4, 0};
+  return {n < 655360 ? 1 : 2, 4, 0};
 }
 
 // Refine calls in progress per device: a cooperative grid over the whole GPU

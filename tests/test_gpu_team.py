@@ -30,7 +30,7 @@ def _same(a, b):
 # vertices: no chunk, one partial chunk, whole chunks, one CTA / cluster / grid limits, fewer chunks than CTAs
 @pytest.mark.parametrize("n,k,weighted", [
     (1, 1, False), (7, 3, True), (32, 2, False), (33, 4, True), (2048, 128, True), (2049, 65, False),
-    (2080, 2, True), (16384, 2, False), (16385, 33, True), (20000, 128, False), (70001, 64, True),
+    (2080, 2, True), (12288, 2, False), (12289, 33, True), (16384, 2, False), (20000, 128, False), (70001, 64, True),
     # more than 128 blocks: two, four or eight lanes per vertex
     (1000, 129, True), (1500, 1024, False), (9000, 300, False), (30000, 300, True), (40000, 1024, True),
     (50000, 513, False), (300, 256, False)])
@@ -93,7 +93,7 @@ def test_team_node_list(lp):
           _refine(lp, inst.hg, 16, inst.part, nodes=nodes, flags=lp.FLAG_MULTI_LAUNCH))
 
 
-@pytest.mark.parametrize("n,size,skew", [(16384, 40, 0.0), (16384, 12, 0.6), (1800, 30, 0.0), (2048, 7, 0.0)])
+@pytest.mark.parametrize("n,size,skew", [(12288, 50, 0.0), (12288, 16, 0.6), (1800, 30, 0.0), (2048, 7, 0.0), (16384, 40, 0.0)])
 def test_team_resident_part(lp, n, size, skew):
     """Instances whose arrays do not fit a CTA's shared memory, that fit in all
     but one CTA of the team (its chunks hold most incidences), or in part."""
