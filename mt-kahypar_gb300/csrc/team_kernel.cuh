@@ -68,7 +68,10 @@ struct TeamGlob {
   __device__ ull* count(int r) const { return reinterpret_cast<ull*>(thr_from() + K) + r * kMaxSubrounds; }
 };
 
-constexpr int kTeamStage = 2048;  // selection keys a CTA holds in registers and shared memory
+// Selection keys a CTA holds in registers and shared memory; more leave the L1
+// cache less (1M vertices, k = 32, 1,024 / 2,048 / 4,096 keys: 4,575 / 4,558 /
+// 4,895 us; 131,071 1,975 / 1,986 / 2,060; row-net 4.2M 10,995 / 11,020 / 11,370).
+constexpr int kTeamStage = 1024;
 constexpr int kSelBits = 11;      // key bits per pass of the CTA selection
 constexpr size_t kSelArea = (size_t)kTeamStage * 12 + (sizeof(unsigned) << kSelBits);
 constexpr size_t kWarpSelArea = (size_t)kTeamWarps * 256 * sizeof(unsigned);
@@ -825,9 +828,10 @@ __device__ void team_heavy(const PxParams& P, const RoundCtx& c, const Team& tm,
   }
 }
 
-// Incidences a thread handles per step of the CTA-flat walks: one CTA per SM
-// has 512 threads to hide the latency of an L2 round trip with.
-constexpr int kTeamGroup = 4;
+// Incidences a thread handles per step of the CTA-flat walks (1M vertices, k =
+// 32: 1 4,596, 2 4,558, 4 4,648, 8 5,126 us per refine; row-net 4.2M 10,980 /
+// 11,010 / 11,030 / 11,400).
+constexpr int kTeamGroup = 2;
 
 // Collects into f the candidates [c0, c0 + kFlatItems) of the CTA's list that
 // pass `take(i, rec)`, as moves from `from` to `to` (back: the reverse), and
