@@ -6,6 +6,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <type_traits>
 #include <string>
 #include <vector>
 
@@ -177,12 +178,12 @@ struct lpgpu_session_s {
   int32_t num_inst = 0;
   int32_t kmax = 0;
   std::vector<int64_t> h_inst_voff, h_inst_noff, h_inst_weight;
-  std::vector<int64_t> h_inst_pins;  // pins of every instance (work estimate of the persistent rounds)
+  std::vector<int64_t> h_inst_pins;  // pins of every instance (work estimate of the team rounds)
   std::vector<int32_t> h_inst_boff, h_inst_k;
-  // persistent rounds: instance descriptors, work order, what they were built from
+  // team rounds: instance descriptors, work order, the rule it follows
   DevBuf<PxInst> px;
   DevBuf<int32_t> px_order;
-  std::vector<int64_t> px_key;
+  int px_order_rule = 0;
   bool has_tuning = false;
   lpgpu_tuning tuning{};
   std::vector<PxInst> h_px;  // host copy of the descriptors
@@ -348,7 +349,7 @@ struct lpgpu_session_s {
     px_order.release(&mem);
     team.release(&mem);
     rep.release(&mem);
-    px_key.clear();
+    h_px.clear();
     vinst.release(&mem);
     inst_voff.release(&mem);
     inst_noff.release(&mem);
@@ -1010,16 +1011,11 @@ struct InFlight {
   ~InFlight() { c.fetch_sub(1); }
 };
 
-// Instance descriptors of the persistent rounds over the session's current
-// buffers, and the work order (rebuilt when a buffer or the order changed).
+// Instance descriptors of the team rounds over the session's current state,
+// and the work order. They are compared by content with what the device holds:
+// a session that takes another input can keep all its buffers and sizes.
 static lpgpu_status build_px(lpgpu_session* s, int order) {
   const int32_t I = s->batched ? s->num_inst : 1;
-  const std::vector<int64_t> key = {
-      (int64_t)s->stats.p, (int64_t)s->part.p, (int64_t)s->phi.p,  (int64_t)s->conn.p,      (int64_t)s->bw.p,
-      (int64_t)s->rec.p,   (int64_t)s->seg_key.p, (int64_t)s->revl.p, (int64_t)s->next_flag.p, (int64_t)s->net_off.p,
-      (int64_t)s->inets.p, (int64_t)s->lmax.p, (int64_t)s->list.p, order, s->kmax, s->k, s->W, s->n, s->m, I, s->max_we,
-      s->unit_nets ? 1 : 0};
-  if (s->px.p && s->px_key == key) return LPGPU_OK;
   std::vector<PxInst> h(I);
   for (int32_t i = 0; i < I; ++i) {
     PxInst& x = h[i];
@@ -1057,6 +1053,11 @@ static lpgpu_status build_px(lpgpu_session* s, int order) {
     x.max_we = s->max_we;
     x.round = 0;
   }
+  static_assert(std::is_trivially_copyable<PxInst>::value && sizeof(PxInst) % 8 == 0, "compared bytewise");
+  if (s->px.p && s->px_order_rule == order && s->h_px.size() == h.size() &&
+      std::memcmp(s->h_px.data(), h.data(), sizeof(PxInst) * h.size()) == 0)
+    return LPGPU_OK;
+  s->h_px.clear();
   std::vector<int32_t> ord(I);
   for (int32_t i = 0; i < I; ++i) ord[i] = i;
   if (order == 0)  // largest instance first: the longest jobs start first on the work queue
@@ -1066,10 +1067,10 @@ static lpgpu_status build_px(lpgpu_session* s, int order) {
   CK(s->px.alloc(I, fp));
   CK(s->px_order.alloc(I, fp));
   CK(cudaMemcpyAsync(s->px.p, h.data(), sizeof(PxInst) * I, cudaMemcpyHostToDevice, s->st));
-  s->h_px = h;
   CK(cudaMemcpyAsync(s->px_order.p, ord.data(), sizeof(int32_t) * I, cudaMemcpyHostToDevice, s->st));
   CK(cudaStreamSynchronize(s->st));
-  s->px_key = key;
+  s->h_px = std::move(h);
+  s->px_order_rule = order;
   return LPGPU_OK;
 }
 
@@ -1142,8 +1143,8 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
   for (int64_t i = 0; i < num_nodes; ++i)
     if (nodes[i] < 0 || nodes[i] >= s->n) return invalid("refinement node out of range");
   // the team rounds, forced by the flag, chosen by the tuning or, where no tuning
-  // applies, by default; the multi-launch pipeline otherwise (k above the team
-  // kernel's, per-phase timing, forced or tuned)
+  // applies, by default; the multi-launch pipeline otherwise (per-phase timing, forced
+  // or tuned)
   lpgpu_tuning tu;
   const bool tuned = find_tuning(s, &tu);
   const int kmax = s->batched ? s->kmax : s->k;
@@ -1323,7 +1324,7 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
   return LPGPU_OK;
 }
 
-// ---- stepped refinement: one persistent round of many sessions per launch
+// ---- stepped refinement: one team round of many sessions per launch
 
 lpgpu_status lpgpu_session_begin_rounds(lpgpu_session* s, const lpgpu_config* cfg_in) {
   lpgpu_status ps = need_part(s);

@@ -111,3 +111,42 @@ def test_team_resident_part(lp, n, size, skew):
                         np.ones(m, np.int32))
     part = rng.integers(0, 61, n).astype(np.int32)
     _same(_refine(lp, hg, 61, part, rounds=3), _refine(lp, hg, 61, part, rounds=3, flags=lp.FLAG_MULTI_LAUNCH))
+
+
+# a session that takes another input with all its buffers and sizes as they were
+@pytest.mark.parametrize("change", ["instance sizes", "instance k"])
+def test_team_batch_descriptors_follow_the_input(lp, change):
+    from lpgpu import gen
+    a = [gen.random_small(3, n=900, m=1000, k=4, max_size=9), gen.random_small(4, n=300, m=350, k=8, max_size=9)]
+    b = a[::-1] if change == "instance sizes" else a
+    ks = [[x.k for x in a], [x.k for x in b] if change == "instance sizes" else [8, 4]]
+    rng = np.random.default_rng(5)
+    with lp.Session(0) as s:
+        for insts, k in zip([a, b], ks):
+            parts = [rng.integers(0, q, x.hg.n).astype(np.int32) for x, q in zip(insts, k)]
+            got = []
+            for flags in (0, lp.FLAG_MULTI_LAUNCH):
+                s.upload_batch([x.hg for x in insts])
+                s.set_partition_batch(k, parts, eps=0.03)
+                r = s.refine(lp.default_config(flags=flags))
+                got.append((s.partition(), s.pin_counts(), s.instance_km1(), r.delta, r.moves))
+            _same(*got)
+
+
+def test_team_descriptors_follow_the_pin_count_width(lp):
+    from lpgpu import gen
+    n, rng = 70001, np.random.default_rng(6)
+    part = rng.integers(0, 2, n).astype(np.int32)
+    small = np.full(500, 4)
+    with lp.Session(0) as s:
+        for big in ([35000, 35000], [69995, 5]):  # 16-bit, then 32-bit pin counts; the same n, m and pins
+            sizes = np.concatenate([big, small])
+            pins = np.concatenate([rng.choice(n, z, replace=False) for z in sizes]).astype(np.int32)
+            off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+            hg = gen.Hypergraph(n, len(sizes), off, pins, np.ones(n, np.int32), rng.integers(1, 9, len(sizes)).astype(np.int32))
+            s.upload(hg)
+            s.set_partition(2, part, eps=0.03)
+            r = s.refine(lp.default_config())
+            want = _refine(lp, hg, 2, part, flags=lp.FLAG_MULTI_LAUNCH)
+            _same((s.partition(), s.block_weights(), s.pin_counts(), r.delta, r.moves),
+                  (want[0], want[1], want[2], want[6][2], want[6][3]))
