@@ -28,7 +28,7 @@ refinement per step.
 
 Systems workloads (default run, one GPU; `--no-systems` skips them; also
 alone with `--workload batch|served`): `batch`, 4,096 small hypergraphs refined
-together (persistent rounds when the tuning table picks them) against the
+together (team rounds when the tuning table picks them) against the
 plain one-instance-per-call loop; `served`, 256 Poisson-arriving requests
 through the round-granular server against the plain sequential loop (p50,
 p99, throughput). Both check that every result is identical.
@@ -444,10 +444,10 @@ def pinned_instances(lpgpu, gen, insts):
 
 def batch_measure(args, insts, plain_modes=(0, None)):
     """Many small hypergraphs refined by one batched session (the tuned form,
-    persistent rounds when the tuning table picks them) vs the plain loop (one
+    team rounds when the tuning table picks them) vs the plain loop (one
     instance per call sequence), both end to end from page-locked host buffers
     (upload, set partition, 5 rounds, download); device-resident refines of
-    both the persistent and the multi-launch form from the same start. Every
+    both the team ("persistent") and the multi-launch form from the same start. Every
     instance's km1 must be identical in all of them."""
     import lpgpu
     from lpgpu import I32P, _check, gen, lib

@@ -74,12 +74,12 @@ typedef struct {
 /* lpgpu_config.flags: launch the refine directly instead of capturing it once
  * as a CUDA graph and replaying it (useful when every call has new sizes). */
 #define LPGPU_FLAG_NO_GRAPH 1
-/* lpgpu_config.flags: run the refine as one persistent launch per round (every
- * CTA refines whole instances taken from a device work queue), or force the
+/* lpgpu_config.flags: run the refine as one persistent launch (teams of CTAs
+ * refine whole instances taken from a device work queue), or force the
  * multi-launch sub-round pipeline. Without either flag the session's tuning
  * decides (lpgpu_session_set_tuning, else the process-wide tuning table), and
- * a single instance with k <= 128 that no tuning covers runs all its rounds in
- * one launch (a CTA, a thread-block cluster or the whole grid, by its size).
+ * what no tuning covers runs all its rounds in one launch (a CTA, a thread-block
+ * cluster or the whole grid per instance, by its size).
  * The persistent form needs every instance's k <= LPGPU_PERSISTENT_MAX_K and
  * no explicit refinement node list; otherwise the refine returns
  * LPGPU_ERR_INVALID_ARG when it is forced and takes the multi-launch form
@@ -91,13 +91,13 @@ typedef struct {
 /* How a refine runs (the knobs the autotuner searches). */
 typedef enum {
   LPGPU_MODE_MULTI_LAUNCH = 0, /* the sub-round pipeline over the whole (union) hypergraph */
-  LPGPU_MODE_PERSISTENT = 1    /* one launch per round, instances as work items */
+  LPGPU_MODE_PERSISTENT = 1    /* one launch, instances as work items */
 } lpgpu_mode;
 
 typedef struct {
   int32_t mode;        /* lpgpu_mode */
   int32_t ctas_per_sm; /* persistent: resident CTAs per SM (1: up to 128 registers, 2: up to 64) */
-  int32_t unroll;      /* persistent: incidences per lane step of the sweep (4 or 8) */
+  int32_t unroll;      /* persistent: incidences per lane step of the sweep (4, or 8 with 2 CTAs per SM and k <= 64) */
   int32_t order;       /* persistent: 0 largest instance first, 1 instance order */
 } lpgpu_tuning;
 
@@ -277,9 +277,10 @@ LPGPU_API lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config
 
 /* Process-wide tuning table (the autotuner's output, rows in priority order;
  * the first row that applies wins; count 0 clears it). Without a matching
- * row, and without a session tuning, refines use the grid-wide form (one
- * launch for a single instance with k <= 128, else the multi-launch pipeline;
- * reported as LPGPU_MODE_MULTI_LAUNCH). This has no counterpart in the reference, which has no device code to tune. */
+ * row, and without a session tuning, refines take the library's default (one
+ * launch for all rounds, teams of CTAs by instance size; reported as
+ * LPGPU_MODE_MULTI_LAUNCH). This has no counterpart in the reference, which has
+ * no device code to tune. */
 LPGPU_API lpgpu_status lpgpu_set_tuning_table(const lpgpu_tuning_entry* entries, int32_t count);
 
 /* Tuning of one session (NULL: back to the table). lpgpu_session_tuning gives

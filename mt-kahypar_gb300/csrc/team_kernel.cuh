@@ -12,12 +12,11 @@
 // What bounds it: a sub-round of a small instance is a chain of dependent L2
 // accesses (0.5 us each) and barriers (a grid barrier about 2 us, a cluster
 // barrier 1.2 us). The multi-launch form pays six launches for it, 30 us per
-// sub-round on 1,024 vertices; a team pays four to six barriers: 1,024
-// vertices 1,112 -> 598 us per refine, 131,071 (k = 64) 3,517 -> 2,130 us,
-// 1M (k = 32) 5,857 -> 4,984 us. As persistent rounds (T = 1, two CTAs per SM)
-// the CTA selection in one pass and the CTA-wide heavy vertices take a
-// 1,280-instance batch from 55.7 to 39.0 ms end to end and 24 stepped sessions
-// from 38.1 to 20.2 ms.
+// sub-round on 1,024 vertices; a team pays four to six barriers. Per refine,
+// before (multi-launch) and now: 1,024 vertices 1,122 -> 434 us, 131,071
+// (k = 64) 3,530 -> 2,009 us, 1M (k = 32) 5,744 -> 4,611 us. A 1,280-instance
+// batch (clusters, CTA selection in one pass, CTA-wide heavy vertices) takes
+// 42.1 -> 29.0 ms end to end and 24 stepped sessions 38.0 -> 6.6 ms.
 //
 // A vertex is swept, selected, moved and undone by one CTA per sub-round, whose
 // candidate and kept-move lists live in its own part of the instance's scratch

@@ -478,7 +478,7 @@ class Session:
 
 
 class Stepper:
-    """Runs one LP round of many sessions per persistent launch (lpgpu_stepper_*)."""
+    """Runs one LP round of many sessions per launch of team rounds (lpgpu_stepper_*)."""
 
     def __init__(self, device: int = 0):
         self._h = ctypes.c_void_p()

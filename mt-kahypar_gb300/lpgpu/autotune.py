@@ -3,7 +3,7 @@ writes the tuning table the library loads at start-up.
 
 Search space (lpgpu_tuning):
   * mode: the multi-launch sub-round pipeline over the union hypergraph, or
-    persistent rounds (one launch per round, instances as work items);
+    team rounds (one launch, instances as work items);
   * persistent: resident CTAs per SM (1: up to 128 registers, 2: up to 64),
     sweep unroll (4 or 8 incidences per lane step), work order (largest
     instance first, or instance order).

@@ -6,8 +6,8 @@ completion.
 
 * Small requests (at most `large_pins` pins and k <= 64) each get a session
   from a pool and join the stepper's running set at the next round boundary.
-  Every step runs one LP round of every running request in one persistent
-  launch (lpgpu_stepper_launch). While a step runs, the requests admitted for
+  Every step runs one LP round of every running request in one launch of
+  team rounds (lpgpu_stepper_launch). While a step runs, the requests admitted for
   the next one are uploaded on their own streams; after it, finished requests
   leave and their partitions are read back. A request never waits for the
   remaining rounds of another: it joins after at most one round and leaves as
