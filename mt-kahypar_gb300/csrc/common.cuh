@@ -240,8 +240,14 @@ cudaError_t launch_build_incidence(const Launch& L, int64_t n, int64_t m, int64_
 cudaError_t launch_init_partition(const Launch& L, const RoundCtx& c);
 // Adds km1 and cut to out[0] and out[1] (zeroed by the caller).
 cudaError_t launch_metrics(const Launch& L, const RoundCtx& c, int64_t* out);
-// dst = a[0 .. na) followed by b[0 .. nb): what the host reads after a call, in one copy.
-cudaError_t launch_report(const Launch& L, int64_t* dst, const int64_t* a, int64_t na, const int64_t* b, int64_t nb);
+// What team rounds need before their first round: metrics before (added to before[0] and before[1], zeroed by
+// the caller), cleared statistics, stamps, team scratch and work counter, and (mark) every vertex's flag.
+cudaError_t launch_refine_begin(const Launch& L, const RoundCtx& c, int64_t* before, int64_t* stats, int64_t nstats,
+                                int64_t* scratch, int64_t nscratch, int64_t* queue, bool mark);
+// dst = a[0 .. na) followed by b[0 .. nb): what the host reads after a call, in one copy; the metrics are added
+// to `after` unless it is null; clear: every vertex's flag is dropped.
+cudaError_t launch_refine_end(const Launch& L, const RoundCtx& c, int64_t* after, int64_t* dst, const int64_t* a,
+                              int64_t na, const int64_t* b, int64_t nb, bool clear);
 cudaError_t launch_instance_metrics(const Launch& L, const RoundCtx& c, int64_t* km1_inst);
 cudaError_t launch_best_moves(const Launch& L, const RoundCtx& c, int32_t* to, int32_t* gain,
                               uint8_t* border);
@@ -379,13 +385,14 @@ constexpr int kTeamMaxCluster = 16;
 // from the work queue counter `queue` (zeroed here) by up to `teams` teams of
 // P.T CTAs each. W: Λ words class of all instances; unit: every net
 // weight is 1; ctas_per_sm: the 1- or 2-CTA-per-SM build of the kernel.
-// `scratch`: teams * team_scratch_words(P.kcap) words (P.T > 1, zeroed here).
+// `scratch`: teams * team_scratch_words(P.kcap) words (P.T > 1);
+// it and the work counter `queue` are zeroed here unless they are `cleared`.
 // A grid barrier that gives up sets *err. More than kTeamMaxCluster CTAs per
 // team need count == 1. `own_bytes`: shared memory a CTA's part of the largest
 // instance wants (team_own_bytes).
 cudaError_t launch_px_round(const Launch& L, const PxInst* insts, const int32_t* order, int32_t count,
                             PxParams P, int W, bool unit, int ctas_per_sm, int teams, int64_t* scratch,
-                            int64_t* queue, int64_t* err, int64_t own_bytes);
+                            int64_t* queue, int64_t* err, int64_t own_bytes, bool cleared);
 // Bytes a CTA of a team of T keeps of an instance, on average: its vertices'
 // offsets, weights, blocks and list entries and their incident nets; alone also
 // the records and pin counts.

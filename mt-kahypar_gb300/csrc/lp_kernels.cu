@@ -434,11 +434,15 @@ cudaError_t launch_init_partition(const Launch& L, const RoundCtx& c) {
   return cudaSuccess;
 }
 
-// metrics::km1 / hyperedgeCut (metrics.cpp:29-65): thread per net.
-__global__ void k_metrics(RoundCtx c, int64_t* out) {
+// metrics::km1 / hyperedgeCut (metrics.cpp:29-65): thread per net; added to
+// out[0] and out[1]. With EPOCH the nets' activation stamps are cleared too.
+// The whole block calls it.
+template <bool EPOCH>
+__device__ __forceinline__ void add_metrics(const RoundCtx& c, int64_t* out) {
   int64_t km1 = 0, cut = 0;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < c.m;
        e += (int64_t)gridDim.x * blockDim.x) {
+    if (EPOCH) c.net_epoch[e] = 0;
     int lam = 0;
     for (int w = 0; w < c.W; ++w) lam += __popc(c.conn[e * 2 * c.W + w]);
     const int64_t we = c.w_e[e];
@@ -451,6 +455,61 @@ __global__ void k_metrics(RoundCtx c, int64_t* out) {
     atomicAdd(reinterpret_cast<ull*>(&out[0]), (ull)km1);
     atomicAdd(reinterpret_cast<ull*>(&out[1]), (ull)cut);
   }
+}
+
+__global__ void k_metrics(RoundCtx c, int64_t* out) { add_metrics<false>(c, out); }
+
+// Every vertex's activation flag set to 0 or 1: 16 flags per store.
+__device__ __forceinline__ void fill_flags(uint8_t* flag, int64_t n, uint32_t value) {
+  const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  const uint32_t x = value * 0x01010101u;
+  const int64_t quads = n >> 4;  // the buffer starts on an allocation's boundary
+  for (int64_t i = i0; i < quads; i += step) reinterpret_cast<uint4*>(flag)[i] = make_uint4(x, x, x, x);
+  for (int64_t i = (quads << 4) + i0; i < n; i += step) flag[i] = (uint8_t)value;
+}
+
+// What a refinement by team rounds needs before its first round, in one
+// launch: metrics before, cleared stamps, statistics and team scratch, and
+// (mark) every vertex's flag set. Bound by its launch below a million nets.
+// One launch instead of six operations before the rounds and one instead of
+// three after them (k_refine_end): a refine of 16,384 vertices 803 -> 769 us,
+// 24 stepped sessions 6.56 -> 6.16 ms.
+__global__ void k_refine_begin(RoundCtx c, int64_t* before, int64_t* stats, int64_t nstats, int64_t* scratch,
+                               int64_t nscratch, int64_t* queue, int mark) {
+  const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = i0; i < nstats; i += step) stats[i] = 0;
+  for (int64_t i = i0; i < nscratch; i += step) scratch[i] = 0;
+  if (queue && i0 == 0) *queue = 0;
+  if (mark) fill_flags(c.next_flag, c.n, 1);
+  add_metrics<true>(c, before);
+}
+
+cudaError_t launch_refine_begin(const Launch& L, const RoundCtx& c, int64_t* before, int64_t* stats, int64_t nstats,
+                                int64_t* scratch, int64_t nscratch, int64_t* queue, bool mark) {
+  const int64_t work = std::max(std::max(c.m, c.n / 16), std::max<int64_t>(nscratch, 1));
+  k_refine_begin<<<grid_for(L, work, 256), 256, 0, L.st>>>(c, before, stats, nstats, scratch, nscratch, queue,
+                                                           mark ? 1 : 0);
+  LAUNCHED("k_refine_begin");
+  return cudaGetLastError();
+}
+
+// What the host reads after a call, in one launch: a (statistics) and b (block
+// weights) to dst, the metrics added to `after` unless it is null; with
+// `clear` the flags the last round left are dropped.
+__global__ void k_refine_end(RoundCtx c, int64_t* after, int64_t* dst, const int64_t* a, int64_t na, const int64_t* b,
+                             int64_t nb, int clear) {
+  const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = i0; i < na + nb; i += step) dst[i] = i < na ? a[i] : b[i - na];
+  if (clear) fill_flags(c.next_flag, c.n, 0);
+  if (after) add_metrics<false>(c, after);
+}
+
+cudaError_t launch_refine_end(const Launch& L, const RoundCtx& c, int64_t* after, int64_t* dst, const int64_t* a,
+                              int64_t na, const int64_t* b, int64_t nb, bool clear) {
+  const int64_t work = std::max(std::max(after ? c.m : 0, clear ? c.n / 16 : 0), std::max<int64_t>(na + nb, 1));
+  k_refine_end<<<grid_for(L, work, 256), 256, 0, L.st>>>(c, after, dst, a, na, b, nb, clear ? 1 : 0);
+  LAUNCHED("k_refine_end");
+  return cudaGetLastError();
 }
 
 // km1 of every instance of a batched session (net instance = instance of its first pin).
@@ -481,17 +540,6 @@ cudaError_t launch_metrics(const Launch& L, const RoundCtx& c, int64_t* out) {
     k_metrics<<<grid_for(L, c.m, 256), 256, 0, L.st>>>(c, out);
     LAUNCHED("k_metrics");
   }
-  return cudaGetLastError();
-}
-
-__global__ void k_report(int64_t* dst, const int64_t* a, int64_t na, const int64_t* b, int64_t nb) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < na + nb; i += (int64_t)gridDim.x * blockDim.x)
-    dst[i] = i < na ? a[i] : b[i - na];
-}
-
-cudaError_t launch_report(const Launch& L, int64_t* dst, const int64_t* a, int64_t na, const int64_t* b, int64_t nb) {
-  k_report<<<grid_for(L, na + nb, 256), 256, 0, L.st>>>(dst, a, na, b, nb);
-  LAUNCHED("k_report");
   return cudaGetLastError();
 }
 

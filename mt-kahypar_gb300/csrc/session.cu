@@ -889,9 +889,12 @@ lpgpu_status lpgpu_session_project_partition(lpgpu_session* fine, const lpgpu_se
 }
 
 // Reads the report back: its head, `nstats` words of statistics and the block
-// weights, in one copy (the caller has reserved it and written its head).
-static lpgpu_status fetch_report(lpgpu_session* s, const int64_t* stats, int64_t nstats, std::vector<int64_t>* h) {
-  CK(launch_report(s->launch(), s->rep.p + kRepHead, stats, nstats, s->bw.p, s->k));
+// weights, in one copy (the caller has reserved it and cleared its head).
+// `metrics` adds km1 and cut at kRepAfter, `clear` drops the active flags.
+static lpgpu_status fetch_report(lpgpu_session* s, const int64_t* stats, int64_t nstats, std::vector<int64_t>* h,
+                                 bool metrics, bool clear = false) {
+  CK(launch_refine_end(s->launch(), s->ctx(), metrics ? s->rep.p + kRepAfter : nullptr, s->rep.p + kRepHead, stats,
+                       nstats, s->bw.p, s->k, clear));
   h->resize(kRepHead + nstats + s->k);
   CK(cudaMemcpyAsync(h->data(), s->rep.p, sizeof(int64_t) * h->size(), cudaMemcpyDeviceToHost, s->st));
   CK(cudaStreamSynchronize(s->st));
@@ -908,9 +911,8 @@ static double imbalance_of(const lpgpu_session* s, const int64_t* w) {
 static lpgpu_status read_metrics(lpgpu_session* s, int64_t* km1, int64_t* cut, double* imbalance) {
   CK(s->reserve_report(kRepHead + s->k));
   CK(cudaMemsetAsync(s->rep.p, 0, sizeof(int64_t) * kRepHead, s->st));
-  CK(launch_metrics(s->launch(), s->ctx(), s->rep.p + kRepAfter));
   std::vector<int64_t> h;
-  const lpgpu_status st = fetch_report(s, nullptr, 0, &h);
+  const lpgpu_status st = fetch_report(s, nullptr, 0, &h, true);
   if (st != LPGPU_OK) return st;
   if (km1) *km1 = h[kRepAfter];
   if (cut) *cut = h[kRepAfter + 1];
@@ -1206,7 +1208,6 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
   const int64_t nstats = (int64_t)std::max(1, R) * kStats;
   CK(s->reserve_report(kRepHead + nstats + s->k));
   CK(cudaMemsetAsync(s->rep.p, 0, sizeof(int64_t) * kRepHead, st));
-  CK(launch_metrics(L, c, s->rep.p + kRepBefore));
   TmpBuf<int32_t> dnodes(s->mem);
   if (num_nodes > 0) {
     CK(dnodes.alloc(num_nodes));
@@ -1216,11 +1217,17 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
   // The whole refine is a fixed sequence of launches whose element counts live
   // in device memory: the multi-launch form is captured once as a CUDA graph and
   // replayed.
+  const bool mark_all = num_nodes == 0 && cfg.rebalancing != 0;
   auto enqueue = [&]() -> cudaError_t {
     cudaError_t e;
-    if ((e = cudaMemsetAsync(s->stats.p, 0, sizeof(int64_t) * std::max(1, R) * kStats, st)) != cudaSuccess) return e;
-    if (s->m > 0 && (e = cudaMemsetAsync(s->net_epoch.p, 0, sizeof(int32_t) * s->m, st)) != cudaSuccess) return e;
-    if (!use_team) {  // accumulators of the multi-launch kernels
+    if (use_team) {
+      if ((e = launch_refine_begin(L, c, s->rep.p + kRepBefore, s->stats.p, nstats, s->team.p,
+                                   shape.T > 1 ? team_scratch_words(kmax) * team_slots(L, px_count, shape.T) : 0,
+                                   s->scal.p + kPxQueue, mark_all)) != cudaSuccess)
+        return e;
+    } else {  // statistics and accumulators of the multi-launch kernels
+      if ((e = cudaMemsetAsync(s->stats.p, 0, sizeof(int64_t) * nstats, st)) != cudaSuccess) return e;
+      if (s->m > 0 && (e = cudaMemsetAsync(s->net_epoch.p, 0, sizeof(int32_t) * s->m, st)) != cudaSuccess) return e;
       if ((e = cudaMemsetAsync(s->blk64.p, 0, sizeof(int64_t) * (7 * s->k + 1), st)) != cudaSuccess) return e;
       if ((e = cudaMemsetAsync(s->scal.p, 0, sizeof(int64_t) * kScalars, st)) != cudaSuccess) return e;
       if ((e = cudaMemsetAsync(s->bin_cnt.p, 0, sizeof(int64_t) * kMaxSubrounds * kDegClasses, st)) != cudaSuccess)
@@ -1230,16 +1237,16 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
     }
     if (num_nodes > 0) {
       if ((e = launch_mark_list(L, c, dnodes.p(), num_nodes)) != cudaSuccess) return e;
-    } else if ((e = launch_mark_all(L, c, cfg.rebalancing)) != cudaSuccess) {  // sets every vertex's flag
+    } else if (!(use_team && mark_all) &&
+               (e = launch_mark_all(L, c, cfg.rebalancing)) != cudaSuccess) {  // sets every vertex's flag
       return e;
     }
     if (use_team) {  // all rounds in one launch
       if ((e = launch_px_round(L, s->px.p, s->px_order.p, px_count, pxp, s->W, s->unit_nets, shape.per_sm,
                                team_slots(L, px_count, shape.T), s->team.p, s->scal.p + kPxQueue,
-                               s->rep.p + kRepErr, own_bytes)) != cudaSuccess)
+                               s->rep.p + kRepErr, own_bytes, true)) != cudaSuccess)
         return e;
-      if (s->n > 0 && (e = cudaMemsetAsync(s->next_flag.p, 0, s->n, st)) != cudaSuccess) return e;
-      return cudaSuccess;
+      return cudaSuccess;  // the flags are dropped with the report
     }
     for (int r = 0; r < R; ++r) {
       if ((e = launch_bin_active(L, c, r, S, s->bin_cnt.p, tm)) != cudaSuccess) return e;
@@ -1251,6 +1258,7 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
     if (s->n > 0 && (e = cudaMemsetAsync(s->next_flag.p, 0, s->n, st)) != cudaSuccess) return e;
     return cudaSuccess;
   };
+  if (!use_team) CK(launch_metrics(L, c, s->rep.p + kRepBefore));
   if (num_nodes > 0 || tm || use_team || (cfg.flags & LPGPU_FLAG_NO_GRAPH)) {
     // direct launches: explicit node lists, per-phase event timing, and the few of the team form
     if (tm) tm->reset();
@@ -1294,9 +1302,8 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
     CK(cudaGraphLaunch(s->graph, st));
     add_kernel_launches(s->graph_kernels);
   }
-  if (result) CK(launch_metrics(L, c, s->rep.p + kRepAfter));
   std::vector<int64_t> h;
-  ps = fetch_report(s, s->stats.p, nstats, &h);
+  ps = fetch_report(s, s->stats.p, nstats, &h, result != nullptr, use_team);
   if (ps != LPGPU_OK) return ps;
   if (h[kRepErr]) {
     s->has_part = false;  // the moves of an unfinished sub-round
@@ -1344,10 +1351,9 @@ lpgpu_status lpgpu_session_begin_rounds(lpgpu_session* s, const lpgpu_config* cf
   if (!s->step_ev) CK(cudaEventCreateWithFlags(&s->step_ev, cudaEventDisableTiming));
   RoundCtx c = s->ctx(&cfg);
   CK(cudaMemsetAsync(s->scal.p + kStepKm1, 0, sizeof(int64_t) * 2, st));
-  CK(launch_metrics(s->launch(), c, s->scal.p + kStepKm1));
-  CK(cudaMemsetAsync(s->stats.p, 0, sizeof(int64_t) * std::max(1, R) * kStats, st));
-  if (s->m > 0) CK(cudaMemsetAsync(s->net_epoch.p, 0, sizeof(int32_t) * s->m, st));
-  CK(launch_mark_all(s->launch(), c, cfg.rebalancing));
+  CK(launch_refine_begin(s->launch(), c, s->scal.p + kStepKm1, s->stats.p, (int64_t)std::max(1, R) * kStats, nullptr, 0,
+                         nullptr, cfg.rebalancing != 0));
+  if (!cfg.rebalancing) CK(launch_mark_all(s->launch(), c, 0));
   s->step_cfg = cfg;
   s->step_round = 0;
   s->step_done = R == 0;
@@ -1367,10 +1373,8 @@ lpgpu_status lpgpu_session_end_rounds(lpgpu_session* s, lpgpu_result* result) {
   CK(s->reserve_report(kRepHead + nstats + s->k));
   CK(cudaMemsetAsync(s->rep.p, 0, sizeof(int64_t) * kRepHead, s->st));
   CK(cudaMemcpyAsync(s->rep.p + kRepBefore, s->scal.p + kStepKm1, sizeof(int64_t) * 2, cudaMemcpyDeviceToDevice, s->st));
-  if (result) CK(launch_metrics(s->launch(), s->ctx(), s->rep.p + kRepAfter));
-  if (s->n > 0) CK(cudaMemsetAsync(s->next_flag.p, 0, s->n, s->st));
   std::vector<int64_t> h;
-  const lpgpu_status ps = fetch_report(s, s->stats.p, nstats, &h);
+  const lpgpu_status ps = fetch_report(s, s->stats.p, nstats, &h, result != nullptr, true);
   if (ps != LPGPU_OK) return ps;
   s->stepping = false;
   book_rounds(s, h, R, result);
@@ -1574,7 +1578,8 @@ lpgpu_status lpgpu_stepper_launch(lpgpu_stepper* t, lpgpu_session* const* sessio
     }
     CK(launch_px_round(Lg, t->table.p + gr.second.first, nullptr, gr.second.second, P, k.W, k.unit != 0,
                        tuned ? tu.ctas_per_sm : 2, team_slots(L, gr.second.second, T),
-                       T > 1 ? t->team.p + used : nullptr, t->queue.p + 2 * gi, t->queue.p + 2 * gi + 1, own_bytes));
+                       T > 1 ? t->team.p + used : nullptr, t->queue.p + 2 * gi, t->queue.p + 2 * gi + 1, own_bytes,
+                       false));
     if (T > 1) used += words * team_slots(L, gr.second.second, T);
   }
   for (size_t i = 0; i + 1 < G && i < 3; ++i) {  // the round ends with its last group
@@ -2000,10 +2005,9 @@ lpgpu_status lpgpu_session_rebalance(lpgpu_session* s, int32_t max_rounds, lpgpu
   // km1 and the block weights before, in one round trip; every round brings its
   // statistics, the new weights and the new km1 in another
   CK(cudaMemsetAsync(s->rep.p, 0, sizeof(int64_t) * kRepHead, st));
-  CK(launch_metrics(s->launch(), c, s->rep.p + kRepAfter));
   CK(cudaMemcpyAsync(s->sub_off.p, sub, sizeof(sub), cudaMemcpyHostToDevice, st));
   std::vector<int64_t> h;
-  ps = fetch_report(s, nullptr, 0, &h);
+  ps = fetch_report(s, nullptr, 0, &h, true);
   if (ps != LPGPU_OK) return ps;
   const int64_t km1_before = h[kRepAfter];
   const std::vector<int64_t>& hl = s->h_lmax;
@@ -2074,8 +2078,7 @@ lpgpu_status lpgpu_session_rebalance(lpgpu_session* s, int32_t max_rounds, lpgpu
     CK(cudaMemsetAsync(s->blk64.p, 0, sizeof(int64_t) * 3 * k, st));  // in_w, in_cnt, cand_out
     CK(cudaMemsetAsync(s->rep.p, 0, sizeof(int64_t) * kRepHead, st));
     CK(launch_rebalance_round(s->launch(), c, r, s->heavy.p, s->revl.p, rb.p()));
-    CK(launch_metrics(s->launch(), c, s->rep.p + kRepAfter));
-    ps = fetch_report(s, s->stats.p + (int64_t)r * kStats, kStats, &h);
+    ps = fetch_report(s, s->stats.p + (int64_t)r * kStats, kStats, &h, true);
     if (ps != LPGPU_OK) return ps;
     km1_after = h[kRepAfter];
     const int64_t* hs = h.data() + kRepHead;

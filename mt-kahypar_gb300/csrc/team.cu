@@ -115,16 +115,16 @@ cudaError_t launch_px_active(const Launch& L, const PxInst* insts, int32_t count
 
 cudaError_t launch_px_round(const Launch& L, const PxInst* insts, const int32_t* order, int32_t count, PxParams P,
                             int W, bool unit, int ctas_per_sm, int teams, int64_t* scratch, int64_t* queue,
-                            int64_t* err, int64_t own_bytes) {
+                            int64_t* err, int64_t own_bytes, bool cleared) {
   if (count <= 0 || P.rounds <= 0) return cudaSuccess;
   if (W < 1 || W > 32 || (W & (W - 1)) || P.T < 1 || P.kcap > kTeamMaxK) return cudaErrorInvalidValue;
   const bool grid = P.T > kTeamMaxCluster;
   if (grid && (count != 1 || teams != 1)) return cudaErrorInvalidValue;
-  cudaError_t e = cudaMemsetAsync(queue, 0, sizeof(int64_t), L.st);
+  cudaError_t e = cleared ? cudaSuccess : cudaMemsetAsync(queue, 0, sizeof(int64_t), L.st);
   if (e != cudaSuccess) return e;
   if (P.T > 1) {
     if (!scratch) return cudaErrorInvalidValue;
-    e = cudaMemsetAsync(scratch, 0, sizeof(int64_t) * teams * team_scratch_words(P.kcap), L.st);
+    if (!cleared) e = cudaMemsetAsync(scratch, 0, sizeof(int64_t) * teams * team_scratch_words(P.kcap), L.st);
     if (e != cudaSuccess) return e;
   } else {
     scratch = nullptr;

@@ -13,10 +13,10 @@
 // accesses (0.5 us each) and barriers (a grid barrier about 2 us, a cluster
 // barrier 1.2 us). The multi-launch form pays six launches for it, 30 us per
 // sub-round on 1,024 vertices; a team pays four to six barriers. Per refine,
-// before (multi-launch) and now: 1,024 vertices 1,122 -> 434 us, 131,071
-// (k = 64) 3,530 -> 2,009 us, 1M (k = 32) 5,744 -> 4,611 us. A 1,280-instance
+// before (multi-launch) and now: 1,024 vertices 1,130 -> 435 us, 131,071
+// (k = 64) 3,552 -> 2,009 us, 1M (k = 32) 5,830 -> 4,601 us. A 1,280-instance
 // batch (clusters, CTA selection in one pass, CTA-wide heavy vertices) takes
-// 42.1 -> 29.0 ms end to end and 24 stepped sessions 38.0 -> 6.6 ms.
+// 42.1 -> 28.7 ms end to end and 24 stepped sessions 38.2 -> 6.2 ms.
 //
 // A vertex is swept, selected, moved and undone by one CTA per sub-round, whose
 // candidate and kept-move lists live in its own part of the instance's scratch

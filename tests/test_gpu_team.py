@@ -150,3 +150,26 @@ def test_team_descriptors_follow_the_pin_count_width(lp):
             want = _refine(lp, hg, 2, part, flags=lp.FLAG_MULTI_LAUNCH)
             _same((s.partition(), s.block_weights(), s.pin_counts(), r.delta, r.moves),
                   (want[0], want[1], want[2], want[6][2], want[6][3]))
+
+
+# flags are set and dropped 16 at a time: ends of the vector part, and what one refine leaves for the next
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 47, 4099, 16385])
+@pytest.mark.parametrize("rebalancing", [0, 1])
+def test_team_flags_between_refines(lp, n, rebalancing):
+    from lpgpu import gen
+    rng = np.random.default_rng(n)
+    off = np.arange(0, 3 * n + 1, 3, dtype=np.int64)
+    hg = gen.Hypergraph(n, n, off, rng.integers(0, n, 3 * n).astype(np.int32), np.ones(n, np.int32), np.ones(n, np.int32))
+    part, nodes = rng.integers(0, 4, n).astype(np.int32), rng.integers(0, n, max(1, n // 3)).astype(np.int32)
+    got = []
+    for first in (0, lp.FLAG_MULTI_LAUNCH):
+        with lp.Session(0) as s:
+            s.upload(hg)
+            s.set_partition(4, part, eps=0.1)
+            out = []
+            for flags, which in [(first, None), (first, nodes), (lp.FLAG_MULTI_LAUNCH, None), (first, None)]:
+                r = s.refine(lp.default_config(flags=flags, rounds=2, rebalancing=rebalancing), nodes=which)
+                out += [s.partition(), [[x[q] for q in KEYS] for x in s.round_stats()], s.metrics(),
+                        (r.km1_before, r.km1_after, r.delta, r.moves, r.rounds)]
+            got.append(out)
+    _same(*got)
