@@ -83,7 +83,7 @@ enum Scalar : int {
   kHeavyCount = 11, // heavy vertices a per-vertex query deferred to k_sweep_heavy
   kRevCount = 12,  // moves marked for revert in the current sub-round
   kPxQueue = 13,   // work queue counter of a persistent round
-  kStepKm1 = 14,   // km1 and cut at the start of a stepped refinement
+  kStepKm1 = 14,   // km1 and cut at the start of a stepped refinement (kept until it ends: the last two words)
   kScalars = 16
 };
 

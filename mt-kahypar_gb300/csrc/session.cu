@@ -1229,7 +1229,8 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
       if ((e = cudaMemsetAsync(s->stats.p, 0, sizeof(int64_t) * nstats, st)) != cudaSuccess) return e;
       if (s->m > 0 && (e = cudaMemsetAsync(s->net_epoch.p, 0, sizeof(int32_t) * s->m, st)) != cudaSuccess) return e;
       if ((e = cudaMemsetAsync(s->blk64.p, 0, sizeof(int64_t) * (7 * s->k + 1), st)) != cudaSuccess) return e;
-      if ((e = cudaMemsetAsync(s->scal.p, 0, sizeof(int64_t) * kScalars, st)) != cudaSuccess) return e;
+      // a stepped refinement's metrics at its start stay
+      if ((e = cudaMemsetAsync(s->scal.p, 0, sizeof(int64_t) * kStepKm1, st)) != cudaSuccess) return e;
       if ((e = cudaMemsetAsync(s->bin_cnt.p, 0, sizeof(int64_t) * kMaxSubrounds * kDegClasses, st)) != cudaSuccess)
         return e;
       if (s->batched && (e = cudaMemsetAsync(s->inst_delta.p, 0, sizeof(int64_t) * s->num_inst, st)) != cudaSuccess)

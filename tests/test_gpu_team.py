@@ -173,3 +173,18 @@ def test_team_flags_between_refines(lp, n, rebalancing):
                         (r.km1_before, r.km1_after, r.delta, r.moves, r.rounds)]
             got.append(out)
     _same(*got)
+
+
+# a stepped refinement reports the metrics of its start, whatever runs on the session before it ends
+@pytest.mark.parametrize("flags", ["multi-launch", "team"])
+def test_stepped_start_metrics_survive_a_refine(lp, flags):
+    from lpgpu import gen
+    inst = gen.random_small(11, n=700, m=800, k=6)
+    with lp.Session(0) as s:
+        s.upload(inst.hg)
+        s.set_partition(6, inst.part, eps=0.03)
+        km1 = s.metrics()[0]
+        assert km1 > 0
+        s.begin_rounds(lp.default_config(rounds=5))
+        s.refine(lp.default_config(rounds=5, flags=lp.FLAG_MULTI_LAUNCH if flags == "multi-launch" else 0))
+        assert s.end_rounds().km1_before == km1
