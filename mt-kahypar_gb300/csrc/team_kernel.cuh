@@ -165,6 +165,7 @@ __device__ __forceinline__ bool team_sync(Team& tm, TS& s) {
     return true;
   }
   if (tm.sync == kSyncCluster) {
+    __syncwarp();  // .aligned wants whole warps, and the callers' thread-0 and strided code diverges
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     return true;
   }
