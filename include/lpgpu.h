@@ -79,7 +79,9 @@ typedef struct {
  * multi-launch sub-round pipeline. Without either flag the session's tuning
  * decides (lpgpu_session_set_tuning, else the process-wide tuning table), and
  * what no tuning covers runs all its rounds in one launch (a CTA, a thread-block
- * cluster or the whole grid per instance, by its size).
+ * cluster or the whole grid per instance, by its vertices and pins), or the
+ * pipeline where that is faster (a few hundred vertices with thousands of pins
+ * each).
  * The persistent form needs every instance's k <= LPGPU_PERSISTENT_MAX_K and
  * no explicit refinement node list; otherwise the refine returns
  * LPGPU_ERR_INVALID_ARG when it is forced and takes the multi-launch form

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "lpgpu.h"
+#include "team_rules.h"
 
 namespace lpgpu {
 
@@ -376,10 +377,6 @@ struct PxParams {
 __host__ __device__ inline int64_t team_scratch_words(int kcap) {
   return 32 + 17 * (int64_t)kcap + 3 * kMaxSubrounds;
 }
-
-// CTAs per team of a launch over one instance of n vertices (1: a CTA; up to
-// kTeamMaxCluster: a thread-block cluster; more: the whole cooperative grid).
-constexpr int kTeamMaxCluster = 16;
 
 // Runs LP rounds of `count` instances, taken in `order` (null: 0..count-1)
 // from the work queue counter `queue` (zeroed here) by up to `teams` teams of

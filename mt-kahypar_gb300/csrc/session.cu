@@ -977,26 +977,12 @@ static lpgpu_tuning session_tuning(const lpgpu_session* s) {
 }
 
 // ---- one instance refined by one team (team.cu)
-//
-// CTAs of the team and of an SM by the number of vertices. Measured (GB300,
-// whole refine call in us, one CTA / cluster of 16 / one CTA per SM / two per
-// SM; multi-launch pipeline in brackets): 1,024 vertices (k = 2) 467 / 556 / - /
-// - [1,094]; 2,048 (k = 4) 608 / 617 / - / -; 4,096 (k = 2) 976 / 681 / - / -;
-// 10,007 (k = 8) 1,634 / 797 / 888 / -; 16,384 (k = 64, weighted) 5,508 / 1,852 /
-// 1,660 / - [2,917]; 65,536 (k = 32) - / 2,678 / 1,703 / 2,015; 262,144 (k = 16)
-// - / 5,877 / 2,184 / 2,242 [3,203]; 524,288 (k = 32) - / 11,319 / 2,924 / 2,887,
-// unweighted k = 8 1,777 / 1,903; 1M (k = 32) - / - / 5,195 / 4,641 [5,563]; 4.2M
-// (k = 128) - / - / 12,145 / 11,015 [11,371].
-struct TeamShape {
-  int per_sm;  // kernel build: resident CTAs per SM
-  int unroll;
-  int T;       // CTAs of the team (0: as many as are resident)
-};
-static TeamShape team_shape(int64_t n, int num_sms, int in_flight) {
-  if (n <= 2048) return {1, 4, 1};
-  if (n <= 12288) return {1, 4, kTeamMaxCluster};
-  if (in_flight > 1) return {2, 4, 2 * num_sms / std::min(in_flight, 4)};
-  return {n < 655360 ? 1 : 2, 4, 0};
+
+// The team of a single-instance refine when `in_flight` refines run on the device.
+static TeamShape shared_shape(int64_t n, int64_t pins, int num_sms, int in_flight) {
+  TeamShape t = team_shape(n, pins);
+  if (t.T == kTeamAll && in_flight > 1) t = {2, 4, 2 * num_sms / std::min(in_flight, 4)};
+  return t;
 }
 
 // Refine calls in progress per device: a cooperative grid over the whole GPU
@@ -1166,10 +1152,12 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
   const int32_t px_count = s->batched ? s->num_inst : 1;
   TeamShape shape{2, 8, 1};
   int64_t own_bytes = 0;
+  const bool must_team = tuned || (cfg.flags & LPGPU_FLAG_PERSISTENT);  // the form itself is not ours to choose
+  if (use_team && px_count == 1 && !must_team && team_shape(s->n, s->P).T == kTeamNone) use_team = false;
   if (use_team) {
     const Launch L = s->launch();
     if (px_count == 1) {
-      shape = team_shape(s->n, L.num_sms, in_flight.now);
+      shape = shared_shape(s->n, s->P, L.num_sms, in_flight.now);
     } else {
       int64_t max_n = 0;
       for (int32_t i = 0; i < px_count; ++i) max_n = std::max(max_n, s->h_inst_voff[i + 1] - s->h_inst_voff[i]);
@@ -1179,9 +1167,10 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
       shape.per_sm = tu.ctas_per_sm;
       shape.unroll = tu.unroll;
     }
-    if (shape.T == 0 || shape.T > kTeamMaxCluster) {
+    if (shape.T == kTeamNone) shape.T = kTeamAll;
+    if (shape.T == kTeamAll || shape.T > kTeamMaxCluster) {
       const int most = team_resident(L, s->W, s->unit_nets, shape.unroll, shape.per_sm);
-      shape.T = shape.T == 0 ? most : std::min(shape.T, most);
+      shape.T = shape.T == kTeamAll ? most : std::min(shape.T, most);
     }
     for (int32_t i = 0; i < px_count; ++i)
       own_bytes = std::max(own_bytes, team_own_bytes(s->h_inst_voff[i + 1] - s->h_inst_voff[i],

@@ -188,3 +188,55 @@ def test_stepped_start_metrics_survive_a_refine(lp, flags):
         s.begin_rounds(lp.default_config(rounds=5))
         s.refine(lp.default_config(rounds=5, flags=lp.FLAG_MULTI_LAUNCH if flags == "multi-launch" else 0))
         assert s.end_rounds().km1_before == km1
+
+
+def _dense(n, pins, size, seed, weighted=True):
+    """n vertices and exactly `pins` pins (a multiple of `size`): every net holds
+    `size` vertices at fixed distances from a random one."""
+    from lpgpu import gen
+    rng = np.random.default_rng([seed, n])
+    m = pins // size
+    assert m * size == pins and size <= n
+    steps = rng.choice(n, size, replace=False)
+    ids = ((rng.integers(0, n, m)[:, None] + steps[None, :]) % n).astype(np.int32).ravel()
+    return gen.Hypergraph(n, m, np.arange(0, pins + 1, size, dtype=np.int64), ids,
+                          rng.integers(1, 4, n).astype(np.int32) if weighted else np.ones(n, np.int32),
+                          rng.integers(1, 9, m).astype(np.int32) if weighted else np.ones(m, np.int32))
+
+
+# the pins at which a vertex count goes from one CTA to a cluster, to the grid and to the pipeline
+@pytest.mark.parametrize("n,pins,size", [
+    (2048, 16384, 4), (2048, 16388, 4), (700, 21776, 4), (700, 21780, 4), (2048, 131072, 8), (2048, 131080, 8),
+    (12288, 131072, 4), (12288, 131076, 4), (128, 128 * 4100, 4), (129, 129 * 4096, 4), (129, 129 * 4100, 4)])
+def test_team_sizes_by_pins(lp, n, pins, size):
+    hg = _dense(n, pins, size, 3)
+    part = (np.arange(n) * 7 % 9).astype(np.int32)
+    _same(_refine(lp, hg, 9, part, rounds=3), _refine(lp, hg, 9, part, rounds=3, flags=lp.FLAG_MULTI_LAUNCH))
+
+
+def _fastest(s, cfg, passes=4):
+    import time
+    best = float("inf")
+    for _ in range(passes):
+        s.restore_partition()
+        s.synchronize()
+        t0 = time.perf_counter()
+        s.refine(cfg)
+        best = min(best, time.perf_counter() - t0)
+    return best, s.partition()
+
+
+# Few vertices with many pins: the default form is never far behind the pipeline
+# (up to 1.05 times its time measured; one CTA took 3.2, 3.9 and 2.1 times).
+@pytest.mark.parametrize("n,degree,size,k", [(1024, 3000, 8, 32), (2048, 2000, 30, 32), (256, 20000, 8, 2)])
+def test_dense_instances_stay_near_the_pipeline(lp, n, degree, size, k):
+    hg = _dense(n, n * degree // size * size, size, 5, weighted=k > 2)
+    part = np.random.default_rng(n).permutation(np.arange(n) % k).astype(np.int32)
+    with lp.Session(0) as s:
+        s.upload(hg)
+        s.set_partition(k, part, eps=0.03)
+        s.save_partition()
+        pipeline, want = _fastest(s, lp.default_config(flags=lp.FLAG_MULTI_LAUNCH))
+        default, got = _fastest(s, lp.default_config())
+    assert np.array_equal(got, want)
+    assert default < 2 * pipeline
