@@ -81,7 +81,8 @@ typedef struct {
  * what no tuning covers runs all its rounds in one launch (a CTA, a thread-block
  * cluster or the whole grid per instance, by its vertices and pins), or the
  * pipeline where that is faster (a few hundred vertices with thousands of pins
- * each).
+ * each; a batch whose largest instance would outlast all the others, also where
+ * a row of the table says otherwise).
  * The persistent form needs every instance's k <= LPGPU_PERSISTENT_MAX_K and
  * no explicit refinement node list; otherwise the refine returns
  * LPGPU_ERR_INVALID_ARG when it is forced and takes the multi-launch form

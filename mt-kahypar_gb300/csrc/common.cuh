@@ -395,9 +395,6 @@ cudaError_t launch_px_round(const Launch& L, const PxInst* insts, const int32_t*
 // the records and pin counts.
 int64_t team_own_bytes(int64_t n, int64_t m, int64_t pins, int T, int k, int W, bool phi16,
                        int per_sm);
-// CTAs per team of a launch over `count` > 1 instances, the largest of max_n
-// vertices, with about `per_sm` CTAs' worth of teams per SM at most.
-int team_cluster(const Launch& L, int64_t count, int64_t max_n, int per_sm);
 // Teams of T CTAs that can be resident at once (an upper bound for clusters).
 int team_slots(const Launch& L, int64_t count, int T);
 // Largest number of CTAs of the kernel build that can be resident at once.

@@ -1152,16 +1152,25 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
   const int32_t px_count = s->batched ? s->num_inst : 1;
   TeamShape shape{2, 8, 1};
   int64_t own_bytes = 0;
-  const bool must_team = tuned || (cfg.flags & LPGPU_FLAG_PERSISTENT);  // the form itself is not ours to choose
-  if (use_team && px_count == 1 && !must_team && team_shape(s->n, s->P).T == kTeamNone) use_team = false;
+  // the largest instance (vertices, pins: perhaps of two)
+  int64_t max_n = 0, max_pins = 0;
+  for (int32_t i = 0; i < px_count; ++i) {
+    max_n = std::max(max_n, s->h_inst_voff[i + 1] - s->h_inst_voff[i]);
+    max_pins = std::max(max_pins, s->h_inst_pins[i]);
+  }
+  // a flag or the session's own tuning settles the form; a row of the table is chosen
+  // by the mean size and knows nothing of a batch's largest instance
+  const bool must_team = s->has_tuning || (cfg.flags & LPGPU_FLAG_PERSISTENT);
+  if (use_team && !must_team)
+    use_team = px_count == 1 ? tuned || team_shape(s->n, s->P).T != kTeamNone
+                             : !batch_wants_pipeline(max_pins, s->P,
+                                                     team_of_batch(px_count, max_n, max_pins, s->num_sms, kmax));
   if (use_team) {
     const Launch L = s->launch();
     if (px_count == 1) {
       shape = shared_shape(s->n, s->P, L.num_sms, in_flight.now);
     } else {
-      int64_t max_n = 0;
-      for (int32_t i = 0; i < px_count; ++i) max_n = std::max(max_n, s->h_inst_voff[i + 1] - s->h_inst_voff[i]);
-      shape.T = team_cluster(L, px_count, max_n, 5);
+      shape.T = team_of_batch(px_count, max_n, max_pins, L.num_sms, kmax);
     }
     if (tuned && tu.mode == LPGPU_MODE_PERSISTENT) {
       shape.per_sm = tu.ctas_per_sm;
@@ -1517,9 +1526,11 @@ lpgpu_status lpgpu_stepper_launch(lpgpu_stepper* t, lpgpu_session* const* sessio
   const Launch L{t->st, t->num_sms};
   // the groups of a round run side by side, so the team size follows their total;
   // all teams are resident at once, which leaves room for other sessions' work
-  int64_t max_n = 0;
+  int64_t max_n = 0, max_pins = 0;
   for (const PxInst& x : t->h) max_n = std::max(max_n, x.v1 - x.v0);
-  const int T = rows > 0 ? team_cluster(L, (int64_t)rows, max_n, 2) : 1;
+  for (int32_t i = 0; i < count; ++i)
+    for (int64_t p : sessions[i]->h_inst_pins) max_pins = std::max(max_pins, p);
+  const int T = rows > 0 ? team_of_many((int64_t)rows, max_n, max_pins, L.num_sms, 2) : 1;
   int64_t own_bytes = 0;
   for (int32_t i = 0; i < count; ++i) {
     const lpgpu_session* s = sessions[i];

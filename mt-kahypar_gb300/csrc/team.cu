@@ -73,21 +73,6 @@ int64_t team_own_bytes(int64_t n, int64_t m, int64_t pins, int T, int k, int W, 
   return all <= most ? all : nets <= most ? nets : own;
 }
 
-// Larger teams finish the largest instance sooner, more of them keep the SMs
-// busy; a batch is fastest with clusters as large as keep per_sm = 5 (of which
-// two are resident at once).
-// Whole refine, T = 1 / 2 / 4 / 8 / 16 (GB300, ms): 1,280 instances of up to
-// 65,536 vertices 16.1 / 20.2 / 27.3 / 42.1 / 87.9 (multi-launch pipeline 33.8);
-// 320: 11.3 / 6.9 / 7.2 / 10.7 / 22.3 (9.0); 80: 9.3 / 5.5 / 3.5 / 3.2 / 5.9
-// (3.9); 24: 8.9 / 5.2 / 3.1 / 2.0 / 2.2 (2.6); 1,280 of up to 4,096: 4.0 / 7.9 /
-// 14.4 / 27.9 / 68.1 (7.9). Up to 2,048 vertices one CTA is the fastest team of a
-// single instance too.
-int team_cluster(const Launch& L, int64_t count, int64_t max_n, int per_sm) {
-  int T = 1;
-  while (max_n > 2048 && T < 8 && count * 2 * T <= per_sm * (int64_t)L.num_sms) T *= 2;
-  return T;
-}
-
 int team_slots(const Launch& L, int64_t count, int T) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(count, 2 * (int64_t)L.num_sms / T));
 }

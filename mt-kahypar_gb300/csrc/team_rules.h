@@ -48,4 +48,47 @@ inline TeamShape team_shape(int64_t n, int64_t pins) {
   return {n < 655360 ? 1 : 2, 4, kTeamAll};
 }
 
+// Several instances, the largest of max_n vertices and of max_pins pins: CTAs per
+// team, with about `per_sm` CTAs' worth of teams per SM at most (stepped rounds, which
+// leave room for other sessions' work, ask for 2; a batch for 5, of which two are
+// resident at once). Larger teams finish the largest instance sooner, more of them
+// keep the SMs busy. Whole refine, T = 1 / 2 / 4 / 8 / 16 (GB300, ms): 1,280 instances
+// of up to 65,536 vertices 16.1 / 20.2 / 27.3 / 42.1 / 87.9 (multi-launch pipeline
+// 33.8); 320: 11.3 / 6.9 / 7.2 / 10.7 / 22.3 (9.0); 80: 9.3 / 5.5 / 3.5 / 3.2 / 5.9
+// (3.9); 24: 8.9 / 5.2 / 3.1 / 2.0 / 2.2 (2.6); 1,280 of up to 4,096: 4.0 / 7.9 / 14.4
+// / 27.9 / 68.1 (7.9).
+// One CTA serves what it serves alone (team_shape). Few vertices with many pins take
+// teams that are all resident: 37 of 2,048 vertices and 61,384 pins 1.89 / 1.54 / 1.39
+// / 2.03 / 3.04 (4.5), 204,633 pins 5.1 / 3.1 / 2.1 / 2.5 / 3.4 (8.4).
+inline int team_of_many(int64_t count, int64_t max_n, int64_t max_pins, int64_t num_sms, int per_sm) {
+  if (max_n <= 2048) {
+    if (max_pins + 4 * max_n <= 24576) return 1;
+    per_sm = 1;
+  }
+  int T = 1;
+  while (T < 8 && count * 2 * T <= per_sm * num_sms) T *= 2;
+  return T;
+}
+
+// The team of a batch of several instances. Clusters of 16 where every one of them
+// finds its SMs and the instances are large (us, clusters of 8 / 16): 2 of 16,384
+// vertices 1,037 / 931, 2 of 65,536 1,890 / 1,350, 8 of 65,536 k = 2 / 8 / 64 1,779 /
+// 1,570, 1,939 / 1,717, 2,640 / 2,362, but 8 of 4,096 831 / 870; for k > 128 an SM holds
+// one CTA, and 8 of 16,384 and k = 300 take 1,919 / 2,797.
+inline int team_of_batch(int64_t count, int64_t max_n, int64_t max_pins, int64_t num_sms, int kmax) {
+  const int T = team_of_many(count, max_n, max_pins, num_sms, 5);
+  return T == 8 && kmax <= 128 && max_pins > 65536 && count * 16 <= num_sms ? kTeamMaxCluster : T;
+}
+
+// A team's time is about 33 ns per pin of its instance and CTA. Where the largest
+// instance so outlasts the whole pipeline (its 1.1 ms of extra launches and 0.6 ns per
+// pin of the batch), the pipeline refines the batch. Pipeline / teams, us: 2 of 262,144
+// vertices and 5 pins each 3,012 / 5,467, 4 4,123 / 3,390 (16 CTAs), 8 7,270 / 6,205; 2
+// of 1M 9,190 / 21,508, 4 15,487 / 12,798 (16), 8 33,278 / 26,758; one of 65,536 beside 20
+// of 1,024 1,978 / 1,835, one of 262,144 2,338 / 5,414, one of 1M 4,887 / 20,318, beside
+// 200 5,785 / 77,412 (one CTA each).
+inline bool batch_wants_pipeline(int64_t max_pins, int64_t sum_pins, int T) {
+  return max_pins / T > 34000 + sum_pins / 55;
+}
+
 }  // namespace lpgpu

@@ -240,3 +240,38 @@ def test_dense_instances_stay_near_the_pipeline(lp, n, degree, size, k):
         default, got = _fastest(s, lp.default_config())
     assert np.array_equal(got, want)
     assert default < 2 * pipeline
+
+
+def _batch(lp, hgs, k, flags=0, rounds=3):
+    with lp.Session(0) as s:
+        s.upload_batch(hgs)
+        s.set_partition_batch([k] * len(hgs), [(np.arange(h.n) * 5 % k).astype(np.int32) for h in hgs], eps=0.03)
+        r = s.refine(lp.default_config(flags=flags, rounds=rounds))
+        return s.partition(), s.block_weights(), s.instance_km1(), (r.km1_before, r.km1_after, r.delta, r.moves)
+
+
+# batches around the pins at which the teams grow, clusters of 16 among them, and the pipeline takes over
+@pytest.mark.parametrize("count,n,pins,k", [(3, 2048, 16384, 5), (3, 2048, 16388, 5), (40, 2048, 16388, 5), (2, 16384, 65536, 3),
+                                            (2, 16384, 65540, 3), (9, 9000, 70000, 70), (10, 9000, 70000, 70), (2, 3000, 70000, 200),
+                                            (2, 700, 700 * 800, 33), (2, 700, 700 * 1000, 33)])
+def test_batch_team_sizes_by_pins(lp, count, n, pins, k):
+    hgs = [_dense(n, pins, 4, i) for i in range(count - 1)] + [_dense(300, 900, 3, 99)]
+    _same(_batch(lp, hgs, k), _batch(lp, hgs, k, flags=lp.FLAG_MULTI_LAUNCH))
+
+
+# One large instance among small ones: the batch stays near the pipeline (its
+# time here; the teams of 8 and of 1 CTAs took 2.2 and 10 times as long).
+@pytest.mark.parametrize("insts,k", [([(262144, 5, 4)] + [(1024, 5, 4)] * 20, 8),
+                                     ([(262144, 5, 4)] + [(1024, 5, 4)] * 400, 8)])
+def test_batches_stay_near_the_pipeline(lp, insts, k):
+    made = {x: _dense(x[0], x[0] * x[1] // x[2] * x[2], x[2], 5) for x in set(insts)}
+    hgs = [made[x] for x in insts]
+    rng = np.random.default_rng(8)
+    with lp.Session(0) as s:
+        s.upload_batch(hgs)
+        s.set_partition_batch([k] * len(hgs), [rng.permutation(np.arange(h.n) % k).astype(np.int32) for h in hgs], eps=0.03)
+        s.save_partition()
+        pipeline, want = _fastest(s, lp.default_config(flags=lp.FLAG_MULTI_LAUNCH))
+        default, got = _fastest(s, lp.default_config())
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
+    assert default < 1.7 * pipeline
