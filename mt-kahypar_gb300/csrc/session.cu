@@ -978,25 +978,21 @@ static lpgpu_tuning session_tuning(const lpgpu_session* s) {
 
 // ---- one instance refined by one team (team.cu)
 
-// The team of a single-instance refine when `in_flight` refines run on the device.
-static TeamShape shared_shape(int64_t n, int64_t pins, int num_sms, int in_flight) {
-  TeamShape t = team_shape(n, pins);
-  if (t.T == kTeamAll && in_flight > 1) t = {2, 4, 2 * num_sms / std::min(in_flight, 4)};
-  return t;
-}
-
-// Refine calls in progress per device: a cooperative grid over the whole GPU
-// keeps every other session's kernels out until it ends, so sessions that are
-// refined from several threads at once take an equal share of the SMs each (64
-// registers per thread, so that two CTAs fit an SM). 131,071 vertices, k = 64,
-// 1 / 2 / 4 threads, us per refine: whole grid 2,110 / 2,034 / 2,014, shares
-// 2,110 / 1,247 / 763 (multi-launch pipeline 3,508 / 1,952 / 1,154).
-static std::atomic<int> g_in_flight[16];
+// Refine calls in progress per device, and those among them whose team would be
+// the whole grid alone: what shared_team_shape shares the SMs out by. A count is
+// read once, at entry, so the first of several callers still takes the whole grid,
+// and the next ones wait for its one refine.
+static std::atomic<int> g_in_flight[16], g_grids[16];
 struct InFlight {
-  std::atomic<int>& c;
-  const int now;
-  explicit InFlight(int device) : c(g_in_flight[device & 15]), now(c.fetch_add(1) + 1) {}
-  ~InFlight() { c.fetch_sub(1); }
+  std::atomic<int>* c = nullptr;
+  int now = 0;  // with this call
+  void enter(std::atomic<int>* counts, int device) {
+    c = &counts[device & 15];
+    now = c->fetch_add(1) + 1;
+  }
+  ~InFlight() {
+    if (c) c->fetch_sub(1);
+  }
 };
 
 // Instance descriptors of the team rounds over the session's current state,
@@ -1144,7 +1140,6 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
   }
   if (cfg.flags & LPGPU_FLAG_MULTI_LAUNCH) use_team = false;
   DeviceGuard g(s->device);
-  const InFlight in_flight(s->device);
   s->gc_valid = false;  // refinement moves without gain-cache maintenance
   const int R = cfg.rounds, S = cfg.subrounds;
   Mem* fp = &s->mem;
@@ -1161,17 +1156,18 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
   // a flag or the session's own tuning settles the form; a row of the table is chosen
   // by the mean size and knows nothing of a batch's largest instance
   const bool must_team = s->has_tuning || (cfg.flags & LPGPU_FLAG_PERSISTENT);
-  if (use_team && !must_team)
-    use_team = px_count == 1 ? tuned || team_shape(s->n, s->P).T != kTeamNone
-                             : !batch_wants_pipeline(max_pins, s->P,
-                                                     team_of_batch(px_count, max_n, max_pins, s->num_sms, kmax));
+  InFlight all, grids;
+  all.enter(g_in_flight, s->device);
+  if (use_team && px_count == 1) {
+    if (team_shape(s->n, s->P).T == kTeamAll) grids.enter(g_grids, s->device);
+    shape = shared_team_shape(s->n, s->P, kmax, s->num_sms, grids.now, all.now);
+    use_team = must_team || shape.T != kTeamNone;
+  } else if (use_team) {
+    shape.T = team_of_batch(px_count, max_n, max_pins, s->num_sms, kmax);
+    use_team = must_team || !batch_wants_pipeline(max_pins, s->P, shape.T);
+  }
   if (use_team) {
     const Launch L = s->launch();
-    if (px_count == 1) {
-      shape = shared_shape(s->n, s->P, L.num_sms, in_flight.now);
-    } else {
-      shape.T = team_of_batch(px_count, max_n, max_pins, L.num_sms, kmax);
-    }
     if (tuned && tu.mode == LPGPU_MODE_PERSISTENT) {
       shape.per_sm = tu.ctas_per_sm;
       shape.unroll = tu.unroll;

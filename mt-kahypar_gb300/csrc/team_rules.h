@@ -48,6 +48,46 @@ inline TeamShape team_shape(int64_t n, int64_t pins) {
   return {n < 655360 ? 1 : 2, 4, kTeamAll};
 }
 
+// The same on a device with `all` refines in progress (this one included), `grids` of
+// which want the whole grid. A cooperative grid on every SM keeps the others out until
+// it ends: beside one of 131,071 vertices (k = 64) a 1,024-vertex refine takes 2,347
+// instead of 430 us, a pipeline 50 ms, and the grid gains nothing (2,347 us).
+// - One grid beside other refines leaves them room: with two CTAs per SM half of the
+//   GPU, a third of the CTAs from three refines on (us, the grid / the others. 131,071
+//   vertices and a small one: half 2,231 / 478, a third 2,248 / 487, a quarter 2,395 /
+//   472; and three clusters: 2,410 / 815, 2,272 / 820, 2,426 / 794; 1M and three small
+//   ones: 6,105 / 451, 6,313 / 447, 7,574 / 441). For k > 128 an SM holds one CTA:
+//   three quarters of the SMs, then two thirds (131,071 vertices in that build: 2,049 /
+//   480 and one cluster 2,026 / 794).
+// - Several grids take equal shares, of whole SMs up to 200,000 vertices and for 33 to
+//   64 blocks, of CTAs two to an SM above (us per refine, 2 / 4 / 8 threads, whole SMs |
+//   two CTAs per SM [pipeline]): 16,384 vertices 405 / 220 / 127 | 472 / 252 / 139 [780 /
+//   410 / 223]; 131,071, k = 64 1,177 / 841 / 617 | 1,317..1,811 / 991 / 681 [1,904 / 1,146 /
+//   784]; 400,003, k = 64 2,054 / 1,666 / 1,512 | 1,969 / 1,791 / 1,578 [2,434 / 1,679 /
+//   1,465]; 262,144, k = 16 1,376 / 1,022 / 824 | 1,252 / 885 / 684 [1,947 / 1,206 / 897];
+//   524,288, k = 8 1,178 / 897 / 766 | 1,076 / 737 / 592 [1,419 / 896 / 720]; 250,007, k =
+//   300 1,407 / 1,041 / 847 | - [2,365 / 1,721 / 1,558].
+// - The pipeline serves several large ones as well or better, from 589,824 vertices on
+//   (600,011 2,410 / 1,953 / 1,852 | 2,153..2,937 / 1,878 / 1,706 [2,550 / 1,813 / 1,660]; 1M
+//   4,171 / 3,764 / 3,853 | 3,905 / 3,214 / 3,314 [3,879 / 3,131 / 3,045]), and three from
+//   393,216 on for more than 32 blocks (500,000, k = 128: 1,277 / 1,217 / 994 [1,591 / 1,096 /
+//   995]).
+inline TeamShape shared_team_shape(int64_t n, int64_t pins, int k, int num_sms, int grids, int all) {
+  TeamShape t = team_shape(n, pins);
+  if (t.T != kTeamAll || all <= 1) return t;
+  if (grids > 1 && k <= 128 && (n >= 589824 || (grids > 2 && n >= 393216 && k > 32)))
+    return {t.per_sm, t.unroll, kTeamNone};
+  if (grids <= 1) {
+    t.per_sm = k > 128 ? 1 : 2;
+    t.T = k > 128 ? (all == 2 ? 3 * num_sms / 4 : 2 * num_sms / 3) : 2 * num_sms / (all < 3 ? all : 3);
+  } else {
+    t.per_sm = k <= 128 && n >= 200000 && (k <= 32 || k > 64) ? 2 : 1;
+    t.T = t.per_sm * num_sms / (all < 8 ? all : 8);
+  }
+  if (t.T <= kTeamMaxCluster) t.T = kTeamMaxCluster + 1;
+  return t;
+}
+
 // Several instances, the largest of max_n vertices and of max_pins pins: CTAs per
 // team, with about `per_sm` CTAs' worth of teams per SM at most (stepped rounds, which
 // leave room for other sessions' work, ask for 2; a batch for 5, of which two are
