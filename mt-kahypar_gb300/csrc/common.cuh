@@ -395,6 +395,9 @@ cudaError_t launch_px_round(const Launch& L, const PxInst* insts, const int32_t*
 // the records and pin counts.
 int64_t team_own_bytes(int64_t n, int64_t m, int64_t pins, int T, int k, int W, bool phi16,
                        int per_sm);
+// Whether the GPU can hold one team of T CTAs at once (a cluster needs its SMs within
+// one group of them, a grid all its CTAs; a partition of the GPU may have neither).
+bool team_fits(const Launch& L, int T, int W, bool unit, int unroll, int ctas_per_sm, int64_t own_bytes);
 // Teams of T CTAs that can be resident at once (an upper bound for clusters).
 int team_slots(const Launch& L, int64_t count, int T);
 // Largest number of CTAs of the kernel build that can be resident at once.

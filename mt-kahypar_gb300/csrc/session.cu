@@ -1177,10 +1177,24 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
       const int most = team_resident(L, s->W, s->unit_nets, shape.unroll, shape.per_sm);
       shape.T = shape.T == kTeamAll ? most : std::min(shape.T, most);
     }
-    for (int32_t i = 0; i < px_count; ++i)
-      own_bytes = std::max(own_bytes, team_own_bytes(s->h_inst_voff[i + 1] - s->h_inst_voff[i],
-                                                     s->h_inst_noff[i + 1] - s->h_inst_noff[i], s->h_inst_pins[i],
-                                                     shape.T, kmax, s->W, s->phi16(), shape.per_sm));
+    auto own_of = [&](int T) {
+      int64_t most = 0;
+      for (int32_t i = 0; i < px_count; ++i)
+        most = std::max(most, team_own_bytes(s->h_inst_voff[i + 1] - s->h_inst_voff[i],
+                                             s->h_inst_noff[i + 1] - s->h_inst_noff[i], s->h_inst_pins[i], T, kmax,
+                                             s->W, s->phi16(), shape.per_sm));
+      return most;
+    };
+    own_bytes = own_of(shape.T);
+    // no place for the team: the pipeline, or one CTA where the form is settled
+    if (!team_fits(L, shape.T, s->W, s->unit_nets, shape.unroll, shape.per_sm, own_bytes)) {
+      use_team = must_team;
+      shape.T = 1;
+      own_bytes = own_of(1);
+    }
+  }
+  if (use_team) {
+    const Launch L = s->launch();
     if (shape.T > 1) CK(s->team.alloc(team_scratch_words(kmax) * team_slots(L, px_count, shape.T), fp));
     ps = build_px(s, tu.order);
     if (ps != LPGPU_OK) return ps;
@@ -1526,14 +1540,28 @@ lpgpu_status lpgpu_stepper_launch(lpgpu_stepper* t, lpgpu_session* const* sessio
   for (const PxInst& x : t->h) max_n = std::max(max_n, x.v1 - x.v0);
   for (int32_t i = 0; i < count; ++i)
     for (int64_t p : sessions[i]->h_inst_pins) max_pins = std::max(max_pins, p);
-  const int T = rows > 0 ? team_of_many((int64_t)rows, max_n, max_pins, L.num_sms, 2) : 1;
-  int64_t own_bytes = 0;
-  for (int32_t i = 0; i < count; ++i) {
-    const lpgpu_session* s = sessions[i];
-    for (size_t j = 0; j < s->h_px.size(); ++j)
-      own_bytes = std::max(own_bytes, team_own_bytes(s->h_px[j].v1 - s->h_px[j].v0, s->h_px[j].e1 - s->h_px[j].e0,
-                                                     s->h_inst_pins[j], T, s->h_px[j].kstride, s->W, s->phi16(), 2));
+  int T = rows > 0 ? team_of_many((int64_t)rows, max_n, max_pins, L.num_sms, 2) : 1;
+  auto own_of = [&](int teams_of) {
+    int64_t most = 0;
+    for (int32_t i = 0; i < count; ++i) {
+      const lpgpu_session* s = sessions[i];
+      for (size_t j = 0; j < s->h_px.size(); ++j)
+        most = std::max(most, team_own_bytes(s->h_px[j].v1 - s->h_px[j].v0, s->h_px[j].e1 - s->h_px[j].e0,
+                                             s->h_inst_pins[j], teams_of, s->h_px[j].kstride, s->W, s->phi16(), 2));
+    }
+    return most;
+  };
+  // the kernel build of a group is that of its first session's tuning when that is a
+  // persistent one, else 2 CTAs per SM with unroll 8
+  std::vector<std::pair<int, int>> builds;  // unroll, CTAs per SM
+  for (const auto& gr : ranges) {
+    const lpgpu_tuning tu = session_tuning(sessions[groups[gr.first].front()]);
+    const bool tuned = tu.mode == LPGPU_MODE_PERSISTENT;
+    builds.push_back({tuned ? tu.unroll : 8, tuned ? tu.ctas_per_sm : 2});
+    while (!team_fits(L, T, gr.first.W, gr.first.unit != 0, builds.back().first, builds.back().second, own_of(T)))
+      T /= 2;
   }
+  const int64_t own_bytes = own_of(T);
   const int64_t words = team_scratch_words(kPxMaxK);
   const size_t G = ranges.size();
   if (t->queue.count < 2 * G) CK(t->queue.alloc(2 * G, &t->mem));
@@ -1547,10 +1575,6 @@ lpgpu_status lpgpu_stepper_launch(lpgpu_stepper* t, lpgpu_session* const* sessio
   for (size_t gi = 0; gi < G; ++gi) {
     const auto& gr = ranges[gi];
     const Group& k = gr.first;
-    // the kernel build of the group's first session's tuning when that is a
-    // persistent one, else 2 CTAs per SM with unroll 8
-    const lpgpu_tuning tu = session_tuning(sessions[groups[k].front()]);
-    const bool tuned = tu.mode == LPGPU_MODE_PERSISTENT;
     PxParams P{};
     P.S = k.S;
     P.zero_gain = k.zero_gain;
@@ -1562,7 +1586,7 @@ lpgpu_status lpgpu_stepper_launch(lpgpu_stepper* t, lpgpu_session* const* sessio
     P.activate_last = 1;
     P.T = T;
     P.kcap = kPxMaxK;
-    P.unroll = tuned ? tu.unroll : 8;
+    P.unroll = builds[gi].first;
     Launch Lg = L;
     const int lane = (int)(gi % 4) - 1;  // -1: the stepper's own stream
     if (lane >= 0) {
@@ -1574,7 +1598,7 @@ lpgpu_status lpgpu_stepper_launch(lpgpu_stepper* t, lpgpu_session* const* sessio
       CK(cudaStreamWaitEvent(Lg.st, t->ev, 0));
     }
     CK(launch_px_round(Lg, t->table.p + gr.second.first, nullptr, gr.second.second, P, k.W, k.unit != 0,
-                       tuned ? tu.ctas_per_sm : 2, team_slots(L, gr.second.second, T),
+                       builds[gi].second, team_slots(L, gr.second.second, T),
                        T > 1 ? t->team.p + used : nullptr, t->queue.p + 2 * gi, t->queue.p + 2 * gi + 1, own_bytes,
                        false));
     if (T > 1) used += words * team_slots(L, gr.second.second, T);

@@ -98,6 +98,63 @@ cudaError_t launch_px_active(const Launch& L, const PxInst* insts, int32_t count
   return launched("k_px_active");
 }
 
+// One launch of the kernel: build, shared memory, how its teams meet.
+namespace {
+struct TeamLaunch {
+  const void* kern;
+  size_t smem, base;
+  int resident;  // CTAs of the build that the GPU holds
+  TeamSync sync;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at{};
+  TeamLaunch(const Launch& L, int T, int W, bool unit, int unroll, int ctas_per_sm, int64_t own_bytes) {
+    const int minb = team_min_blocks(W, ctas_per_sm);
+    kern = team_kernel_for(W, unit, unroll, minb);
+    smem = team_smem_bytes(minb, T, W, own_bytes);
+    base = team_smem_base(W, minb < 2);
+    resident = L.num_sms * team_occupancy(kern, minb, smem);
+    sync = T == 1 ? kSyncCta : T > kTeamMaxCluster ? kSyncGrid : kSyncCluster;
+    cfg.gridDim = dim3((unsigned)T);
+    cfg.blockDim = dim3(kTeamThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = L.st;
+  }
+  // Attributes of the launch, once the object has its place.
+  cudaError_t attributes(int T) {
+    if (sync == kSyncCta) return cudaSuccess;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (sync == kSyncGrid) {
+      at.id = cudaLaunchAttributeCooperative;
+      at.val.cooperative = 1;
+      return cudaSuccess;
+    }
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)T;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    return T > 8 ? cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) : cudaSuccess;
+  }
+};
+}  // namespace
+
+// Most CTAs a team may have; a smaller limit stands in for a GPU partition.
+#ifndef LPGPU_TEAM_MOST
+#define LPGPU_TEAM_MOST (1 << 20)
+#endif
+
+bool team_fits(const Launch& L, int T, int W, bool unit, int unroll, int ctas_per_sm, int64_t own_bytes) {
+  if (T <= 1) return true;
+  if (T > LPGPU_TEAM_MOST) return false;
+  TeamLaunch t(L, T, W, unit, unroll, ctas_per_sm, own_bytes);
+  if (t.sync == kSyncGrid) return T <= t.resident;
+  int clusters = 0;
+  if (t.attributes(T) != cudaSuccess || cudaOccupancyMaxActiveClusters(&clusters, t.kern, &t.cfg) != cudaSuccess) {
+    cudaGetLastError();  // no cluster of this size: the answer, not a failure
+    return false;
+  }
+  return clusters > 0;
+}
+
 cudaError_t launch_px_round(const Launch& L, const PxInst* insts, const int32_t* order, int32_t count, PxParams P,
                             int W, bool unit, int ctas_per_sm, int teams, int64_t* scratch, int64_t* queue,
                             int64_t* err, int64_t own_bytes, bool cleared) {
@@ -114,36 +171,16 @@ cudaError_t launch_px_round(const Launch& L, const PxInst* insts, const int32_t*
   } else {
     scratch = nullptr;
   }
-  const int minb = team_min_blocks(W, ctas_per_sm);
-  const void* kern = team_kernel_for(W, unit, P.unroll, minb);
-  const size_t smem = team_smem_bytes(minb, P.T, W, own_bytes), base = team_smem_base(W, minb < 2);
-  P.resident = (int32_t)(smem - base);
-  const int resident = L.num_sms * team_occupancy(kern, minb, smem);
-  if (grid && P.T > resident) return cudaErrorCooperativeLaunchTooLarge;
-  teams = std::max(1, std::min(teams, std::min<int>(count, std::max(1, resident / P.T))));
-  int sync = P.T == 1 ? kSyncCta : grid ? kSyncGrid : kSyncCluster;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(teams * P.T));
-  cfg.blockDim = dim3(kTeamThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = L.st;
-  cudaLaunchAttribute at[1];
-  cfg.attrs = at;
-  if (sync == kSyncCluster) {
-    if (P.T > 8 && (e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess)
-      return e;
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)P.T;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.numAttrs = 1;
-  } else if (sync == kSyncGrid) {
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.numAttrs = 1;
-  }
+  TeamLaunch t(L, P.T, W, unit, P.unroll, ctas_per_sm, own_bytes);
+  P.resident = (int32_t)(t.smem - t.base);
+  if (grid && P.T > t.resident) return cudaErrorCooperativeLaunchTooLarge;
+  teams = std::max(1, std::min(teams, std::min<int>(count, std::max(1, t.resident / P.T))));
+  t.cfg.gridDim = dim3((unsigned)(teams * P.T));
+  if ((e = t.attributes(P.T)) != cudaSuccess) return e;
+  int sync = t.sync;
   void* args[] = {(void*)&insts, (void*)&order, (void*)&count, (void*)&P, (void*)&sync, (void*)&scratch,
                   (void*)&queue, (void*)&err};
-  e = cudaLaunchKernelExC(&cfg, kern, args);
+  e = cudaLaunchKernelExC(&t.cfg, t.kern, args);
   if (e != cudaSuccess) {
     set_error(std::string("k_team: ") + cudaGetErrorString(e));
     return e;
