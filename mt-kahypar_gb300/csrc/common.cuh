@@ -73,8 +73,6 @@ enum Scalar : int {
   kDeltaSub = 0,   // summed attributed delta of the current sub-round
   kAnyOverTo = 1,  // some target block overflows
   kAnyOverFrom = 2,
-  kKm1 = 3,        // km1 accumulator (metrics)
-  kCut = 4,        // cut accumulator (metrics)
   kPinTiles = 5,   // tile counter of the pin counts
   kApplyDelta = 6, // apply_moves delta
   kDeltaRb = 7,    // delta of a sub-round rollback

@@ -289,19 +289,20 @@ __global__ void k_block_weights(RoundCtx c) {
 
 
 // Φ, Λ and Λ1 (blocks holding exactly one pin of the net) from scratch
-// (initializePinCountInPart, h:1086-1110), fused with the km1 / cut sums. A CTA
-// takes `tn` consecutive nets, whose pins, Φ rows and records are one contiguous
-// range each: the threads spread over the pins (the net of a pin by binary
-// search in the tile's offsets), count in an image of the Φ rows in shared
+// (initializePinCountInPart, h:1086-1110). A CTA takes `tn` consecutive nets,
+// whose pins, Φ rows and records are one contiguous range each: the threads
+// spread over the pins (the net of a pin by binary search in the tile's
+// offsets), count in an image of the Φ rows in shared
 // memory, and the image and the records are then written in whole lines, zeros
 // included. The count an atomic returns drives the bits as in the commit: Λ when
 // it leaves 0, Λ1 whenever it enters or leaves 1. Four pins per thread are in
 // flight and a large net keeps the whole CTA busy; one warp per 32 nets walked
 // about ten dependent 32-pin groups one after another and wrote single entries.
-// initializePartition, before -> after: 1M vertices k = 32 153 -> 130 us, row-net
-// 1M k = 61 143 -> 129, 250,007 k = 300 93 -> 81, 16,384 21.5 -> 17.3; row-net
-// 4.2M k = 128 527 -> 552 (1.1 GB of Φ rows, mostly zeros). Net e's record is conn[e * 2W .. e * 2W + 2W): W words of Λ(e),
-// then W words of Λ1(e).
+// initializePartition, before -> after: 1M vertices k = 32 155 -> 125 us, row-net
+// 1M k = 61 143 -> 125, 250,007 k = 300 98 -> 75, 16,384 24.0 -> 19.8, row-net
+// 4.2M k = 128 530 -> 515 (1.1 GB of Φ rows, mostly zeros; 548 when it also summed
+// km1 and the cut, which every query computes for itself). Net e's record is
+// conn[e * 2W .. e * 2W + 2W): W words of Λ(e), then W words of Λ1(e).
 constexpr int kPinTile = 256;  // threads per CTA
 constexpr int kPinNets = 256;  // most nets per tile
 template <bool PHI16, bool BATCHED>
@@ -316,7 +317,6 @@ __global__ void __launch_bounds__(kPinTile) k_pin_counts(RoundCtx c, int tn) {
   uint32_t* s_rec = s_phi + row_words;
   Off* s_off = reinterpret_cast<Off*>(s_rec + ((tn * 2 * W + 3) & ~3));
   int* s_bo = reinterpret_cast<int*>(s_off + tn + 1);
-  int64_t km1 = 0, cut = 0;
   __shared__ int64_t s_tile;
   // tiles from a counter: power-law nets make them uneven
   for (;;) {
@@ -380,29 +380,15 @@ __global__ void __launch_bounds__(kPinTile) k_pin_counts(RoundCtx c, int tn) {
       for (int i = threadIdx.x; i < words; i += kPinTile) reinterpret_cast<uint32_t*>(out)[i] = s_phi[i];
     }
     for (int i = threadIdx.x; i < nets * 2 * W; i += kPinTile) c.conn[e0 * 2 * W + i] = s_rec[i];
-    for (int i = threadIdx.x; i < nets; i += kPinTile) {
-      int lam = 0;
-      for (int w = 0; w < W; ++w) lam += __popc(s_rec[i * 2 * W + w]);
-      if (lam > 1) {
-        const int64_t we = c.w_e[e0 + i];
-        km1 += (int64_t)(lam - 1) * we;
-        cut += we;
-      }
-    }
     __syncthreads();  // the image is cleared for the next tile
-  }
-  km1 = block_sum_i64(km1);
-  cut = block_sum_i64(cut);
-  if (threadIdx.x == 0) {
-    if (km1) atomicAdd(reinterpret_cast<ull*>(&c.scal[kKm1]), (ull)km1);
-    if (cut) atomicAdd(reinterpret_cast<ull*>(&c.scal[kCut]), (ull)cut);
   }
 }
 
 // Nets per tile: an image of at most 24 KB (initializePartition of row-net 4.2M,
-// k = 128 / geometric 250,007, k = 300: 8 KB 722 / 124 us, 16 KB 544 / 91, 24 KB
-// 552 / 81, 32 KB 554 / 82), an even number so that every tile starts on a word
-// of 16-bit entries, and at least two tiles per SM where the nets allow it.
+// k = 128 / geometric 250,007, k = 300: 8 KB 623 / 107 us, 16 KB 493 / 81, 20 KB 490 /
+// 76, 24 KB 515 / 75, 32 KB 519 / 75; others within 2 %), an even number so that
+// every tile starts on a word of 16-bit entries, and at least two tiles per SM
+// where the nets allow it.
 static int pin_tile(const Launch& L, const RoundCtx& c) {
   const int64_t row = (int64_t)c.kmax * (c.phi16 ? 2 : 4);
   int64_t tn = std::min<int64_t>(kPinNets, std::max<int64_t>(2, 24576 / row));
@@ -413,9 +399,7 @@ static int pin_tile(const Launch& L, const RoundCtx& c) {
 cudaError_t launch_init_partition(const Launch& L, const RoundCtx& c) {
   cudaError_t e;
   if ((e = cudaMemsetAsync(c.bw, 0, sizeof(int64_t) * c.k, L.st)) != cudaSuccess) return e;
-  // km1, cut and the tile counter
-  static_assert(kCut == kKm1 + 1 && kPinTiles == kKm1 + 2, "cleared together");
-  if ((e = cudaMemsetAsync(c.scal + kKm1, 0, sizeof(int64_t) * 3, L.st)) != cudaSuccess) return e;
+  if ((e = cudaMemsetAsync(c.scal + kPinTiles, 0, sizeof(int64_t), L.st)) != cudaSuccess) return e;
   if (c.n > 0) {
     k_block_weights<<<grid_for(L, c.n, 256, 8), 256, c.batched ? 0 : sizeof(ull) * c.k, L.st>>>(c);
     LAUNCHED("k_block_weights");
