@@ -180,10 +180,11 @@ struct lpgpu_session_s {
   std::vector<int64_t> h_inst_voff, h_inst_noff, h_inst_weight;
   std::vector<int64_t> h_inst_pins;  // pins of every instance (work estimate of the team rounds)
   std::vector<int32_t> h_inst_boff, h_inst_k;
-  // team rounds: instance descriptors, work order, the rule it follows
+  // team rounds: instance descriptors, work order, the rule and the pins it follows
   DevBuf<PxInst> px;
   DevBuf<int32_t> px_order;
   int px_order_rule = 0;
+  std::vector<int64_t> h_px_pins;
   bool has_tuning = false;
   lpgpu_tuning tuning{};
   std::vector<PxInst> h_px;  // host copy of the descriptors
@@ -996,8 +997,9 @@ struct InFlight {
 };
 
 // Instance descriptors of the team rounds over the session's current state,
-// and the work order. They are compared by content with what the device holds:
-// a session that takes another input can keep all its buffers and sizes.
+// and the work order. Both are compared by content with what the device holds (the
+// order by the pins that it is sorted by): a session that takes another input can
+// keep all its buffers and sizes.
 static lpgpu_status build_px(lpgpu_session* s, int order) {
   const int32_t I = s->batched ? s->num_inst : 1;
   std::vector<PxInst> h(I);
@@ -1038,7 +1040,7 @@ static lpgpu_status build_px(lpgpu_session* s, int order) {
     x.round = 0;
   }
   static_assert(std::is_trivially_copyable<PxInst>::value && sizeof(PxInst) % 8 == 0, "compared bytewise");
-  if (s->px.p && s->px_order_rule == order && s->h_px.size() == h.size() &&
+  if (s->px.p && s->px_order_rule == order && s->h_px_pins == s->h_inst_pins && s->h_px.size() == h.size() &&
       std::memcmp(s->h_px.data(), h.data(), sizeof(PxInst) * h.size()) == 0)
     return LPGPU_OK;
   s->h_px.clear();
@@ -1054,6 +1056,7 @@ static lpgpu_status build_px(lpgpu_session* s, int order) {
   CK(cudaMemcpyAsync(s->px_order.p, ord.data(), sizeof(int32_t) * I, cudaMemcpyHostToDevice, s->st));
   CK(cudaStreamSynchronize(s->st));
   s->h_px = std::move(h);
+  s->h_px_pins = s->h_inst_pins;
   s->px_order_rule = order;
   return LPGPU_OK;
 }
