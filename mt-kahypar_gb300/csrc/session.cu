@@ -2088,11 +2088,11 @@ lpgpu_status lpgpu_session_rebalance(lpgpu_session* s, int32_t max_rounds, lpgpu
     }
   }
   if (moved_before) {
-    double unused = 0;
-    ps = read_metrics(s, &km1_after, nullptr, &unused);
+    CK(cudaMemsetAsync(s->rep.p, 0, sizeof(int64_t) * kRepHead, st));
+    ps = fetch_report(s, nullptr, 0, &h, true);
     if (ps != LPGPU_OK) return ps;
-    CK(cudaMemcpyAsync(hb.data(), s->bw.p, sizeof(int64_t) * k, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    km1_after = h[kRepAfter];
+    hb.assign(h.begin() + kRepHead, h.end());
   }
   for (int r = 0; r < R; ++r) {
     bool over = false;
