@@ -154,10 +154,20 @@ struct Team {
   int builds;    // active lists built so far
 };
 
+// Limit of a grid barrier's wait: clocks (about 20 s: a barrier waits for the slowest
+// CTA's phase, one net of a billion pins takes a second, and a GPU that is shared in
+// time counts its absence), looked at every so many polls (a power of two).
+#ifndef LPGPU_TEAM_WAIT_CLOCKS
+#define LPGPU_TEAM_WAIT_CLOCKS 40000000000ll
+#endif
+#ifndef LPGPU_TEAM_WAIT_POLLS
+#define LPGPU_TEAM_WAIT_POLLS 1024u
+#endif
+
 // Barrier of the team: everything its CTAs wrote before is visible after. The
-// grid barrier (one arrival per CTA on a counter that only grows) gives up
-// after about 20 s of polling and then raises the team's abort flag, which
-// ends the kernel in every CTA; false: aborted.
+// grid barrier (one arrival per CTA on a counter that only grows) gives up at
+// its limit and then raises the team's abort flag, which ends the kernel in
+// every CTA; false: aborted.
 template <typename TS>
 __device__ __forceinline__ bool team_sync(Team& tm, TS& s) {
   if (tm.sync == kSyncCta) {
@@ -180,8 +190,8 @@ __device__ __forceinline__ bool team_sync(Team& tm, TS& s) {
       ull seen;
       asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(tm.G.arrivals()) : "memory");
       if (seen >= tm.arrivals) break;
-      if ((polls & 1023u) == 1023u) {
-        if (*(volatile int64_t*)tm.G.abort_flag() || clock64() - t0 > 40000000000ll) {
+      if ((polls & (LPGPU_TEAM_WAIT_POLLS - 1)) == LPGPU_TEAM_WAIT_POLLS - 1) {
+        if (*(volatile int64_t*)tm.G.abort_flag() || clock64() - t0 > LPGPU_TEAM_WAIT_CLOCKS) {
           *(volatile int64_t*)tm.G.abort_flag() = 1;
           s.abort = 1;
           break;

@@ -301,3 +301,24 @@ def test_batch_order_follows_the_input(lp):
         got, b = _fastest(s, cfg, 8)
     assert all(np.array_equal(x, y) for x, y in zip(a, b))
     assert got < 1.2 * want
+
+
+# the pipeline captures its launches once and replays them: the same from every start, and as launched directly
+def test_pipeline_graph_replay(lp):
+    from lpgpu import gen
+    inst = gen.random_small(21, n=4000, m=5000, k=12)
+    with lp.Session(0) as s:
+        s.upload(inst.hg)
+        s.set_partition(12, inst.part, eps=0.03)
+        s.save_partition()
+        got, launches = [], []
+        for flags in (lp.FLAG_MULTI_LAUNCH, lp.FLAG_MULTI_LAUNCH, lp.FLAG_MULTI_LAUNCH | lp.FLAG_NO_GRAPH, lp.FLAG_MULTI_LAUNCH):
+            s.restore_partition()
+            before = lp.kernel_launches()
+            r = s.refine(lp.default_config(flags=flags))
+            launches.append(lp.kernel_launches() - before)
+            got.append((s.partition(), s.pin_counts(), [[x[q] for q in KEYS] for x in s.round_stats()],
+                        (r.km1_before, r.km1_after, r.delta, r.moves)))
+        for x in got[1:]:
+            _same(got[0], x)
+        assert len(set(launches)) == 1

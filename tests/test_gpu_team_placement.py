@@ -2,14 +2,9 @@
 a cooperative grid) the refine takes the pipeline, or one CTA when its form is
 settled. The library is linked a second time with a limit on the team in place of
 such a partition, and runs in a process of its own."""
-import glob
-import os
-import subprocess
-import sys
-
 import pytest
 
-from conftest import PKG, ROOT
+from variant import run_with_variant
 
 pytestmark = pytest.mark.gpu
 
@@ -69,15 +64,4 @@ print("ok")
 
 @pytest.mark.parametrize("most", [1, 4, 16])
 def test_refines_without_room_for_their_team(lp, tmp_path, most):
-    import importlib.util
-    spec = importlib.util.spec_from_file_location("_lpgpu_build", os.path.join(PKG, "build.py"))
-    recipe = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(recipe)
-    obj, so = str(tmp_path / "team.o"), str(tmp_path / "liblpgpu_most.so")
-    subprocess.run([recipe.nvcc()] + recipe.ARCH + recipe.NVCC_FLAGS + ["-DLPGPU_TEAM_MOST=%d" % most, "-c",
-                   os.path.join(recipe.CSRC, "team.cu"), "-o", obj], check=True)
-    others = [o for o in glob.glob(os.path.join(recipe.BUILD, "*.o")) if os.path.basename(o) != "team.o"]
-    subprocess.run([recipe.nvcc()] + recipe.ARCH + ["-shared", "-o", so, obj] + others + ["-cudart", "static"], check=True)
-    r = subprocess.run([sys.executable, "-c", PROGRAM, so, str(most)], capture_output=True, text=True, timeout=300,
-                       env=dict(os.environ, PYTHONPATH=os.pathsep.join([PKG, ROOT])))
-    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
+    run_with_variant(tmp_path, "team.cu", ["-DLPGPU_TEAM_MOST=%d" % most], PROGRAM, str(most))
