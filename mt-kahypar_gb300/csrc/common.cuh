@@ -58,6 +58,14 @@ __host__ __device__ inline int subround_of(int64_t v, int round, int S) {
                (uint32_t)S);
 }
 
+// Nets are cut into units of about equal work for the pin counts: net e starts at
+// net_off[e] + kUnitNet * e on a scale of pins and nets (a net's row and record cost
+// as much as kUnitNet pins), and unit u holds the nets that start in
+// [u * kUnit, (u + 1) * kUnit).
+constexpr int64_t kUnit = 256, kUnitNet = 16;
+__host__ __device__ inline int64_t net_place(int64_t off, int64_t e) { return off + kUnitNet * e; }
+__host__ __device__ inline int64_t net_units(int64_t m, int64_t P) { return net_place(P, m) / kUnit + 1; }
+
 // Candidate ordering key: (gain, vertex) as one unsigned 64-bit integer. The
 // gain maps to (gain - 1) XOR 2^31, which keeps the order of every gain above
 // INT32_MIN (gains stay within +-INT32_MAX) and sends the non-positive gains of
@@ -235,8 +243,9 @@ int64_t scan_tmp_elems(int64_t count);
 cudaError_t launch_build_incidence(const Launch& L, int64_t n, int64_t m, int64_t P, const int64_t* net_off,
                                    const int32_t* pins, int64_t* vtx_off, int32_t* inets,
                                    int32_t* rank, int64_t* scan_tmp, int64_t scan_tmp_elems,
-                                   int64_t* deg_hist);
-cudaError_t launch_init_partition(const Launch& L, const RoundCtx& c);
+                                   int64_t* deg_hist, int32_t* unit_first);
+// unit_first: the first net of each of the `units` units, and m (launch_build_incidence).
+cudaError_t launch_init_partition(const Launch& L, const RoundCtx& c, const int32_t* unit_first, int64_t units);
 // Adds km1 and cut to out[0] and out[1] (zeroed by the caller).
 cudaError_t launch_metrics(const Launch& L, const RoundCtx& c, int64_t* out);
 // What team rounds need before their first round: metrics before (added to before[0] and before[1], zeroed by

@@ -174,13 +174,14 @@ __global__ void k_degree_hist(int64_t n, const int64_t* __restrict__ cnt, int64_
 // sectors of their vertices' lists stay in L2 until they are complete (a
 // grid-stride loop lets CTAs drift apart over nets of uneven size). A warp per 32
 // nets walked its pins in dependent 32-pin groups: 400K vertices 99 -> 43 us,
-// row-net 4.2M 917 -> 680 us.
+// row-net 4.2M 917 -> 680 us. The tile's offsets also give the units' first nets.
 constexpr int kScatterNets = 128;
 __global__ void __launch_bounds__(256) k_scatter_incidence(int64_t m, const int64_t* __restrict__ net_off,
                                                            const int32_t* __restrict__ pins,
                                                            const int64_t* __restrict__ vtx_off,
                                                            const int32_t* __restrict__ rank,
-                                                           int32_t* __restrict__ inets, ull* next_net) {
+                                                           int32_t* __restrict__ inets, ull* next_net,
+                                                           int32_t* __restrict__ unit_first) {
   __shared__ int64_t s_off[kScatterNets + 1];
   __shared__ ull s_next;
   for (;;) {
@@ -192,6 +193,17 @@ __global__ void __launch_bounds__(256) k_scatter_incidence(int64_t m, const int6
     for (int i = threadIdx.x; i <= nets; i += blockDim.x) s_off[i] = net_off[e0 + i];
     __syncthreads();
     const int64_t p1 = s_off[nets];
+    // units that start behind this tile's first net: the first net at or behind the start
+    const int64_t u0 = e0 > 0 ? net_place(s_off[0], e0) / kUnit + 1 : 0, u1 = net_place(p1, e0 + nets) / kUnit;
+    for (int64_t u = u0 + threadIdx.x; u <= u1; u += blockDim.x) {
+      int lo = 0, hi = nets;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (net_place(s_off[mid], e0 + mid) >= u * kUnit) hi = mid; else lo = mid + 1;
+      }
+      unit_first[u] = (int32_t)(e0 + lo);
+    }
+    if (e0 + nets == m && threadIdx.x == 0) unit_first[u1 + 1] = (int32_t)m;
     for (int64_t j0 = s_off[0] + threadIdx.x; j0 < p1; j0 += 4 * (int64_t)blockDim.x) {
       int64_t at[4];
       int r[4];
@@ -223,7 +235,7 @@ __global__ void __launch_bounds__(256) k_scatter_incidence(int64_t m, const int6
 cudaError_t launch_build_incidence(const Launch& L, int64_t n, int64_t m, int64_t P, const int64_t* net_off,
                                    const int32_t* pins, int64_t* vtx_off, int32_t* inets,
                                    int32_t* rank, int64_t* scan_tmp, int64_t scan_tmp_elems,
-                                   int64_t* deg_hist) {
+                                   int64_t* deg_hist, int32_t* unit_first) {
   cudaError_t e = cudaMemsetAsync(vtx_off, 0, sizeof(int64_t) * (n + 1), L.st);
   if (e != cudaSuccess) return e;
   if (P > 0) {
@@ -243,7 +255,7 @@ cudaError_t launch_build_incidence(const Launch& L, int64_t n, int64_t m, int64_
     ull* next_net = reinterpret_cast<ull*>(scan_tmp);  // free again after the scan
     if ((e = cudaMemsetAsync(next_net, 0, sizeof(ull), L.st)) != cudaSuccess) return e;
     k_scatter_incidence<<<grid_for(L, (m + kScatterNets - 1) / kScatterNets, 1, 8), 256, 0, L.st>>>(
-        m, net_off, pins, vtx_off, rank, inets, next_net);
+        m, net_off, pins, vtx_off, rank, inets, next_net, unit_first);
     LAUNCHED("k_scatter_incidence");
   }
   return cudaGetLastError();
@@ -289,114 +301,128 @@ __global__ void k_block_weights(RoundCtx c) {
 
 
 // Φ, Λ and Λ1 (blocks holding exactly one pin of the net) from scratch
-// (initializePinCountInPart, h:1086-1110). A CTA takes `tn` consecutive nets,
-// whose pins, Φ rows and records are one contiguous range each: the threads
-// spread over the pins (the net of a pin by binary search in the tile's
-// offsets), count in an image of the Φ rows in shared
+// (initializePinCountInPart, h:1086-1110). A CTA takes the next `span` units of
+// nets, up to `tn` nets at a time; their pins, Φ rows and records are one
+// contiguous range each: the threads spread over the pins (the net of a pin by
+// binary search in the offsets), count in an image of the Φ rows in shared
 // memory, and the image and the records are then written in whole lines, zeros
 // included. The count an atomic returns drives the bits as in the commit: Λ when
 // it leaves 0, Λ1 whenever it enters or leaves 1. Four pins per thread are in
 // flight and a large net keeps the whole CTA busy; one warp per 32 nets walked
 // about ten dependent 32-pin groups one after another and wrote single entries.
-// initializePartition, before -> after: 1M vertices k = 32 155 -> 125 us, row-net
-// 1M k = 61 143 -> 125, 250,007 k = 300 98 -> 75, 16,384 24.0 -> 19.8, row-net
-// 4.2M k = 128 530 -> 515 (1.1 GB of Φ rows, mostly zeros; 548 when it also summed
-// km1 and the cut, which every query computes for itself). Net e's record is
+// Units are cut by pins and nets, so large nets side by side (sorted by size,
+// say) go to many CTAs: with a fixed number of nets per CTA 256 nets of 60,000
+// pins took 26,597 us (a warp per 32 nets: 5,119), now 145; Zipf 1M sorted by size 1,240
+// (578), now 114.
+// initializePartition, a warp per 32 nets -> now: 1M vertices k = 32 155 -> 124 us,
+// row-net 1M k = 61 143 -> 122, 250,007 k = 300 98 -> 81, 16,384 24.0 -> 20.0, row-net
+// 4.2M k = 128 530 -> 527 (1.1 GB of Φ rows, mostly zeros). Net e's record is
 // conn[e * 2W .. e * 2W + 2W): W words of Λ(e), then W words of Λ1(e).
 constexpr int kPinTile = 256;  // threads per CTA
-constexpr int kPinNets = 256;  // most nets per tile
+constexpr int kPinNets = 256;  // most nets at a time
 template <bool PHI16, bool BATCHED>
-__global__ void __launch_bounds__(kPinTile) k_pin_counts(RoundCtx c, int tn) {
+__global__ void __launch_bounds__(kPinTile) k_pin_counts(RoundCtx c, int tn, int span, const int32_t* __restrict__ unit_first,
+                                                         int64_t units) {
   extern __shared__ __align__(16) unsigned char s_pin[];
   // offsets inside a tile: 16-bit entries mean nets of fewer than 2^16 pins
   using Off = typename std::conditional<PHI16, int32_t, int64_t>::type;
   constexpr int esz = PHI16 ? 2 : 4;
   const int k = c.kmax, W = c.W;
-  const int row_words = (tn * k * esz + 15) >> 4 << 2;  // the image, in whole 16-byte units
+  const int row_words = (tn * k * esz + 15) >> 4 << 2;  // room for the image, in whole 16-byte units
   uint32_t* s_phi = reinterpret_cast<uint32_t*>(s_pin);
   uint32_t* s_rec = s_phi + row_words;
   Off* s_off = reinterpret_cast<Off*>(s_rec + ((tn * 2 * W + 3) & ~3));
   int* s_bo = reinterpret_cast<int*>(s_off + tn + 1);
-  __shared__ int64_t s_tile;
-  // tiles from a counter: power-law nets make them uneven
+  __shared__ int64_t s_unit;
   for (;;) {
-    if (threadIdx.x == 0) s_tile = (int64_t)atomicAdd(reinterpret_cast<ull*>(&c.scal[kPinTiles]), 1ull) * tn;
+    if (threadIdx.x == 0) s_unit = (int64_t)atomicAdd(reinterpret_cast<ull*>(&c.scal[kPinTiles]), 1ull) * span;
     __syncthreads();
-    const int64_t e0 = s_tile;
-    if (e0 >= c.m) break;
-    const int nets = (int)(c.m - e0 < tn ? c.m - e0 : tn);
-    for (int i = threadIdx.x; i < (row_words >> 2); i += kPinTile) reinterpret_cast<uint4*>(s_phi)[i] = make_uint4(0, 0, 0, 0);
-    const int64_t p0 = c.net_off[e0];
-    for (int i = threadIdx.x; i < nets * 2 * W; i += kPinTile) s_rec[i] = 0;
-    for (int i = threadIdx.x; i <= nets; i += kPinTile) {
-      const int64_t o = c.net_off[e0 + i];
-      s_off[i] = (Off)(o - p0);
-      if (BATCHED && i < nets) s_bo[i] = c.net_off[e0 + i + 1] > o ? block_offset(c, c.pins[o]) : 0;
-    }
-    __syncthreads();
-    const Off p1 = s_off[nets];
-    const int32_t* pins = c.pins + p0;
-    for (Off j0 = threadIdx.x; j0 < p1; j0 += 4 * kPinTile) {
-      int b[4];
+    const int64_t u0 = s_unit, u1 = u0 + span;
+    if (u0 >= units) break;
+    // from an even net: every image starts on a word of 16-bit entries
+    const int64_t from = unit_first[u0] & ~1, to = u1 < units ? unit_first[u1] & ~1 : c.m;
+    if (from >= to) __syncthreads();  // s_unit is read
+    for (int64_t e0 = from; e0 < to; e0 += tn) {
+      const int nets = (int)(to - e0 < tn ? to - e0 : tn);
+      const int words = (nets * k * esz + 3) >> 2;
+      for (int i = threadIdx.x; i < (words + 3) >> 2; i += kPinTile) reinterpret_cast<uint4*>(s_phi)[i] = make_uint4(0, 0, 0, 0);
+      const int64_t p0 = c.net_off[e0];
+      for (int i = threadIdx.x; i < nets * 2 * W; i += kPinTile) s_rec[i] = 0;
+      for (int i = threadIdx.x; i <= nets; i += kPinTile) {
+        const int64_t o = c.net_off[e0 + i];
+        s_off[i] = (Off)(o - p0);
+        if (BATCHED && i < nets) s_bo[i] = c.net_off[e0 + i + 1] > o ? block_offset(c, c.pins[o]) : 0;
+      }
+      __syncthreads();
+      const Off p1 = s_off[nets];
+      const int32_t* pins = c.pins + p0;
+      for (Off j0 = threadIdx.x; j0 < p1; j0 += 4 * kPinTile) {
+        int b[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) b[u] = j0 + u * kPinTile < p1 ? pins[j0 + u * kPinTile] : -1;
+        for (int u = 0; u < 4; ++u) b[u] = j0 + u * kPinTile < p1 ? pins[j0 + u * kPinTile] : -1;
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (b[u] >= 0) b[u] = c.part[b[u]];
+        for (int u = 0; u < 4; ++u)
+          if (b[u] >= 0) b[u] = c.part[b[u]];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (b[u] < 0) continue;
-        const Off j = j0 + u * kPinTile;
-        int lo = 0, hi = nets - 1;  // the last net that starts at or before j
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (s_off[mid] <= j) lo = mid; else hi = mid - 1;
-        }
-        const int blk = BATCHED ? b[u] - s_bo[lo] : b[u], i = lo * k + blk;
-        unsigned old;
-        if constexpr (PHI16) {
-          const int sh = (i & 1) * 16;
-          old = (atomicAdd(&s_phi[i >> 1], 1u << sh) >> sh) & 0xFFFFu;
-        } else {
-          old = atomicAdd(&s_phi[i], 1u);
-        }
-        if (old <= 1) {
-          uint32_t* rec = s_rec + lo * 2 * W + (blk >> 5);
-          if (old == 0) atomicOr(rec, 1u << (blk & 31));
-          atomicXor(rec + W, 1u << (blk & 31));
+        for (int u = 0; u < 4; ++u) {
+          if (b[u] < 0) continue;
+          const Off j = j0 + u * kPinTile;
+          int lo = 0, hi = nets - 1;  // the last net that starts at or before j
+          while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (s_off[mid] <= j) lo = mid; else hi = mid - 1;
+          }
+          const int blk = BATCHED ? b[u] - s_bo[lo] : b[u], i = lo * k + blk;
+          unsigned old;
+          if constexpr (PHI16) {
+            const int sh = (i & 1) * 16;
+            old = (atomicAdd(&s_phi[i >> 1], 1u << sh) >> sh) & 0xFFFFu;
+          } else {
+            old = atomicAdd(&s_phi[i], 1u);
+          }
+          if (old <= 1) {
+            uint32_t* rec = s_rec + lo * 2 * W + (blk >> 5);
+            if (old == 0) atomicOr(rec, 1u << (blk & 31));
+            atomicXor(rec + W, 1u << (blk & 31));
+          }
         }
       }
+      __syncthreads();
+      // whole lines out: Φ is allocated in whole words
+      unsigned char* out = reinterpret_cast<unsigned char*>(c.phi) + e0 * k * esz;
+      if ((reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+        for (int i = threadIdx.x; i < (words >> 2); i += kPinTile)
+          reinterpret_cast<uint4*>(out)[i] = reinterpret_cast<const uint4*>(s_phi)[i];
+        for (int i = (words & ~3) + threadIdx.x; i < words; i += kPinTile) reinterpret_cast<uint32_t*>(out)[i] = s_phi[i];
+      } else {
+        for (int i = threadIdx.x; i < words; i += kPinTile) reinterpret_cast<uint32_t*>(out)[i] = s_phi[i];
+      }
+      for (int i = threadIdx.x; i < nets * 2 * W; i += kPinTile) c.conn[e0 * 2 * W + i] = s_rec[i];
+      __syncthreads();  // the image is cleared for the next nets
     }
-    __syncthreads();
-    // whole lines out: Φ is allocated in whole words, a tile starts on a word
-    unsigned char* out = reinterpret_cast<unsigned char*>(c.phi) + e0 * k * esz;
-    const int64_t words = ((int64_t)nets * k * esz + 3) >> 2;
-    if ((reinterpret_cast<uintptr_t>(out) & 15) == 0) {
-      for (int i = threadIdx.x; i < (words >> 2); i += kPinTile)
-        reinterpret_cast<uint4*>(out)[i] = reinterpret_cast<const uint4*>(s_phi)[i];
-      for (int i = (int)(words & ~(int64_t)3) + threadIdx.x; i < words; i += kPinTile)
-        reinterpret_cast<uint32_t*>(out)[i] = s_phi[i];
-    } else {
-      for (int i = threadIdx.x; i < words; i += kPinTile) reinterpret_cast<uint32_t*>(out)[i] = s_phi[i];
-    }
-    for (int i = threadIdx.x; i < nets * 2 * W; i += kPinTile) c.conn[e0 * 2 * W + i] = s_rec[i];
-    __syncthreads();  // the image is cleared for the next tile
   }
 }
 
-// Nets per tile: an image of at most 24 KB (initializePartition of row-net 4.2M,
-// k = 128 / geometric 250,007, k = 300: 8 KB 623 / 107 us, 16 KB 493 / 81, 20 KB 490 /
-// 76, 24 KB 515 / 75, 32 KB 519 / 75; others within 2 %), an even number so that
-// every tile starts on a word of 16-bit entries, and at least two tiles per SM
-// where the nets allow it.
-static int pin_tile(const Launch& L, const RoundCtx& c) {
-  const int64_t row = (int64_t)c.kmax * (c.phi16 ? 2 : 4);
-  int64_t tn = std::min<int64_t>(kPinNets, std::max<int64_t>(2, 24576 / row));
-  tn = std::min(tn, std::max<int64_t>(8, c.m / (2 * (int64_t)L.num_sms)));
-  return (int)(tn & ~(int64_t)1);
+// Nets at a time: what leaves eight CTAs in 196 KB of shared memory and 60 KB of the
+// SM to the L1 cache, which the block gathers live on (row-net 4.2M, k = 128, 64 / 80
+// / 96 nets: 522 / 522 / 680 us, and 96 with the smaller shared memory that is then
+// left for six CTAs 558; 1M, k = 61, 96 / 140 / 180: 126 / 122 / 142; 250,007, k =
+// 300, 28 / 40: 81 / 78). Units per CTA and step: four fifths of those nets on
+// average, so that few ranges need a second image, and at least two ranges per SM.
+#ifndef LPGPU_PIN_SMEM
+#define LPGPU_PIN_SMEM 23900
+#endif
+#ifndef LPGPU_PIN_FILL
+#define LPGPU_PIN_FILL 80
+#endif
+static void pin_tile(const Launch& L, const RoundCtx& c, int64_t units, int* tn, int* span) {
+  const int64_t per_net = (int64_t)c.kmax * (c.phi16 ? 2 : 4) + 8 * (int64_t)c.W + 12;
+  *tn = (int)std::min<int64_t>(kPinNets, std::max<int64_t>(2, LPGPU_PIN_SMEM / per_net)) & ~1;
+  const int64_t fill = *tn * units * LPGPU_PIN_FILL / (100 * c.m), spread = units / (2 * (int64_t)L.num_sms);
+  *span = (int)std::max<int64_t>(1, std::min(fill, spread));
 }
 
-cudaError_t launch_init_partition(const Launch& L, const RoundCtx& c) {
+cudaError_t launch_init_partition(const Launch& L, const RoundCtx& c, const int32_t* unit_first, int64_t units) {
   cudaError_t e;
   if ((e = cudaMemsetAsync(c.bw, 0, sizeof(int64_t) * c.k, L.st)) != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(c.scal + kPinTiles, 0, sizeof(int64_t), L.st)) != cudaSuccess) return e;
@@ -406,13 +432,14 @@ cudaError_t launch_init_partition(const Launch& L, const RoundCtx& c) {
   }
   if (c.m > 0) {
     // k_pin_counts writes all of Φ and the Λ records, zeros included
-    const int tn = pin_tile(L, c);
+    int tn, span;
+    pin_tile(L, c, units, &tn, &span);
     const size_t smem = (((size_t)tn * c.kmax * (c.phi16 ? 2 : 4) + 15) & ~size_t(15)) +
                         4 * (((size_t)tn * 2 * c.W + 3) & ~size_t(3)) + sizeof(int64_t) * (tn + 1) + sizeof(int) * tn;
     auto kern = c.phi16 ? (c.batched ? k_pin_counts<true, true> : k_pin_counts<true, false>)
                         : (c.batched ? k_pin_counts<false, true> : k_pin_counts<false, false>);
-    kern<<<grid_for(L, (c.m + tn - 1) / tn, 1, occupancy((const void*)kern, kPinTile, smem)), kPinTile, smem, L.st>>>(
-        c, tn);
+    kern<<<grid_for(L, (units + span - 1) / span, 1, occupancy((const void*)kern, kPinTile, smem)), kPinTile, smem, L.st>>>(
+        c, tn, span, unit_first, units);
     LAUNCHED("k_pin_counts");
   }
   return cudaSuccess;

@@ -156,7 +156,7 @@ struct lpgpu_session_s {
   DevBuf<int64_t> bw, lmax, perfect;
   std::vector<int64_t> h_perfect;
   // refine scratch
-  DevBuf<int32_t> list, net_epoch, seg_w, heavy, revl;
+  DevBuf<int32_t> list, net_epoch, seg_w, heavy, revl, unit_first;
   DevBuf<int64_t> sub_off, blk64, scal, stats, bin_cnt, scan_tmp;
   DevBuf<uint8_t> next_flag, status, over;
   DevBuf<int4> rec;
@@ -342,7 +342,7 @@ struct lpgpu_session_s {
     release_partition();
     DevBuf<int64_t>* b64[] = {&net_off, &vtx_off, &sub_off, &stats, &bin_cnt, &scan_tmp};
     for (auto* b : b64) b->release(&mem);
-    DevBuf<int32_t>* b32[] = {&pins, &inets, &w_v, &w_e, &list, &net_epoch, &seg_w, &heavy, &revl};
+    DevBuf<int32_t>* b32[] = {&pins, &inets, &w_v, &w_e, &list, &net_epoch, &seg_w, &heavy, &revl, &unit_first};
     for (auto* b : b32) b->release(&mem);
     next_flag.release(&mem);
     saved_part.release(&mem);
@@ -540,6 +540,7 @@ static lpgpu_status upload_impl(lpgpu_session* s, int64_t n, int64_t m, int64_t 
   CK(s->w_v.alloc(n, fp));
   CK(s->w_e.alloc(m, fp));
   CK(s->net_epoch.alloc(m, fp));
+  CK(s->unit_first.alloc(net_units(m, P) + 1, fp));
   CK(s->list.alloc(n, fp));
   CK(s->next_flag.alloc(n, fp));
   CK(s->status.alloc(n, fp));
@@ -659,7 +660,7 @@ static lpgpu_status upload_impl(lpgpu_session* s, int64_t n, int64_t m, int64_t 
   TmpBuf<int32_t> rank(s->mem);  // each pin's slot in its vertex's incident-net list
   CK(rank.alloc((size_t)P));
   CK(launch_build_incidence(s->launch(), n, m, P, s->net_off.p, s->pins.p, s->vtx_off.p, s->inets.p, rank.p(),
-                            s->scan_tmp.p, s->scan_tmp_n, s->vout.p));
+                            s->scan_tmp.p, s->scan_tmp_n, s->vout.p, s->unit_first.p));
   CK(cudaMemcpyAsync(s->deg_inc, s->vout.p, sizeof(s->deg_inc), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   s->has_hg = true;
@@ -766,7 +767,7 @@ static lpgpu_status set_partition_impl(lpgpu_session* s, int32_t K, int32_t kmax
   CK(launch_check_partition(s->launch(), s->n, s->part.p, K, s->batched ? s->vinst.p : nullptr,
                             s->inst_boff.p, s->inst_k.p, s->vout.p));
   RoundCtx c = s->ctx();
-  CK(launch_init_partition(s->launch(), c));
+  CK(launch_init_partition(s->launch(), c, s->unit_first.p, net_units(s->m, s->P)));
   int64_t check = 0;
   CK(cudaMemcpyAsync(&check, s->vout.p + kVErr, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
@@ -1892,6 +1893,7 @@ int64_t lpgpu_estimate_footprint(int64_t n, int64_t m, int64_t P, int32_t k, int
   const int64_t W = word_class_of(std::max(1, k));
   int64_t b = 0;
   b += 8 * (m + 1) + 8 * (n + 1) + 4 * P * 2 + 4 * n + 4 * m;          // CSR + weights
+  b += 4 * (net_units(m, P) + 1);                                      // first net of every unit
   b += 4 * m + 4 * n + n + n + 16 * n + 8 * n + 4 * n + 8 * n;         // epoch, list, flags, status, rec, seg, queues
   b += 8 * (2 * kMaxSubrounds + 1) + 8 * 2 * kMaxSubrounds * kDegClasses;  // sub-round bins
   b += 8 * (scan_tmp_elems(n + 1) + 1);
@@ -1924,7 +1926,7 @@ lpgpu_status lpgpu_session_restore_partition(lpgpu_session* s) {
   if (s->n > 0)
     CK(cudaMemcpyAsync(s->part.p, s->saved_part.p, sizeof(int32_t) * s->n, cudaMemcpyDeviceToDevice, s->st));
   RoundCtx c = s->ctx();
-  CK(launch_init_partition(s->launch(), c));
+  CK(launch_init_partition(s->launch(), c, s->unit_first.p, net_units(s->m, s->P)));
   return LPGPU_OK;
 }
 
