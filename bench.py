@@ -15,9 +15,12 @@ vertices) are reported beside it as `swept_pins_per_s`.
 GPU arm (`value`): inputs resident in HBM, device time with CUDA events on
 the session stream. `e2e`: the same work through the public session API from
 pinned host buffers (upload + set_partition + refine + download per step),
-wall-clock. `roofline`: the sweep kernel (dominant) against the measured HBM
-copy bandwidth, and `round_frac`: the algorithmic bytes of sweep, selection
-and commit of a whole step over the step time, against the same peak.
+wall-clock. `roofline`: the kernel that the timed step
+runs (`k_team`, all rounds in one launch): the algorithmic bytes of sweep,
+selection and commit over the device time of its refine call, against the
+measured HBM copy bandwidth; `round_frac`: the same bytes over the whole step;
+`pipeline_sweep`: the sweep as a kernel of its own, in the multi-launch form
+that per-phase events need (`phases_ms_per_step`).
 `cpu_baseline`: the reference-style asynchronous LP (CPU restatement, all
 host cores) on one full refinement of the same instance.
 
@@ -168,10 +171,10 @@ def hbm_peak():
         return FALLBACK_HBM_GBS, "fallback"
 
 
-def ncu_traffic_ratio():
-    """DRAM bytes / algorithmic bytes of the sweep kernel from the committed ncu
-    summary (profiles/k_sweep_rownet.txt), or None."""
-    path = os.path.join(ROOT, "profiles", "k_sweep_rownet.txt")
+def ncu_traffic_ratio(name):
+    """DRAM bytes / algorithmic bytes of a kernel on the row-net workload from
+    its committed ncu summary (profiles/<name>.txt), or None."""
+    path = os.path.join(ROOT, "profiles", name + ".txt")
     try:
         for line in open(path):
             if line.startswith("traffic_over_algorithmic:"):
@@ -290,7 +293,7 @@ def gpu_arm(args):
     dist.barrier()
     s.synchronize()
     clocks.start()
-    # timed region 1: whole steps (CUDA-graph replay), device time between events
+    # timed region 1: whole steps, device time between events
     launches0 = lpgpu.kernel_launches()
     s.record(0)
     pins = 0
@@ -302,8 +305,16 @@ def gpu_arm(args):
     s.record(1)
     elapsed_ms = s.elapsed_ms(0, 1)
     launches = lpgpu.kernel_launches() - launches0
-    # timed region 2: the same steps with CUDA events around every phase
-    # (direct launches) for the per-kernel roofline of the sweep
+    # timed region 2: the refine calls alone (k_team between its begin and end kernels)
+    refine_ms = 0.0
+    for _ in range(args.steps):
+        s.restore_partition()
+        s.record(0)
+        s.refine(cfg)
+        s.record(1)
+        refine_ms += s.elapsed_ms(0, 1)
+    stats = s.round_stats()
+    # timed region 3: the multi-launch form with CUDA events around every phase
     s.enable_timing(True)
     sweep_ms = 0.0
     sweep_launches = 0
@@ -311,10 +322,10 @@ def gpu_arm(args):
     phase_tot = {}
     for _ in range(args.steps):
         step()
-        stats, phases = s.round_stats(), s.phase_times()
+        phases = s.phase_times()
         sweep_ms += phases["sweep"][1]
         sweep_launches += phases["sweep"][0]
-        sweep_alg += sweep_bytes(stats, inst.k)
+        sweep_alg += sweep_bytes(s.round_stats(), inst.k)
         for name, (cnt, ms) in phases.items():
             a = phase_tot.setdefault(name, [0, 0.0])
             a[0] += cnt
@@ -328,18 +339,24 @@ def gpu_arm(args):
     swept = dist.reduce(pins, "sum") / (max_ms / 1e3)
 
     peak, peak_kind = hbm_peak()
-    achieved = (sweep_alg / sweep_launches) / ((sweep_ms / sweep_launches) / 1e3) / 1e9
-    ratio = ncu_traffic_ratio()
     b_sweep, b_select, b_commit = round_bytes(stats, inst.k, cfg.subrounds)  # every step is the same refinement
+    alg = b_sweep + b_select + b_commit
+    achieved = alg / (refine_ms / args.steps / 1e3) / 1e9
     step_s = max_ms / args.steps / 1e3
-    roofline = {"bound": "hbm", "kernel": "k_sweep", "achieved": achieved, "peak": peak,
+    traffic = {x: ncu_traffic_ratio(x + "_rownet") if args.workload == "rownet" else None for x in ("k_team", "k_sweep")}
+    sweep_gbs = sweep_alg / (sweep_ms / 1e3) / 1e9
+    roofline = {"bound": "hbm", "kernel": "k_team", "achieved": achieved, "peak": peak,
                 "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)"
                 if peak_kind == "measured" else "fallback 6.8 TB/s",
-                "traffic": None if ratio is None else ratio * sweep_alg / sweep_launches,
-                "algorithmic_bytes_per_launch": sweep_alg / sweep_launches,
-                "avg_launch_ms": sweep_ms / sweep_launches, "launches": sweep_launches,
-                "round_frac": (b_sweep + b_select + b_commit) / step_s / 1e9 / peak,
-                "round_bytes_per_step": {"sweep": b_sweep, "select": b_select, "commit": b_commit}}
+                "traffic": None if traffic["k_team"] is None else traffic["k_team"] * alg,
+                "algorithmic_bytes_per_launch": alg, "avg_launch_ms": refine_ms / args.steps, "launches": args.steps,
+                "round_frac": alg / step_s / 1e9 / peak,
+                "round_bytes_per_step": {"sweep": b_sweep, "select": b_select, "commit": b_commit},
+                "pipeline_sweep": {"kernel": "k_sweep", "achieved": sweep_gbs, "frac": sweep_gbs / peak,
+                                   "traffic": None if traffic["k_sweep"] is None
+                                   else traffic["k_sweep"] * sweep_alg / sweep_launches,
+                                   "algorithmic_bytes_per_launch": sweep_alg / sweep_launches,
+                                   "avg_launch_ms": sweep_ms / sweep_launches, "launches": sweep_launches}}
 
     e2e = None
     if not args.no_e2e:
