@@ -124,3 +124,62 @@ def test_rebalance_with_empty_blocks_matches_oracle(lp, orc, k):
     assert km1 == km0 + r.delta == r.km1_after
     _, _, ebw = orc.init_partition(hg, k, epart)
     assert np.array_equal(bw, ebw) and (bw > 0).all()
+
+
+def _by_degree(n, pins, k, order, seed=1):
+    """Vertex degrees of a power law, the largest first or anywhere; the 64 largest
+    and a third of the others in block 0."""
+    from lpgpu import gen
+    rng = np.random.default_rng(seed)
+    m = pins // 4
+    p = np.cumsum((np.arange(n) + 1.0) ** -0.6)
+    v = np.minimum(np.searchsorted(p / p[-1], rng.random(4 * m)), n - 1)
+    part = rng.permutation(np.arange(n) % k)
+    part[rng.random(n) < 0.3] = 0
+    part[:64] = 0
+    place = np.arange(n) if order == "first" else rng.permutation(n)
+    key = np.unique(np.repeat(np.arange(m, dtype=np.int64), 4) * n + place[v])
+    off = np.zeros(m + 1, np.int64)
+    np.cumsum(np.bincount(key // n, minlength=m), out=off[1:])
+    part_of = np.empty(n, np.int32)
+    part_of[place] = part
+    return gen.Hypergraph(n, m, off, (key % n).astype(np.int32), rng.integers(1, 4, n).astype(np.int32),
+                          rng.integers(1, 9, m).astype(np.int32)).with_incidence(), part_of
+
+
+@pytest.mark.parametrize("k", [2, 100, 129, 300])
+def test_rebalance_of_neighbouring_hubs_matches_oracle(lp, orc, k):
+    hg, part = _by_degree(3000, 60000, k, "first")
+    perfect = -(-int(hg.w_v.sum()) // k)
+    lmax = np.full(k, int(1.03 * perfect), np.int64)
+    with lp.Session(0) as s:
+        s.upload(hg)
+        s.set_partition(k, part, lmax=lmax, perfect=np.full(k, perfect, np.int64))
+        s.rebalance(8)
+        got, stats = s.partition(), s.round_stats()
+    want, want_stats = orc.rebalance(hg, k, lmax, part, 8)
+    assert np.array_equal(got, want)
+    keys = ["active", "pins", "candidates", "moved", "delta"]
+    assert [[x[q] for q in keys] for x in stats] == [[x[q] for q in keys] for x in want_stats]
+
+
+# The largest vertices side by side cost no more than the same ones anywhere: within 1.8
+# times (1.0 and 1.2 measured; 2.5 and 5.9 times when a warp took 32 neighbours in turn).
+@pytest.mark.parametrize("k", [16, 300])
+def test_rebalance_time_of_neighbouring_hubs(lp, k):
+    import time
+    times = []
+    for order in ("first", "anywhere"):
+        hg, part = _by_degree(200000, 2000000, k, order)
+        with lp.Session(0) as s:
+            s.upload(hg)
+            best = float("inf")
+            for _ in range(4):
+                s.set_partition(k, part, eps=0.03)
+                s.synchronize()
+                t0 = time.perf_counter()
+                r = s.rebalance(1)
+                best = min(best, time.perf_counter() - t0)
+            assert r.rounds >= 1
+        times.append(best)
+    assert times[0] < 1.8 * times[1]
