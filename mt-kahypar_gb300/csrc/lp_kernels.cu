@@ -2552,7 +2552,7 @@ cudaError_t launch_expand_nets(const Launch& L, const RoundCtx& c, int S, PhaseT
 // candidates leave a few overloaded blocks. 200,003 vertices, k = 32, 87,000 of
 // them in overloaded blocks: 234 -> 66 us (and k_rb_emit 85 -> 14).
 template <int W, bool UNIT>
-__global__ void __launch_bounds__(256) k_rb_candidates(RoundCtx c, int round, int32_t* __restrict__ rb_to,
+__global__ void __launch_bounds__(256) k_rb_candidates(RoundCtx c, int round, int at, int32_t* __restrict__ rb_to,
                                                        int32_t* __restrict__ rb_score, int64_t* __restrict__ rb) {
   constexpr bool kLv = W <= 4;
   constexpr int PL = UNIT ? 6 : 8, WL = kLv ? W : 1;
@@ -2576,10 +2576,10 @@ __global__ void __launch_bounds__(256) k_rb_candidates(RoundCtx c, int round, in
   // another, and the largest may lie side by side (300,000 vertices sorted by degree, up
   // to 10,469 nets each: a whole rebalance 5.1 -> 1.4 ms for k = 16, 123 -> 16.9 ms for k =
   // 300, where every vertex takes the warp).
-  const int64_t apart = (c.n + 31) >> 5;
+  const int64_t apart = (c.n + at - 1) / at;
   for (int64_t w = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); w < apart;
        w += (int64_t)gridDim.x * (blockDim.x >> 5)) {
-    const int64_t v = w + lane * apart;
+    const int64_t v = lane < at ? w + lane * apart : c.n;
     int from = 0, d = 0, wv = 0, to = -1, score = 0;
     int64_t o0 = 0;
     bool mine = false, heavy = false;
@@ -2954,8 +2954,11 @@ cudaError_t launch_rebalance_round(const Launch& L, const RoundCtx& c, int round
     const size_t smem = sizeof(ull) * 2 * k + (kW <= 4 ? sizeof(uint32_t) * kLvWeights * kW : 0) + (kW <= 4 ? 0 : sizeof(int) * k * 8);
     auto kern = c.unit_nets ? k_rb_candidates<kW, true> : k_rb_candidates<kW, false>;
     allow_dyn_smem(kern, smem);
-    kern<<<grid_for(L, c.n, 256, occupancy((const void*)kern, 256, smem)), 256, smem, L.st>>>(c, round, rb_to, rb_score,
-                                                                                           rb);
+    // vertices a warp takes at a time: one per lane, but for k > 128, where they take turns, no more than keep
+    // every warp busy (3,000 vertices, k = 1,000: a rebalance 2,103 -> 1,979 us, a warp per vertex 2,021)
+    const int per_sm = occupancy((const void*)kern, 256, smem);
+    const int at = kW <= 4 ? 32 : (int)std::min<int64_t>(32, 1 + c.n / (8 * per_sm * (int64_t)L.num_sms));
+    kern<<<grid_for(L, c.n, 8 * at, per_sm), 256, smem, L.st>>>(c, round, at, rb_to, rb_score, rb);
     LAUNCHED("k_rb_candidates");
   });
   k_rb_src_plan<<<1, 1024, 0, L.st>>>(c, rb);

@@ -183,3 +183,20 @@ def test_rebalance_time_of_neighbouring_hubs(lp, k):
             assert r.rounds >= 1
         times.append(best)
     assert times[0] < 1.8 * times[1]
+
+
+# k > 128: one, several and 32 vertices per warp and step, with a remainder
+@pytest.mark.parametrize("n,pins,k", [(9001, 60000, 1000), (60001, 400000, 140), (330001, 1300000, 129)])
+def test_rebalance_of_many_blocks_matches_oracle(lp, orc, n, pins, k):
+    hg, part = _by_degree(n, pins, k, "anywhere", seed=2)
+    perfect = -(-int(hg.w_v.sum()) // k)
+    lmax = np.full(k, int(1.03 * perfect), np.int64)
+    with lp.Session(0) as s:
+        s.upload(hg)
+        s.set_partition(k, part, lmax=lmax, perfect=np.full(k, perfect, np.int64))
+        s.rebalance(2)
+        got, stats = s.partition(), s.round_stats()
+    want, want_stats = orc.rebalance(hg, k, lmax, part, 2)
+    assert np.array_equal(got, want)
+    keys = ["active", "pins", "candidates", "moved", "delta"]
+    assert [[x[q] for q in keys] for x in stats] == [[x[q] for q in keys] for x in want_stats]
