@@ -156,7 +156,7 @@ struct lpgpu_session_s {
   DevBuf<int64_t> bw, lmax, perfect;
   std::vector<int64_t> h_perfect;
   // refine scratch
-  DevBuf<int32_t> list, net_epoch, seg_w, heavy, revl, unit_first;
+  DevBuf<int32_t> list, net_epoch, seg_w, heavy, revl;
   DevBuf<int64_t> sub_off, blk64, scal, stats, bin_cnt, scan_tmp;
   DevBuf<uint8_t> next_flag, status, over;
   DevBuf<int4> rec;
@@ -234,6 +234,9 @@ struct lpgpu_session_s {
     const int x = (int)(1000.0 * 2.0 * heavy / (2.0 * heavy + light));
     return x < 1 ? 1 : x;
   }
+
+  // First net of every unit (kUnit), behind the pins.
+  int32_t* unit_first() const { return pins.p + P; }
 
   // Φ entries fit 16 bits when every net has fewer than 2^16 pins.
   bool phi16() const { return LPGPU_PHI16 && max_net_size < 65536; }
@@ -342,7 +345,7 @@ struct lpgpu_session_s {
     release_partition();
     DevBuf<int64_t>* b64[] = {&net_off, &vtx_off, &sub_off, &stats, &bin_cnt, &scan_tmp};
     for (auto* b : b64) b->release(&mem);
-    DevBuf<int32_t>* b32[] = {&pins, &inets, &w_v, &w_e, &list, &net_epoch, &seg_w, &heavy, &revl, &unit_first};
+    DevBuf<int32_t>* b32[] = {&pins, &inets, &w_v, &w_e, &list, &net_epoch, &seg_w, &heavy, &revl};
     for (auto* b : b32) b->release(&mem);
     next_flag.release(&mem);
     saved_part.release(&mem);
@@ -535,12 +538,11 @@ static lpgpu_status upload_impl(lpgpu_session* s, int64_t n, int64_t m, int64_t 
   TmpBuf<int64_t> staged(s->mem);  // per-instance offsets before the rebase
   CK(s->net_off.alloc(m + 1, fp));
   CK(s->vtx_off.alloc(n + 1, fp));
-  CK(s->pins.alloc(P, fp));
+  CK(s->pins.alloc(P + net_units(m, P) + 1, fp));  // and the units' first nets
   CK(s->inets.alloc(P, fp));
   CK(s->w_v.alloc(n, fp));
   CK(s->w_e.alloc(m, fp));
   CK(s->net_epoch.alloc(m, fp));
-  CK(s->unit_first.alloc(net_units(m, P) + 1, fp));
   CK(s->list.alloc(n, fp));
   CK(s->next_flag.alloc(n, fp));
   CK(s->status.alloc(n, fp));
@@ -660,7 +662,7 @@ static lpgpu_status upload_impl(lpgpu_session* s, int64_t n, int64_t m, int64_t 
   TmpBuf<int32_t> rank(s->mem);  // each pin's slot in its vertex's incident-net list
   CK(rank.alloc((size_t)P));
   CK(launch_build_incidence(s->launch(), n, m, P, s->net_off.p, s->pins.p, s->vtx_off.p, s->inets.p, rank.p(),
-                            s->scan_tmp.p, s->scan_tmp_n, s->vout.p, s->unit_first.p));
+                            s->scan_tmp.p, s->scan_tmp_n, s->vout.p, s->unit_first()));
   CK(cudaMemcpyAsync(s->deg_inc, s->vout.p, sizeof(s->deg_inc), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   s->has_hg = true;
@@ -767,7 +769,7 @@ static lpgpu_status set_partition_impl(lpgpu_session* s, int32_t K, int32_t kmax
   CK(launch_check_partition(s->launch(), s->n, s->part.p, K, s->batched ? s->vinst.p : nullptr,
                             s->inst_boff.p, s->inst_k.p, s->vout.p));
   RoundCtx c = s->ctx();
-  CK(launch_init_partition(s->launch(), c, s->unit_first.p, net_units(s->m, s->P)));
+  CK(launch_init_partition(s->launch(), c, s->unit_first(), net_units(s->m, s->P)));
   int64_t check = 0;
   CK(cudaMemcpyAsync(&check, s->vout.p + kVErr, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
@@ -1926,7 +1928,7 @@ lpgpu_status lpgpu_session_restore_partition(lpgpu_session* s) {
   if (s->n > 0)
     CK(cudaMemcpyAsync(s->part.p, s->saved_part.p, sizeof(int32_t) * s->n, cudaMemcpyDeviceToDevice, s->st));
   RoundCtx c = s->ctx();
-  CK(launch_init_partition(s->launch(), c, s->unit_first.p, net_units(s->m, s->P)));
+  CK(launch_init_partition(s->launch(), c, s->unit_first(), net_units(s->m, s->P)));
   return LPGPU_OK;
 }
 
