@@ -514,7 +514,9 @@ LPGPU_API lpgpu_status lpgpu_session_synchronize(lpgpu_session* s);
 
 /* Kernel-phase timing with CUDA events on the session stream. When enabled,
  * every refine records, per named phase, the summed device time and launch
- * count; lpgpu_session_phase_times returns up to max entries. */
+ * count; lpgpu_session_phase_times returns up to max entries. Phases are
+ * launches of the multi-launch form, which a refine therefore takes unless a
+ * tuning or LPGPU_FLAG_PERSISTENT settles the other; the results are the same. */
 typedef struct {
   char name[24];
   int64_t launches;
