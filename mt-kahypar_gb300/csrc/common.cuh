@@ -332,6 +332,8 @@ cudaError_t launch_repair_candidates(const Launch& L, const RoundCtx& c, int blk
 // persistent form of the API accepts.
 constexpr int kTeamMaxK = LPGPU_MAX_K;
 constexpr int kPxMaxK = 64;
+// Nets of more pins are dealt out one by one when their pins become active.
+constexpr int64_t kTeamWideNet = 512;
 
 // One instance of a team launch. Arrays are indexed by the ids the instance's
 // CSR stores (union ids in a batched session), so several instances may share
@@ -377,6 +379,7 @@ struct PxParams {
   int32_t unroll;       // incidences per lane step of the sweep (8: in the 2-CTA builds for k <= 64)
   int32_t T;            // CTAs per team
   int32_t kcap;         // largest k of the launch
+  int32_t wide;         // nets of more than kTeamWideNet pins may activate theirs
   int32_t resident;     // bytes of shared memory per CTA for the instance's own arrays (set by the launch)
 };
 

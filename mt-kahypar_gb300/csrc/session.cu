@@ -1215,6 +1215,7 @@ lpgpu_status lpgpu_session_refine(lpgpu_session* s, const lpgpu_config* cfg_in,
   pxp.rounds = R;
   pxp.unroll = shape.unroll;
   pxp.kcap = kmax;
+  pxp.wide = std::min(pxp.act_threshold, s->max_net_size) > kTeamWideNet;
   pxp.T = shape.T;
   cudaStream_t st = s->st;
   RoundCtx c = s->ctx(&cfg);
@@ -1592,6 +1593,7 @@ lpgpu_status lpgpu_stepper_launch(lpgpu_stepper* t, lpgpu_session* const* sessio
     P.activate_last = 1;
     P.T = T;
     P.kcap = kPxMaxK;
+    for (int32_t i : groups[k]) P.wide |= std::min(P.act_threshold, sessions[i]->max_net_size) > kTeamWideNet;
     P.unroll = builds[gi].first;
     Launch Lg = L;
     const int lane = (int)(gi % 4) - 1;  // -1: the stepper's own stream

@@ -42,7 +42,7 @@ constexpr int kTeamWarps = kTeamThreads / 32;
 enum TeamSync : int { kSyncCta = 0, kSyncCluster = 1, kSyncGrid = 2 };
 
 // Global scratch of a team (64-bit words): barrier arrivals, abort flag, work
-// item, then three slots of per-block totals (sub-rounds take them in turn: in
+// item, wide nets, then three slots of per-block totals (sub-rounds take them in turn: in
 // sub-round s, after its first barrier, nobody reads the slot of s - 1 any
 // more and nobody adds to it before the first barrier of s + 1, so it is
 // cleared then), then the selection thresholds.
@@ -52,6 +52,7 @@ struct TeamGlob {
   __device__ ull* arrivals() const { return reinterpret_cast<ull*>(g); }
   __device__ int64_t* abort_flag() const { return g + 1; }
   __device__ int64_t* item() const { return g + 2; }
+  __device__ ull* wide() const { return reinterpret_cast<ull*>(g + 3); }  // wide nets listed by an expansion
   __device__ int64_t* slot(int q) const { return g + 8 + (int64_t)q * (5 * K + 8); }
   __device__ ull* in_w(int q) const { return reinterpret_cast<ull*>(slot(q)); }
   __device__ ull* in_cnt(int q) const { return in_w(q) + K; }
@@ -1398,6 +1399,12 @@ __device__ bool team_subround(const PxInst& I, const PxParams& P, const RoundCtx
   return true;
 }
 
+// Nets of more than kTeamWideNet pins are listed by an expansion (P.wide: some can be
+// stamped) and then dealt to the CTAs: where they lie side by side, one CTA's tile
+// held them all (400 nets of 8,192 pins beside 400,000 of 4, k = 2, no threshold:
+// 14,232 us, now 2,113; multi-launch pipeline 9,294. Zipf 1M, k = 32 4,010 -> 4,033,
+// row-net 1M, k = 61 3,780 -> 3,726, 4.2M 10,301 -> 10,165). Above kTeamBigNet they do
+// not fit the flat sums.
 constexpr int kTeamBigNet = 65536;
 
 // Copies `words` 32-bit words from src to dst (whole CTA).
@@ -1618,9 +1625,11 @@ __device__ bool team_instance(const PxInst& I, const PxParams& P, Team& tm, TS& 
     }
     TEAM_SYNC();
     // expansion: the pins of the stamped nets, CTA-flat over tiles of nets
-    // (nets above kTeamBigNet pins one by one: the flat sums stay in 32 bits)
+    ull* wide = T > 1 ? tm.G.wide() : reinterpret_cast<ull*>(&s.hint);
+    if (T == 1 && threadIdx.x == 0) s.hint = 0;
+    const int room = (int)(I.v1 - I.v0);  // entries of I.cand, whose kept moves are read
     for (int64_t b0 = I.e0 + (int64_t)tm.rank * kFlatItems; b0 < I.e1; b0 += (int64_t)T * kFlatItems) {
-      if (threadIdx.x == 0) f.n = s.nhuge = 0;
+      if (threadIdx.x == 0) f.n = 0;
       __syncthreads();
       constexpr int PER = kFlatItems / kTeamThreads;
       int64_t o0[PER], o1[PER];
@@ -1635,13 +1644,21 @@ __device__ bool team_instance(const PxInst& I, const PxParams& P, Team& tm, TS& 
       }
 #pragma unroll
       for (int p = 0; p < PER; ++p) {
-        const bool big = hit[p] && o1[p] - o0[p] > kTeamBigNet;
-        const int slot = flat_append(f, hit[p] && !big);
+        if (P.wide && hit[p] && o1[p] - o0[p] > kTeamWideNet) {
+          const int at = (int)atomicAdd(wide, 1ull);
+          if (at < room) {
+            I.cand[at] = (int)(b0 - I.e0) + p * kTeamThreads + (int)threadIdx.x;
+            hit[p] = false;
+          } else if (o1[p] - o0[p] > kTeamBigNet) {  // no room in either
+            for (int64_t j = o0[p]; j < o1[p]; ++j) I.flag[I.pins[j]] = 1;
+            hit[p] = false;
+          }
+        }
+        const int slot = flat_append(f, hit[p]);
         if (slot >= 0) {
           f.o0[slot] = o0[p];
           f.pre[slot] = (int)(o1[p] - o0[p]);
         }
-        if (big) f.inst[atomicAdd(&s.nhuge, 1)] = (int)(b0 - I.e0) + p * kTeamThreads + (int)threadIdx.x;
       }
       __syncthreads();
       const int n = f.n, total = flat_scan(f, n);
@@ -1657,13 +1674,26 @@ __device__ bool team_instance(const PxInst& I, const PxParams& P, Team& tm, TS& 
         for (int u = 0; u < kTeamGroup; ++u)
           if (pin[u] >= 0) I.flag[pin[u]] = 1;
       }
-      for (int i = 0; i < s.nhuge; ++i) {
-        const int64_t e = I.e0 + f.inst[i];
-        for (int64_t j = I.net_off[e] + threadIdx.x; j < I.net_off[e + 1]; j += kTeamThreads) I.flag[I.pins[j]] = 1;
-      }
       __syncthreads();
     }
     TEAM_SYNC();
+    if (P.wide) {
+      const int listed = (int)min((ull)room, *wide);
+      int64_t p0 = 0, p1 = 0;
+      for (int i = tm.rank - T; i < listed; i += T) {  // the next net's range in flight with a net's pins
+        int64_t q0 = 0, q1 = 0;
+        if (i + T < listed) {
+          const int64_t e = I.e0 + I.cand[i + T];
+          q0 = I.net_off[e];
+          q1 = I.net_off[e + 1];
+        }
+        for (int64_t j = p0 + threadIdx.x; j < p1; j += kTeamThreads) I.flag[I.pins[j]] = 1;
+        p0 = q0;
+        p1 = q1;
+      }
+      TEAM_SYNC();
+      if (T > 1 && tm.rank == 0 && threadIdx.x == 0) *wide = 0;  // nobody lists before the next round's barriers
+    }
   }
   __syncthreads();
   if (T == 1) {

@@ -322,3 +322,64 @@ def test_pipeline_graph_replay(lp):
         for x in got[1:]:
             _same(got[0], x)
         assert len(set(launches)) == 1
+
+
+def _uneven(n, sizes, seed=4):
+    from lpgpu import gen
+    rng = np.random.default_rng([seed, n])
+    pins = np.concatenate([(rng.integers(0, n) + rng.choice(n, z, replace=False)) % n for z in sizes]).astype(np.int32)
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    return gen.Hypergraph(n, len(sizes), off, pins, rng.integers(1, 4, n).astype(np.int32),
+                          rng.integers(1, 9, len(sizes)).astype(np.int32))
+
+
+# nets of more than 512 pins that become active: listed per team, up to one entry per
+# vertex, and dealt to its CTAs; one CTA, a cluster, the grid in both builds, 32-bit counts
+@pytest.mark.parametrize("n,sizes", [
+    (700, [600] * 30 + [3] * 900), (600, [520] * 900), (5000, [512, 513] * 60 + [4] * 5000), (40000, [3] * 9000 + [700] * 300),
+    (70001, [69000] + [600] * 40 + [5] * 30000), (661000, [4] * 300000 + [2000] * 50)])
+@pytest.mark.parametrize("threshold", [0, 512, 513])
+def test_team_activates_wide_nets(lp, n, sizes, threshold):
+    hg = _uneven(n, sizes)
+    part = (np.arange(n) * 3 % 5).astype(np.int32)
+    cfg = dict(rounds=4, activation_threshold=threshold, subrounds=3)
+    _same(_refine(lp, hg, 5, part, **cfg), _refine(lp, hg, 5, part, flags=lp.FLAG_MULTI_LAUNCH, **cfg))
+
+
+def test_stepped_teams_activate_wide_nets(lp):
+    hgs = [_uneven(4000, [900] * 40 + [4] * 4000, 1), _uneven(900, [600] * 20 + [3] * 700, 2), _uneven(3000, [4] * 3000, 3)]
+    cfg = lp.default_config(rounds=4, activation_threshold=0)
+    sessions = [lp.Session(0).upload(h) for h in hgs]
+    for s, h in zip(sessions, hgs):
+        s.set_partition(5, (np.arange(h.n) * 3 % 5).astype(np.int32), eps=0.03)
+        s.begin_rounds(cfg)
+    stepper, running = lp.Stepper(), list(sessions)
+    while running:
+        done = stepper.round(running)
+        running = [s for s, d in zip(running, done) if not d]
+    for s, h in zip(sessions, hgs):
+        s.end_rounds()
+        want = _refine(lp, h, 5, (np.arange(h.n) * 3 % 5).astype(np.int32), flags=lp.FLAG_MULTI_LAUNCH, rounds=4,
+                       activation_threshold=0)
+        assert np.array_equal(s.partition(), want[0])
+        s.close()
+
+
+# Large nets side by side that become active: faster than the pipeline (0.25 times its
+# time measured; 1.5 times when they were all in one CTA's tile).
+def test_wide_nets_side_by_side_stay_near_the_pipeline(lp):
+    from lpgpu import gen
+    rng = np.random.default_rng(2)
+    n, sizes = 400000, np.array([8192] * 400 + [4] * 400000)
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    inside = np.arange(off[-1]) - np.repeat(off[:-1], sizes)
+    pins = ((np.repeat(rng.integers(0, n, len(sizes)), sizes) + 48 * inside) % n).astype(np.int32)
+    hg = gen.Hypergraph(n, len(sizes), off, pins, np.ones(n, np.int32), rng.integers(1, 9, len(sizes)).astype(np.int32))
+    with lp.Session(0) as s:
+        s.upload(hg)
+        s.set_partition(2, rng.permutation(np.arange(n) % 2).astype(np.int32), eps=0.03)
+        s.save_partition()
+        pipeline, want = _fastest(s, lp.default_config(rounds=4, activation_threshold=0, flags=lp.FLAG_MULTI_LAUNCH))
+        default, got = _fastest(s, lp.default_config(rounds=4, activation_threshold=0))
+    assert np.array_equal(got, want)
+    assert default < 0.8 * pipeline
