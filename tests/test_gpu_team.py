@@ -278,7 +278,7 @@ def test_batches_stay_near_the_pipeline(lp, insts, k):
 
 
 # A session that takes another batch with all sizes and buffers as they were, but the
-# pins of its largest instances in another place, starts with those: within 1.2 times
+# pins of its largest instances in another place, starts with those: within 1.3 times
 # a fresh session (1.0 measured; 1.5 with the first batch's order).
 def test_batch_order_follows_the_input(lp):
     n, m, count = 2000, 6000, 1216
@@ -300,7 +300,7 @@ def test_batch_order_follows_the_input(lp):
         want, a = _fastest(fresh, cfg, 8)
         got, b = _fastest(s, cfg, 8)
     assert all(np.array_equal(x, y) for x, y in zip(a, b))
-    assert got < 1.2 * want
+    assert got < 1.3 * want
 
 
 # the pipeline captures its launches once and replays them: the same from every start, and as launched directly
